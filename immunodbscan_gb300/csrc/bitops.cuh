@@ -10,6 +10,9 @@
 //    Computing 10, 2003 -- block-based form with a horizontal delta carried
 //    between 32-row blocks).  The reference computes the same quantity with a
 //    full anti-diagonal DP (cuda/PSDBSCAN.hcu:246-290).
+//  * edit distance <= E by furthest-reaching points on mismatch bit masks
+//    (E. Ukkonen, "Algorithms for approximate string matching", Information and
+//    Control 64, 1985; G. Landau and U. Vishkin, J. Algorithms 10(2), 1989)
 //  * closed-form decode of triangular work-unit grids
 //  * a 64-bit mixing hash for the duplicate table
 #pragma once
@@ -123,6 +126,154 @@ IDB_HD int myers_distance(const uint8_t *p, int m, const uint8_t *t, int n) {
         }
     }
     return myers_value<W>(Pv, Mv, m, n);
+}
+
+// ---------------------------------------------------------------------------
+// Is the edit distance of x (length m) and y (length n = m + G) at most E?
+// Decided on the mismatch masks of a few diagonals instead of a column-by-column
+// recurrence: bit i of the mask of diagonal d says that x[i] != y[i + d].  An
+// alignment with at most E edits from (0,0) to (m,n) only visits the diagonals
+// -LO .. G + LO, LO = (E - G) / 2 (leaving further costs more than E to come
+// back), and on a diagonal it is always best to have consumed as much of x as
+// possible.  "Consumed" is a prefix mask F of x positions:
+//   t = D_d & ~F              mismatches not yet passed
+//   E = (t - 1) & ~t          prefix up to the first one (all ones if none)
+//   G = t ^ (t - 1)           the same with the mismatch itself
+// and with one more edit diagonal d starts from G_d (substitution),
+// E_{d-1} (a character of y skipped) and G_{d+1} (a character of x skipped);
+// the union of prefix masks is the longest, so merging is an OR.  Returns 0 iff
+// diagonal G is passed to its end after E edits.
+// Positions past an end need no masking for LO <= 1 (E <= 3): both strings
+// are padded with the same code, so diagonal G matches there; on a lower
+// diagonal x is exhausted and more prefix gains nothing; on diagonal G + 1 only
+// the last position of x lies past y's end, and passing it for free costs the
+// same one edit (skipping it) on the way back to diagonal G.
+// ---------------------------------------------------------------------------
+template <int E, int G>
+struct LevDiags {
+    static constexpr int lo = (E - G) / 2;       // lowest diagonal is -lo
+    static constexpr int n = G + 2 * lo + 1;
+    // cells (diagonal d, k edits) on some path within the budget
+    static constexpr bool cell(int d, int k) {
+        return k >= 0 && (d < 0 ? -d : d) <= k && (d < G ? G - d : d - G) <= E - k;
+    }
+};
+
+// r = t - 1 over W words, least significant first
+template <int W>
+IDB_HD void dec_words(const uint32_t (&t)[W], uint32_t (&r)[W]) {
+#if defined(__CUDA_ARCH__)
+    if (W == 1) {
+        r[0] = t[0] - 1u;
+    } else if (W == 2) {
+        asm("sub.cc.u32 %0, %2, 1; subc.u32 %1, %3, 0;"
+            : "=&r"(r[0]), "=r"(r[1 % W]) : "r"(t[0]), "r"(t[1 % W]));
+    } else if (W == 3) {
+        asm("sub.cc.u32 %0, %3, 1; subc.cc.u32 %1, %4, 0; subc.u32 %2, %5, 0;"
+            : "=&r"(r[0]), "=&r"(r[1 % W]), "=r"(r[2 % W])
+            : "r"(t[0]), "r"(t[1 % W]), "r"(t[2 % W]));
+    } else {
+        static_assert(W <= 4, "at most four words");
+        asm("sub.cc.u32 %0, %4, 1; subc.cc.u32 %1, %5, 0; subc.cc.u32 %2, %6, 0; subc.u32 %3, %7, 0;"
+            : "=&r"(r[0]), "=&r"(r[1 % W]), "=&r"(r[2 % W]), "=r"(r[3 % W])
+            : "r"(t[0]), "r"(t[1 % W]), "r"(t[2 % W]), "r"(t[3 % W]));
+    }
+#else
+    uint32_t b = 1;
+    for (int w = 0; w < W; ++w) {
+        const uint32_t v = t[w];
+        r[w] = v - b;
+        b = (uint32_t)(v < b);
+    }
+#endif
+}
+
+template <int W, int E, int G>
+IDB_HD uint32_t lev_diag(const uint32_t (&D)[LevDiags<E, G>::n][W]) {
+    using S = LevDiags<E, G>;
+    static_assert(E >= G && G >= 0 && S::lo <= 1, "diagonal test: G <= E <= 3");
+    uint32_t pe[S::n][W], pg[S::n][W];       // E and G masks of the previous edit count
+    uint32_t last = 0;
+#pragma unroll
+    for (int k = 0; k <= E; ++k) {
+        uint32_t ce[S::n][W], cg[S::n][W];
+#pragma unroll
+        for (int q = 0; q < S::n; ++q) {
+            const int d = q - S::lo;
+            if (!S::cell(d, k)) continue;
+            uint32_t t[W];
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                uint32_t f = 0;
+                if (S::cell(d, k - 1)) f |= pg[q][w];
+                if (q > 0 && S::cell(d - 1, k - 1)) f |= pe[q > 0 ? q - 1 : 0][w];
+                if (q + 1 < S::n && S::cell(d + 1, k - 1)) f |= pg[q + 1 < S::n ? q + 1 : q][w];
+                t[w] = D[q][w] & ~f;
+            }
+            if (k == E) {                    // the one cell left: diagonal G
+#pragma unroll
+                for (int w = 0; w < W; ++w) last |= t[w];
+                continue;
+            }
+            uint32_t m[W];
+            dec_words<W>(t, m);
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                ce[q][w] = m[w] & ~t[w];
+                cg[q][w] = m[w] ^ t[w];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < S::n; ++q)
+            if (k < E && S::cell(q - S::lo, k)) {
+#pragma unroll
+                for (int w = 0; w < W; ++w) { pe[q][w] = ce[q][w]; pg[q][w] = cg[q][w]; }
+            }
+    }
+    return last;
+}
+
+// y's bit plane (W words) moved so that bit i holds position i + d, -3 <= d <= 3
+template <int W>
+IDB_HD void shift_words(const uint32_t (&y)[W], int d, uint32_t (&r)[W]) {
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+        if (d == 0) {
+            r[w] = y[w];
+        } else if (d > 0) {
+            const uint32_t up = w + 1 < W ? y[w + 1 < W ? w + 1 : w] : 0u;
+            r[w] = (y[w] >> d) | (up << (32 - d));
+        } else {
+            const uint32_t dn = w > 0 ? y[w > 0 ? w - 1 : 0] : 0u;
+            r[w] = (y[w] << -d) | (dn >> (32 + d));
+        }
+    }
+}
+
+// Mismatch masks of two bit-plane records (word p*W + w, BP planes) and the
+// test above: 0 iff the edit distance is at most E.
+template <int BP, int W, int E, int G>
+IDB_HD uint32_t lev_planes(const uint32_t *x, const uint32_t *y) {
+    using S = LevDiags<E, G>;
+    uint32_t D[S::n][W];
+#pragma unroll
+    for (int q = 0; q < S::n; ++q)
+#pragma unroll
+        for (int w = 0; w < W; ++w) D[q][w] = 0;
+#pragma unroll
+    for (int p = 0; p < BP; ++p) {
+        uint32_t yw[W];
+#pragma unroll
+        for (int w = 0; w < W; ++w) yw[w] = y[p * W + w];
+#pragma unroll
+        for (int q = 0; q < S::n; ++q) {
+            uint32_t r[W];
+            shift_words<W>(yw, q - S::lo, r);
+#pragma unroll
+            for (int w = 0; w < W; ++w) D[q][w] |= x[p * W + w] ^ r[w];
+        }
+    }
+    return lev_diag<W, E, G>(D);
 }
 
 // ---------------------------------------------------------------------------

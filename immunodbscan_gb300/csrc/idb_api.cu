@@ -542,7 +542,25 @@ idb_status derive_plan(Pipeline &pl, const idb_params *prm) {
     if (!P.hamming && !P.fast && P.Lmax > (uint32_t)kGenericMaxLen)
         return fail(IDB_ERR_UNSUPPORTED, "Levenshtein mode supports sequences up to %d bytes",
                     kGenericMaxLen);
-    if (P.fast && P.hamming) {
+    // eps table over the length range, and the largest admissible gap
+    pl.eps_host.assign((size_t)P.NL * P.NL, 0);
+    int dl = 0;
+    int emin_same = INT32_MAX, emax_same = INT32_MIN;
+    int emax = 0;   // largest eps of an admissible length pair
+    for (uint32_t a = 0; a < P.NL; ++a)
+        for (uint32_t b = 0; b < P.NL; ++b) {
+            int e = eps_value(P.Lmin + a, P.Lmin + b, prm->threshold, prm->abs_eps);
+            if (e > 32767) e = 32767;
+            if (e < -1) e = -1;
+            pl.eps_host[(size_t)a * P.NL + b] = (int16_t)e;
+            if (b >= a && e >= (int)(b - a)) {
+                dl = std::max(dl, (int)(b - a));
+                emax = std::max(emax, e);
+            }
+            if (a == b) { emin_same = std::min(emin_same, e); emax_same = std::max(emax_same, e); }
+        }
+    P.lev_diag = P.fast && !P.hamming && emax <= kLevDiagMaxEps;
+    if (P.planes()) {
         P.B = P.A <= 4 ? 2 : 5;
         P.RS = ((P.B * P.W * 4) + 15) & ~15u;
     } else {
@@ -554,29 +572,12 @@ idb_status derive_plan(Pipeline &pl, const idb_params *prm) {
         P.RX = P.W == 1 ? 8 : 4;
         P.TX = 32 * P.RX;
         P.TY = 256;
-    } else if (P.fast) {
-        P.RX = 1;
-        P.TX = 32;
-        P.TY = 256;
     } else {
-        P.RX = 1;
-        P.TX = 32;
+        P.RX = P.lev_diag && P.W == 1 ? 2 : 1;
+        P.TX = 32 * P.RX;
         P.TY = 256;
     }
     if (P.fast) apply_shape(P, prm->tile_rx, prm->tile_ty);
-    // eps table over the length range, and the largest admissible gap
-    pl.eps_host.assign((size_t)P.NL * P.NL, 0);
-    int dl = 0;
-    int emin_same = INT32_MAX, emax_same = INT32_MIN;
-    for (uint32_t a = 0; a < P.NL; ++a)
-        for (uint32_t b = 0; b < P.NL; ++b) {
-            int e = eps_value(P.Lmin + a, P.Lmin + b, prm->threshold, prm->abs_eps);
-            if (e > 32767) e = 32767;
-            if (e < -1) e = -1;
-            pl.eps_host[(size_t)a * P.NL + b] = (int16_t)e;
-            if (b >= a && e >= (int)(b - a) && (int)(b - a) > dl) dl = (int)(b - a);
-            if (a == b) { emin_same = std::min(emin_same, e); emax_same = std::max(emax_same, e); }
-        }
     P.dLmax = P.hamming ? 0 : dl;
     P.hamming_eps_mode = 0;
     if (P.hamming && emin_same == emax_same && emin_same == 1) P.hamming_eps_mode = 1;

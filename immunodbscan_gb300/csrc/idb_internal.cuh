@@ -29,6 +29,9 @@ constexpr uint32_t kTinySide = 8;
 // buckets evaluate their pairs faster (64 repertoires, 1M rows: 2.92 against
 // 3.09 ms per call; eps 1: 1.25 against 0.99 ms for the join).
 constexpr int kJoinMaxEps = 2;
+// Levenshtein with eps <= kLevDiagMaxEps at every admissible length pair uses the
+// diagonal test (bitops.cuh); above that its cost per pair grows with eps^2.
+constexpr int kLevDiagMaxEps = 3;
 constexpr int kMlpIn = 16;              // learned scheduler: features per bin pair
 constexpr int kMlpHidden = 64;          // two hidden layers of 64
 constexpr int kMlpParams = kMlpIn * kMlpHidden + kMlpHidden + kMlpHidden * kMlpHidden + kMlpHidden +
@@ -194,6 +197,9 @@ struct Plan {
     int schedule = 0;
     int hamming_eps_mode = 0;                     // 0 popcount, 1 eps==1, 2 eps==0
     bool sig_exact = true;                        // V genes <= 64 and J genes <= 32
+    bool lev_diag = false;                        // Levenshtein by the diagonal test
+    // records are bit planes (else one code byte per residue)
+    bool planes() const { return fast && (hamming || lev_diag); }
     bool join = false;                            // Hamming by segment join (eps <= kJoinMaxEps)
     uint32_t join_smax = 1;                       // most segments of any length
     bool streamed = false;                        // neighbour pairs not stored: the

@@ -156,14 +156,14 @@ __global__ void k_bin_hist(BinGeom g, const Counters *__restrict__ ctr,
 }
 
 // Record of one unique.
-//  planes (Hamming, fast path): Bp bit planes x W words; bit i of word
+//  planes (fast path; Hamming and the diagonal edit-distance test): Bp bit planes x W words; bit i of word
 //    p*W + i/32 is bit p of the code of residue i.  Hamming distance of two
 //    records = sum over words of popc(OR_p (x_p ^ y_p)).
-//  codes (Levenshtein and generic path): one code byte per residue.
+//  codes (other Levenshtein and the generic path): one code byte per residue.
 // Codes are a bijection of the byte values present, so equality of codes is
 // equality of bytes.
 // The record of one unique (fast paths: at most NR 16-byte words): bit planes
-// (Hamming) or code bytes (Levenshtein), residues read 4 at a time.
+// or code bytes, residues read 4 at a time.
 // Bit planes of one sequence (L <= 128): bit i of wd[p][w] is bit p of the
 // code of residue 32w + i; positions past L keep code 0.  Residues are read 4
 // at a time.
@@ -844,7 +844,7 @@ void launch_fill(const Plan &P, const Buffers &B, cudaStream_t s) {
     BinGeom g{P.Gv, P.Gj, P.NL, P.Lmin, P.VW, P.JW, P.K};
     cudaMemsetAsync(B.bin_cursor, 0, sizeof(uint32_t) * P.nbins, s);
     cudaMemsetAsync(B.sig_and, 0xFF, sizeof(unsigned long long) * 2 * P.nbins, s);
-    const int planes = (P.fast && P.hamming) ? (int)P.B : 0;
+    const int planes = P.planes() ? (int)P.B : 0;
     const uint32_t rs16 = P.RS / 16;
     auto go = [&](auto kern) {
         kern<<<grid_wave(kern, P.N, kThreads), kThreads, 0, s>>>(
@@ -903,7 +903,7 @@ void launch_schedule(const Plan &P, const Buffers &B, cudaStream_t s) {
     cudaMemsetAsync(&B.ctr->n_tiny, 0, 2 * sizeof(uint32_t), s);    // n_tiny, tiny_cursor
     k_cls_scatter<<<grid_for(P.cap_binpairs), kThreads, 0, s>>>(
         B.ctr, B.bp, pred, B.cls_hist, B.cls_hist + 64, B.bp_sorted, B.bp_units, P.TX, P.TY, q,
-        (P.fast && P.hamming) ? 1 : 0, B.bp_small, &B.ctr->n_small, &B.ctr->n_tiny,
+        P.planes() ? 1 : 0, B.bp_small, &B.ctr->n_small, &B.ctr->n_tiny,
         (uint32_t)P.cap_binpairs + 1u);
     scan_u32(B.bp_units, B.bp_units, (uint32_t)P.cap_binpairs, &B.ctr->n_binpairs,
              &B.ctr->n_units, B.scan_part, B.scan_part_cap, s);

@@ -1,0 +1,335 @@
+// lev_diag.cuh -- the neighbour search for edit distances up to kLevDiagMaxEps.
+//
+// Reference: the anti-diagonal DP of levenshtein_distance
+// (cuda/PSDBSCAN.hcu:246-290), one block per pair.  Here a pair costs no
+// recurrence over columns: both sequences are bit planes (as for Hamming), the
+// mismatch masks of the few diagonals an alignment within eps can visit are
+// BP logic operations per word each, and the furthest-reaching test on them
+// (lev_diag, bitops.cuh) is exact, so it needs no filter in front of it.
+//
+// Integer-pipe bound (eps 2, equal lengths, one word, 5 planes: 15 LOP3 for three
+// masks + 14 for the test).  The y-records are staged with one copy per diagonal,
+// already shifted, so the tiled loop reads them as 16-byte broadcasts and does
+// no shifts per pair; RX x-entries per lane share every broadcast.  Against the
+// filters + Myers kernel it replaces for these eps (whole calls): 200,000
+// nucleotide rows, eps 2: 15.2 -> 1.5 ms; 1M rows with skewed gene usage, eps 2
+// (38.9e9 pairs): 95.9 -> 41.2 ms; 2M rows, eps min(3, 0.15 L): 72.0 -> 32.4 ms.
+#pragma once
+#include "distance_common.cuh"
+
+namespace idb {
+
+namespace {
+
+template <int BP, int W>
+struct LevShape {
+    static constexpr int NW = BP * W;            // words per record
+    static constexpr int R16 = (NW + 3) / 4;     // 16-byte words per record
+    static constexpr int YMax = NW;              // 16-byte words of a staged y (4 diagonals)
+    // y-records staged per batch, so that a block's static shared memory stays
+    // below 48 KB
+    static constexpr int YB = NW <= 8 ? 64 : (NW <= 15 ? 32 : 16);
+};
+
+template <int BP, int W>
+__device__ __forceinline__ void load_planes(const uint4 *src, uint32_t (&v)[BP * W]) {
+#pragma unroll
+    for (int q = 0; q < LevShape<BP, W>::R16; ++q) {
+        const uint4 u = __ldg(src + q);
+        const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (4 * q + e < BP * W) v[4 * q + e] = w4[e];
+    }
+}
+
+// One pair straight from its records, any admissible (eps, length gap): 0 iff
+// within eps.  Out of line: the small bin pairs' lanes may hold different ones.
+template <int BP, int W>
+__device__ __noinline__ uint32_t lev_pair(const uint4 *xr, const uint4 *yr, uint32_t e, uint32_t g) {
+    uint32_t x[BP * W], y[BP * W];
+    load_planes<BP, W>(xr, x);
+    load_planes<BP, W>(yr, y);
+    switch (e * 4 + g) {
+        case 0: return lev_planes<BP, W, 0, 0>(x, y);
+        case 4: return lev_planes<BP, W, 1, 0>(x, y);
+        case 5: return lev_planes<BP, W, 1, 1>(x, y);
+        case 8: return lev_planes<BP, W, 2, 0>(x, y);
+        case 9: return lev_planes<BP, W, 2, 1>(x, y);
+        case 10: return lev_planes<BP, W, 2, 2>(x, y);
+        case 12: return lev_planes<BP, W, 3, 0>(x, y);
+        case 13: return lev_planes<BP, W, 3, 1>(x, y);
+        case 14: return lev_planes<BP, W, 3, 2>(x, y);
+        case 15: return lev_planes<BP, W, 3, 3>(x, y);
+    }
+    return 1u;
+}
+
+// A warp's shared memory.
+struct LevSlice {
+    uint4 *sy;       // staged y-records, one shifted copy per diagonal
+    uint4 *sym;      // y side records
+    uint4 *sxm;      // x side records
+    uint32_t *shq;   // deferred hits
+};
+
+// One tiled unit: 32*RX x-entries in registers against the unit's y-entries.
+template <int BP, int W, int RX, int E, int G>
+__device__ __forceinline__ void lev_unit(const DistArgs &a, EdgeWriter &ew, const Unit &U,
+                                         const LevSlice &S, int lane, uint64_t &pairs) {
+    using Sh = LevShape<BP, W>;
+    using Dg = LevDiags<E, G>;
+    constexpr int NW = Sh::NW;
+    constexpr int Y16 = (Dg::n * NW + 3) / 4;    // 16-byte words of a staged y
+    static_assert(Y16 <= Sh::YMax, "staged y-record size");
+    const bool same = U.P.same != 0;
+    uint32_t x[RX][NW], vmask[RX];
+#pragma unroll
+    for (int r = 0; r < RX; ++r) {
+        const uint32_t xi = (uint32_t)r * 32 + lane;
+        const bool ok = xi < U.nx;
+        const uint32_t row = U.P.a_start + U.xbase + (ok ? xi : 0);
+        vmask[r] = ok ? 0u : kOff;
+        load_planes<BP, W>(a.rec + (size_t)row * Sh::R16, x[r]);
+        S.sxm[xi] = __ldg(a.meta + row);
+        if (ok) pairs += unit_pairs(U, U.xbase + xi);
+    }
+    const uint32_t yrow0 = (same ? U.P.a_start : U.P.b_start) + U.ybase;
+    // same bin: y-entries at or before the first x-entry pair with nothing
+    const uint32_t y0 = (same && U.xbase >= U.ybase) ? min(U.ny, U.xbase - U.ybase + 1) : 0u;
+    for (uint32_t yb = y0; yb < U.ny; yb += Sh::YB) {
+        const uint32_t nb = min((uint32_t)Sh::YB, U.ny - yb);
+        __syncwarp();
+        for (uint32_t t = lane; t < nb; t += 32) {
+            uint32_t y[NW], o[4 * Y16];
+            load_planes<BP, W>(a.rec + (size_t)(yrow0 + yb + t) * Sh::R16, y);
+#pragma unroll
+            for (int q = 0; q < Dg::n; ++q)
+#pragma unroll
+                for (int p = 0; p < BP; ++p) {
+                    uint32_t in[W], sh[W];
+#pragma unroll
+                    for (int w = 0; w < W; ++w) in[w] = y[p * W + w];
+                    shift_words<W>(in, q - Dg::lo, sh);
+#pragma unroll
+                    for (int w = 0; w < W; ++w) o[q * NW + p * W + w] = sh[w];
+                }
+#pragma unroll
+            for (int k = Dg::n * NW; k < 4 * Y16; ++k) o[k] = 0u;
+#pragma unroll
+            for (int k = 0; k < Y16; ++k)
+                S.sy[t * Y16 + k] = make_uint4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
+            S.sym[t] = __ldg(a.meta + yrow0 + yb + t);
+        }
+        __syncwarp();
+        // y-entries inside the unit's own x range (same bin) need the mask of the
+        // x-entries before them; they come first in the chunk
+        uint32_t tdiag = 0;
+        if (same && U.ybase + yb < U.xbase + U.nx) tdiag = min(nb, U.xbase + U.nx - (U.ybase + yb));
+        auto is_edge = [&](uint32_t r, uint32_t, const uint4 &my) {
+            return canonical_meta(a, U.P, S.sxm[32 * r + lane], my);
+        };
+        uint32_t qn = 0;
+        for (uint32_t t = 0; t < nb; ++t) {
+            uint32_t y[4 * Y16];
+#pragma unroll
+            for (int k = 0; k < Y16; ++k) {
+                const uint4 v = S.sy[t * Y16 + k];
+                y[4 * k] = v.x; y[4 * k + 1] = v.y; y[4 * k + 2] = v.z; y[4 * k + 3] = v.w;
+            }
+            uint32_t sc[RX];
+#pragma unroll
+            for (int r = 0; r < RX; ++r) {
+                uint32_t D[Dg::n][W];
+#pragma unroll
+                for (int q = 0; q < Dg::n; ++q)
+#pragma unroll
+                    for (int w = 0; w < W; ++w) {
+                        uint32_t d = x[r][w] ^ y[q * NW + w];
+#pragma unroll
+                        for (int p = 1; p < BP; ++p) d |= x[r][p * W + w] ^ y[q * NW + p * W + w];
+                        D[q][w] = d;
+                    }
+                sc[r] = lev_diag<W, E, G>(D) | vmask[r];
+            }
+            if (t < tdiag) {
+                const uint32_t nact = U.ybase + yb + t - U.xbase;   // x-entries before y
+#pragma unroll
+                for (int r = 0; r < RX; ++r)
+                    if ((uint32_t)r * 32 + lane >= nact) sc[r] |= kOff;
+            }
+            uint32_t hit = 0;
+#pragma unroll
+            for (int r = 0; r < RX; ++r) hit |= (uint32_t)(sc[r] == 0) << r;
+            if (hit) S.shq[qn++ * 32 + lane] = (t << 8) | hit;
+            if (__any_sync(0xFFFFFFFFu, qn == (uint32_t)kHitQ)) {
+                __syncwarp();
+                drain_hits(a, ew, S.shq, qn, S.sxm, S.sym, lane, false, is_edge);
+                qn = 0;
+                __syncwarp();
+            }
+        }
+        if (__any_sync(0xFFFFFFFFu, qn)) {
+            __syncwarp();
+            drain_hits(a, ew, S.shq, qn, S.sxm, S.sym, lane, false, is_edge);
+        }
+    }
+    __syncwarp();
+}
+
+// A unit whose x-chunk fills at most one 32-lane block takes the one-block loop.
+template <int BP, int W, int RX, int E, int G>
+__device__ __forceinline__ void lev_unit_rx(const DistArgs &a, EdgeWriter &ew, const Unit &U,
+                                            const LevSlice &S, int lane, uint64_t &pairs) {
+    if (RX > 1 && U.nx <= 32) lev_unit<BP, W, 1, E, G>(a, ew, U, S, lane, pairs);
+    else lev_unit<BP, W, RX, E, G>(a, ew, U, S, lane, pairs);
+}
+
+// Small bin pairs (at most kSmallSide entries a side): a warp each, lanes take
+// pairs and read their records from L1 (the next bin pair's are prefetched).
+template <int BP, int W>
+__device__ __forceinline__ void lev_small_all(const DistArgs &a, EdgeWriter &ew, int lane,
+                                              uint64_t &pairs) {
+    constexpr int R16 = LevShape<BP, W>::R16;
+    const uint32_t n_small = a.ctr->n_small;
+    for (;;) {
+        uint32_t s0 = 0;
+        if (lane == 0) s0 = atomicAdd(&a.ctr->small_cursor, kSmallBatch);
+        s0 = __shfl_sync(0xFFFFFFFFu, s0, 0);
+        if (s0 >= n_small) break;
+        const uint32_t cnt = min(kSmallBatch, n_small - s0);
+        uint32_t myidx = 0;
+        BinPair myP;
+        memset(&myP, 0, sizeof(BinPair));
+        if ((uint32_t)lane < cnt) {
+            myidx = a.small_list[s0 + lane];
+            myP = a.bp[myidx];
+        }
+        for (uint32_t k = 0; k < cnt; ++k) {
+            if (k + 1 < cnt) {
+                const uint32_t na = __shfl_sync(0xFFFFFFFFu, myP.a_start, k + 1);
+                const uint32_t nn = __shfl_sync(0xFFFFFFFFu, myP.a_n, k + 1);
+                const uint32_t nb = __shfl_sync(0xFFFFFFFFu, myP.b_start, k + 1);
+                const uint32_t nm = __shfl_sync(0xFFFFFFFFu, myP.b_n, k + 1);
+                if ((uint32_t)lane < nn) prefetch_l1(a.rec + (size_t)(na + lane) * R16);
+                if ((uint32_t)lane < nm) prefetch_l1(a.rec + (size_t)(nb + lane) * R16);
+            }
+            const BinPair P = shfl_binpair(myP, (int)k);
+            const uint32_t idx = __shfl_sync(0xFFFFFFFFu, myidx, k);
+            const long long t0 = a.bp_cycles ? clock64() : 0;
+            const bool same = P.same != 0;
+            const uint32_t n = P.a_n, npairs = same ? n * (n - 1) / 2 : n * P.b_n;
+            const uint32_t ystart = same ? P.a_start : P.b_start;
+            if (lane == 0) pairs += npairs;
+            uint32_t rmask = 0;           // bit i: the lane's pair of round i is an edge
+            for (uint32_t p0 = 0; p0 < npairs; p0 += 32) {
+                const uint32_t p = p0 + lane;
+                if (p >= npairs) break;
+                uint32_t i, j;
+                small_pair(p, same, n, i, j);
+                if (lev_pair<BP, W>(a.rec + (size_t)(P.a_start + i) * R16,
+                                    a.rec + (size_t)(ystart + j) * R16, (uint32_t)P.eps,
+                                    (uint32_t)(P.lb - P.la)) == 0 &&
+                    canonical_meta(a, P, __ldg(a.meta + P.a_start + i), __ldg(a.meta + ystart + j)))
+                    rmask |= 1u << (p0 >> 5);
+            }
+            __syncwarp();
+            emit_pair_bits(a, ew, lane, rmask, (uint32_t)lane, 32u, same, n, P.a_start, ystart);
+            if (a.bp_cycles && lane == 0)
+                atomicAdd(&a.bp_cycles[idx], (unsigned long long)(clock64() - t0));
+        }
+    }
+}
+
+// Tiny bin pairs: one lane takes every pair of one of them, 32 at a time.
+template <int BP, int W>
+__device__ __forceinline__ void lev_tiny_all(const DistArgs &a, EdgeWriter &ew, int lane,
+                                             uint64_t &pairs) {
+    constexpr int R16 = LevShape<BP, W>::R16;
+    const uint32_t n_tiny = a.ctr->n_tiny;
+    for (;;) {
+        uint32_t s0 = 0;
+        if (lane == 0) s0 = atomicAdd(&a.ctr->tiny_cursor, 32u);
+        s0 = __shfl_sync(0xFFFFFFFFu, s0, 0);
+        if (s0 >= n_tiny) break;
+        const long long t0 = a.bp_cycles ? clock64() : 0;
+        const bool act = s0 + (uint32_t)lane < n_tiny;
+        uint32_t idx = 0;
+        BinPair P;
+        memset(&P, 0, sizeof(BinPair));
+        if (act) {
+            idx = a.small_list[a.small_cap - 1u - (s0 + (uint32_t)lane)];
+            P = a.bp[idx];
+        }
+        const uint32_t n = P.a_n, np = n * (n - 1) / 2;
+        pairs += np;
+        static_assert(kTinySide * (kTinySide - 1) / 2 <= 32, "tiny pair mask");
+        const uint4 *rec = a.rec + (size_t)P.a_start * R16;
+        uint32_t emask = 0;
+        for (uint32_t p = 0; p < np; ++p) {
+            uint32_t i, j;
+            small_pair(p, true, n, i, j);
+            if (lev_pair<BP, W>(rec + (size_t)i * R16, rec + (size_t)j * R16, (uint32_t)P.eps, 0u) == 0 &&
+                canonical_meta(a, P, __ldg(a.meta + P.a_start + i), __ldg(a.meta + P.a_start + j)))
+                emask |= 1u << p;
+        }
+        __syncwarp();
+        emit_pair_bits(a, ew, lane, emask, 0u, 1u, true, n, P.a_start, P.a_start);
+        if (a.bp_cycles) {   // the batch's cycles, shared out by pairs
+            const uint32_t tot = __reduce_add_sync(0xFFFFFFFFu, np);
+            const unsigned long long dt = (unsigned long long)(clock64() - t0);
+            if (act) atomicAdd(&a.bp_cycles[idx], dt * np / (tot ? tot : 1u));
+        }
+    }
+}
+
+template <int BP, int W, int RX>
+__global__ void __launch_bounds__(kWarps * 32, (W <= 2 ? 4 : 3))
+k_lev_diag(DistArgs a) {
+    using Sh = LevShape<BP, W>;
+    __shared__ uint4 sy[kWarps][Sh::YB * Sh::YMax];
+    __shared__ uint4 sym[kWarps][Sh::YB];
+    __shared__ uint4 sxm[kWarps][32 * RX];
+    __shared__ uint32_t shq[kWarps][kHitQ * 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t n_units = a.ctr->n_units, n_bp = a.ctr->n_binpairs;
+    const LevSlice S{sy[wid], sym[wid], sxm[wid], shq[wid]};
+    EdgeWriter ew;
+    ew.init();
+    uint64_t pairs = 0;
+    Unit U;
+    while (next_unit(a, n_units, n_bp, lane, U)) {
+        switch ((uint32_t)U.P.eps * 4 + (uint32_t)(U.P.lb - U.P.la)) {
+            case 0: lev_unit_rx<BP, W, RX, 0, 0>(a, ew, U, S, lane, pairs); break;
+            case 4: lev_unit_rx<BP, W, RX, 1, 0>(a, ew, U, S, lane, pairs); break;
+            case 5: lev_unit_rx<BP, W, RX, 1, 1>(a, ew, U, S, lane, pairs); break;
+            case 8: lev_unit_rx<BP, W, RX, 2, 0>(a, ew, U, S, lane, pairs); break;
+            case 9: lev_unit_rx<BP, W, RX, 2, 1>(a, ew, U, S, lane, pairs); break;
+            case 10: lev_unit_rx<BP, W, RX, 2, 2>(a, ew, U, S, lane, pairs); break;
+            case 12: lev_unit_rx<BP, W, RX, 3, 0>(a, ew, U, S, lane, pairs); break;
+            case 13: lev_unit_rx<BP, W, RX, 3, 1>(a, ew, U, S, lane, pairs); break;
+            case 14: lev_unit_rx<BP, W, RX, 3, 2>(a, ew, U, S, lane, pairs); break;
+            case 15: lev_unit_rx<BP, W, RX, 3, 3>(a, ew, U, S, lane, pairs); break;
+        }
+        log_unit(a, U, lane);
+    }
+    lev_small_all<BP, W>(a, ew, lane, pairs);
+    lev_tiny_all<BP, W>(a, ew, lane, pairs);
+    finish(a, ew, pairs, lane);
+}
+
+template <int BP>
+void launch_lev_diag(const Plan &P, const DistArgs &a, int grid, cudaStream_t s) {
+    switch (P.W) {
+        case 1:
+            if (P.RX == 2) run(k_lev_diag<BP, 1, 2>, a, 0, grid, s);
+            else run(k_lev_diag<BP, 1, 1>, a, 0, grid, s);
+            break;
+        case 2: run(k_lev_diag<BP, 2, 1>, a, 0, grid, s); break;
+        case 3: run(k_lev_diag<BP, 3, 1>, a, 0, grid, s); break;
+        default: run(k_lev_diag<BP, 4, 1>, a, 0, grid, s); break;
+    }
+}
+
+}  // namespace
+}  // namespace idb

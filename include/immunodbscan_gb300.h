@@ -122,7 +122,9 @@ typedef struct idb_stats {
     uint32_t kernel_launches;  /* kernels in the replayed graph; 0 for an eager
                                   call                                             */
     uint32_t core_edges;       /* neighbour pairs with both ends core              */
-    uint64_t lev_columns;      /* text columns consumed by live Levenshtein pairs  */
+    uint64_t lev_columns;      /* text columns consumed by live Levenshtein pairs
+                                  (0 when eps <= 3 everywhere: those pairs are
+                                  decided without a recurrence over columns)      */
     uint32_t candidates;       /* 0: every admissible pair of the buckets scored;
                                   1: Hamming segment join (eps <= 2 at every
                                   length): only pairs sharing a whole segment    */
