@@ -685,9 +685,9 @@ idb_status alloc_fixed(Pipeline &pl) {
         const uint64_t jcap = next_pow2(std::max<uint64_t>(2 * heads, 1024));
         TRY(ensure(c, bJnTab, (sizeof(unsigned long long) + sizeof(uint32_t)) * jcap));
         TRY(ensure(c, bJnISlot, 16 * N1));
-        TRY(ensure(c, bJnStart, 4 * (jcap + 1)));   // group sizes -> starts, per table slot
+        TRY(ensure(c, bJnStart, 4 * jcap));         // group starts, per table slot
         TRY(ensure(c, bJnCur, 4 * (heads + 1)));    // rank of each (unique, segment) in its group
-        TRY(ensure(c, bJnBpIdx, 4 * (jcap + 1)));
+        TRY(ensure(c, bJnBpIdx, 4 * jcap));
         B.jn_key = ptr<unsigned long long>(c, bJnTab);
         B.jn_cnt = reinterpret_cast<uint32_t *>(B.jn_key + jcap);
         B.jn_mask = jcap - 1;
@@ -695,7 +695,6 @@ idb_status alloc_fixed(Pipeline &pl) {
         B.jn_start = ptr<uint32_t>(c, bJnStart);
         B.jn_cur = ptr<uint32_t>(c, bJnCur);
         B.jn_bpidx = ptr<uint32_t>(c, bJnBpIdx);
-        scan_n = std::max<uint64_t>(scan_n, jcap + 1);
     }
     B.scan_part_cap = scan_part_needed(std::max<uint64_t>(scan_n, 1u << 20));
     TRY(ensure(c, bScanPart, 4 * (size_t)B.scan_part_cap));

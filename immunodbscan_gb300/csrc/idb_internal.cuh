@@ -150,7 +150,6 @@ struct Counters {
     uint32_t n_heavy;            // bin pairs the learned predictor evaluates
     uint32_t n_core_edges;       // neighbour pairs with both ends core
     uint32_t n_jslots;           // segment join: table slots in use (the probed prefix)
-    uint32_t n_jslots1;          // n_jslots + 1: the scan of group sizes ends with their total
     uint32_t chunk_uniques[kMaxRowChunks];   // uniques of each row chunk (numbered by chunk)
     uint32_t n_groups;           // segment join: keys held by two or more uniques
     uint32_t n_tiny;             // tiny bin pairs (one lane each), listed from the small list's end
@@ -270,8 +269,8 @@ struct Buffers {
     uint32_t *jn_cnt = nullptr;                     // [jn_mask+1]
     uint64_t jn_mask = 0;
     uint32_t *jn_islot = nullptr;                   // [4*N] slot of (unique, segment)
-    uint32_t *jn_start = nullptr;                   // [jn_mask+2] group size -> start, per table slot
-    uint32_t *jn_bpidx = nullptr;                   // [jn_mask+2] bin pair of a slot's group
+    uint32_t *jn_start = nullptr;                   // [jn_mask+1] first entry of a slot's group, kNone if none
+    uint32_t *jn_bpidx = nullptr;                   // [jn_mask+1] bin pair of a slot's group
     uint32_t *jn_cur = nullptr;                     // [join_smax*N] rank of (unique, segment) in its group
     uint32_t *cls_hist = nullptr;                   // [65]
     float *pred = nullptr;                          // learned cost per bin pair

@@ -559,10 +559,7 @@ __global__ void k_join_clear(Counters *ctr, uint32_t smax, uint64_t cap_mask,
                              unsigned long long *__restrict__ key, uint32_t *__restrict__ cnt,
                              uint32_t rows) {
     const uint32_t n = join_mask(rows ? rows : ctr->n_uniques, smax, cap_mask) + 1u;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        ctr->n_jslots = n;
-        ctr->n_jslots1 = n + 1;
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctr->n_jslots = n;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         key[i] = ~0ull;
@@ -631,54 +628,60 @@ k_join_insert(BinGeom g, Counters *ctr, const uint32_t *__restrict__ urow,
     }
 }
 
-// Size of every key's group, per table slot (0 for an empty slot and for a
-// key held by one unique), and the bin-pair index of the slots that hold
-// groups.  A sequential pass over the probed prefix of the table, four slots
-// per thread (16-byte loads and stores), with one counter atomic per block and
-// pass of 4 x 256 slots (the counter's atomics bounded the pass at one slot per
-// thread).
+// Groups: every slot whose key two or more uniques hold gets a place for its
+// entries and a bin-pair index (kNone / unset otherwise).  Any order of the
+// groups gives the same neighbour pairs, so a block takes the places of its
+// 4 x 256 slots with two counter atomics and one block scan, in one pass over
+// the counts; a device-wide scan in slot order cost three passes more (2.5M
+// rows: 1.472 against 1.456 ms a call).  Four slots per thread (16-byte loads and stores).
 __global__ void __launch_bounds__(256)
-k_join_sizes(Counters *ctr, const uint32_t *__restrict__ tcnt, uint32_t *__restrict__ sizes,
-             uint32_t *__restrict__ bpidx) {
-    __shared__ uint32_t s_w[8];
-    __shared__ uint32_t s_base;
-    const uint32_t ns = ctr->n_jslots;
+k_join_groups(Counters *ctr, const uint32_t *__restrict__ tcnt, uint32_t *__restrict__ start,
+              uint32_t *__restrict__ bpidx) {
+    __shared__ uint2 s_w[8];
+    __shared__ uint2 s_base;
+    const uint32_t ns = ctr->n_jslots;   // a power of two >= 1024: whole blocks of slots
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t stride = 4 * gridDim.x * blockDim.x;
-    if (blockIdx.x == 0 && threadIdx.x == 0) sizes[ns] = 0u;   // the scan's end: the total
     for (uint32_t h0 = 4 * blockIdx.x * blockDim.x; h0 < ns; h0 += stride) {
         const uint32_t h = h0 + 4 * threadIdx.x;
-        uint32_t c[4] = {0u, 0u, 0u, 0u};
-        if (h + 4 <= ns) {   // the probed prefix is a power of two >= 1024: whole quads
-            const uint4 v = *reinterpret_cast<const uint4 *>(tcnt + h);
-            c[0] = v.x; c[1] = v.y; c[2] = v.z; c[3] = v.w;
-        }
-        uint32_t mine = 0;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (c[k] < 2) c[k] = 0;
-            mine += c[k] != 0;
-        }
-        if (h + 4 <= ns) *reinterpret_cast<uint4 *>(sizes + h) = make_uint4(c[0], c[1], c[2], c[3]);
-        // rank of this thread's groups in the block: warp scan, then warp sums
-        uint32_t incl = mine;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-            if (lane >= (uint32_t)d) incl += t;
-        }
-        if (lane == 31) s_w[wid] = incl;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t t = 0;
-            for (uint32_t w = 0; w < blockDim.x / 32; ++w) { const uint32_t x = s_w[w]; s_w[w] = t; t += x; }
-            s_base = t ? atomicAdd(&ctr->n_groups, t) : 0u;
-        }
-        __syncthreads();
-        uint32_t idx = s_base + s_w[wid] + incl - mine;
+        const uint4 v = *reinterpret_cast<const uint4 *>(tcnt + h);
+        const uint32_t c[4] = {v.x, v.y, v.z, v.w};
+        uint32_t groups = 0, entries = 0;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if (c[k]) bpidx[h + k] = idx++;
+            if (c[k] >= 2) { ++groups; entries += c[k]; }
+        uint32_t gi = groups, ei = entries;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t tg = __shfl_up_sync(0xFFFFFFFFu, gi, d);
+            const uint32_t te = __shfl_up_sync(0xFFFFFFFFu, ei, d);
+            if (lane >= (uint32_t)d) { gi += tg; ei += te; }
+        }
+        if (lane == 31) s_w[wid] = make_uint2(gi, ei);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            uint32_t tg = 0, te = 0;
+            for (uint32_t w = 0; w < blockDim.x / 32; ++w) {
+                const uint2 x = s_w[w];
+                s_w[w] = make_uint2(tg, te);
+                tg += x.x;
+                te += x.y;
+            }
+            if (tg) s_base = make_uint2(atomicAdd(&ctr->n_groups, tg), atomicAdd(&ctr->n_entries, te));
+        }
+        __syncthreads();
+        uint32_t idx = s_base.x + s_w[wid].x + gi - groups, pos = s_base.y + s_w[wid].y + ei - entries;
+        uint32_t st[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            st[k] = kNone;
+            if (c[k] >= 2) {
+                bpidx[h + k] = idx++;
+                st[k] = pos;
+                pos += c[k];
+            }
+        }
+        *reinterpret_cast<uint4 *>(start + h) = make_uint4(st[0], st[1], st[2], st[3]);
         __syncthreads();
     }
 }
@@ -713,7 +716,7 @@ k_join_fill(BinGeom g, const Counters *__restrict__ ctr, const uint32_t *__restr
             const uint32_t sl = islot[(size_t)u * 4 + k];
             if (sl == kNone) continue;
             const uint32_t s0 = start[sl];
-            if (start[sl + 1] - s0 < 2) continue;              // a key of one unique: no group
+            if (s0 == kNone) continue;                         // a key of one unique: no group
             const uint64_t pos = (uint64_t)s0 + irank[(size_t)u * smax + k];
             if (pos >= cap_entries) { atomicOr(err, kErrEntryOverflow); continue; }
             // side record (its unique id is the entry's: the join's distance
@@ -736,20 +739,20 @@ __global__ void k_join_nbp(Counters *ctr) {
 // One bin pair (a group against itself) per key held by two or more uniques:
 // a sequential pass over the probed prefix of the table.
 __global__ void k_join_bp_fill(BinGeom g, const Counters *__restrict__ ctr,
-                               const unsigned long long *__restrict__ tkey, const uint32_t *__restrict__ start,
-                               const uint32_t *__restrict__ bpidx, const int16_t *__restrict__ eps_tab,
+                               const unsigned long long *__restrict__ tkey, const uint32_t *__restrict__ tcnt,
+                               const uint32_t *__restrict__ start, const uint32_t *__restrict__ bpidx, const int16_t *__restrict__ eps_tab,
                                uint32_t TX, uint64_t cap_bp, BinPair *__restrict__ out, uint32_t *err) {
     const uint32_t ns = ctr->n_jslots;   // a power of two >= 1024: whole quads of slots
     const uint32_t stride = 4 * gridDim.x * blockDim.x;
     for (uint32_t h0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x); h0 < ns; h0 += stride) {
-        // four slots a thread: their starts in one 16-byte load, and the next
-        // quad's first start (start has ns + 1 entries)
+        // four slots a thread: their starts in one 16-byte load
         const uint4 v = *reinterpret_cast<const uint4 *>(start + h0);
-        const uint32_t sv[5] = {v.x, v.y, v.z, v.w, start[h0 + 4]};
+        const uint32_t sv[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (uint32_t q = 0; q < 4; ++q) {
-            const uint32_t h = h0 + q, s0 = sv[q], c = sv[q + 1] - s0;
-            if (c < 2) continue;
+            const uint32_t h = h0 + q, s0 = sv[q];
+            if (s0 == kNone) continue;
+            const uint32_t c = tcnt[h];
             const uint32_t k = bpidx[h];
             if (k >= cap_bp) { atomicOr(err, kErrBinPairOverflow); continue; }
             const unsigned long long key = tkey[h];
@@ -774,7 +777,7 @@ __global__ void k_join_bp_fill(BinGeom g, const Counters *__restrict__ ctr,
 }  // namespace
 
 void launch_join_init(const Plan &P, const Buffers &B, cudaStream_t s) {
-    cudaMemsetAsync(&B.ctr->n_jslots, 0, 2 * sizeof(uint32_t), s);   // n_jslots, n_groups
+    cudaMemsetAsync(&B.ctr->n_groups, 0, sizeof(uint32_t), s);
     k_join_clear<<<grid_wave(k_join_clear, B.jn_mask + 1, kThreads), kThreads, 0, s>>>(
         B.ctr, P.join_smax, B.jn_mask, B.jn_key, B.jn_cnt, P.front_join ? P.N : 0u);
 }
@@ -796,10 +799,9 @@ void launch_buckets(const Plan &P, const Buffers &B, cudaStream_t s) {
             launch_join_init(P, B, s);
             launch_join_insert(P, B, -1, s);
         }
-        k_join_sizes<<<grid_wave(k_join_sizes, slots, kThreads), kThreads, 0, s>>>(
+        cudaMemsetAsync(&B.ctr->n_entries, 0, sizeof(uint32_t), s);
+        k_join_groups<<<grid_wave(k_join_groups, slots / 4, kThreads), kThreads, 0, s>>>(
             B.ctr, B.jn_cnt, B.jn_start, B.jn_bpidx);
-        scan_u32(B.jn_start, B.jn_start, (uint32_t)slots + 1, &B.ctr->n_jslots1, &B.ctr->n_entries,
-                 B.scan_part, B.scan_part_cap, s);
         return;
     }
     const uint32_t nb = (uint32_t)P.nbins;
@@ -881,8 +883,8 @@ void launch_binpairs(const Plan &P, const Buffers &B, cudaStream_t s) {
 void launch_binpairs_fill(const Plan &P, const Buffers &B, cudaStream_t s) {
     if (P.join) {
         BinGeom g{P.Gv, P.Gj, P.NL, P.Lmin, P.VW, P.JW, P.K};
-        k_join_bp_fill<<<grid_wave(k_join_bp_fill, B.jn_mask + 1, kThreads), kThreads, 0, s>>>(
-            g, B.ctr, B.jn_key, B.jn_start, B.jn_bpidx, B.eps_tab, P.TX, P.cap_binpairs, B.bp,
+        k_join_bp_fill<<<grid_wave(k_join_bp_fill, (B.jn_mask + 1) / 4, kThreads), kThreads, 0, s>>>(
+            g, B.ctr, B.jn_key, B.jn_cnt, B.jn_start, B.jn_bpidx, B.eps_tab, P.TX, P.cap_binpairs, B.bp,
             &B.ctr->error);
         return;
     }
