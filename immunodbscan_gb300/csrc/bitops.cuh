@@ -143,11 +143,11 @@ IDB_HD int myers_distance(const uint8_t *p, int m, const uint8_t *t, int n) {
 // E_{d-1} (a character of y skipped) and G_{d+1} (a character of x skipped);
 // the union of prefix masks is the longest, so merging is an OR.  Returns 0 iff
 // diagonal G is passed to its end after E edits.
-// Positions past an end need no masking for LO <= 1 (E <= 3): both strings
-// are padded with the same code, so diagonal G matches there; on a lower
-// diagonal x is exhausted and more prefix gains nothing; on diagonal G + 1 only
-// the last position of x lies past y's end, and passing it for free costs the
-// same one edit (skipping it) on the way back to diagonal G.
+// Positions past an end need no masking.  Both strings are padded with the same
+// code, so diagonal G matches there; on a diagonal d < G x is exhausted and more
+// prefix gains nothing; on a diagonal d > G the last d - G positions of x lie
+// past y's end, and passing them for free saves nothing: the d - G edits (each
+// skipping a character of x) back to diagonal G are due either way.
 // ---------------------------------------------------------------------------
 template <int E, int G>
 struct LevDiags {

@@ -30,6 +30,7 @@ struct DistArgs {
     // segment join: a hit is a neighbour pair if the V and J sets intersect and
     // no lower segment is identical (that segment's group emits it)
     int join;
+    int vj_meta;                     // the join's side records hold the V and J bits
     // where neighbour pairs go: kSinkEdges = the edge list; kSinkCount /
     // kSinkGrow = the two sweeps of the streamed mode (no edge list kept)
     uint32_t sink;
@@ -195,6 +196,12 @@ __device__ __forceinline__ bool canonical(const DistArgs &a, const BinPair &P, u
     const uint32_t rx = a.urow[ux], ry = a.urow[uy];
     return lowest_common(a.vbits, a.VW, rx, ry) == (int)P.v &&
            lowest_common(a.jbits, a.JW, rx, ry) == (int)P.j;
+}
+
+// V and J sets of two uniques (by id) intersect.
+__device__ __forceinline__ bool vj_intersect(const DistArgs &a, uint32_t ux, uint32_t uy) {
+    const uint32_t rx = a.urow[ux], ry = a.urow[uy];
+    return lowest_common(a.vbits, a.VW, rx, ry) >= 0 && lowest_common(a.jbits, a.JW, rx, ry) >= 0;
 }
 
 // The same from the side records: {V genes below the bin's V gene (64 bits), J

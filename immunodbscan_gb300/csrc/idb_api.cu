@@ -71,7 +71,7 @@ enum BufId {
     bBpSorted, bBpUnits, bClsHist, bPred, bEdges, bCnt, bUCore,
     bParent, bBMin, bRootFlag, bUidFirst, bDepth, bScanPart, bClone, bCore, bCopies, bUniques,
     bCtr, bVTab, bJTab, bSigAnd, bUClass, bEntMeta, bCallAux, bCallTab, bCallRef, bCallTodo, bBpSmall,
-    bJnTab, bJnISlot, bJnStart, bJnCur, bJnBpIdx, bNumBufs
+    bJnTab, bJnISlot, bJnStart, bJnCur, bJnBpIdx, bJnPos, bNumBufs
 };
 
 }  // namespace
@@ -331,6 +331,7 @@ struct Pipeline {
     // that a replay copies them to the host while the rest of the path runs
     bool early_out = false;
     bool copies_issued = false;
+    bool own_shape = true;    // the caller asked for no unit shape
     bool allow_join = true;   // the segment join finds neighbours, not all admissible pairs
     // every return path (errors included) leaves no copy from the caller's host
     // buffers in flight
@@ -578,6 +579,7 @@ idb_status derive_plan(Pipeline &pl, const idb_params *prm) {
         P.TY = 256;
     }
     if (P.fast) apply_shape(P, prm->tile_rx, prm->tile_ty);
+    pl.own_shape = prm->tile_rx <= 0 && prm->tile_ty <= 0;
     P.dLmax = P.hamming ? 0 : dl;
     P.hamming_eps_mode = 0;
     if (P.hamming && emin_same == emax_same && emin_same == 1) P.hamming_eps_mode = 1;
@@ -592,9 +594,18 @@ idb_status derive_plan(Pipeline &pl, const idb_params *prm) {
              P.Gv <= 64 && P.Gj <= 30 && P.R < (1u << 24) - 1 &&
              2ull * (uint64_t)(emax_same + 1) * P.N <= (1ull << 30);
     P.join_smax = P.join ? (uint32_t)std::max(1, emax_same + 1) : 1u;
+    P.join_classes = 1;
+    P.vj_meta = P.Gv <= 64 && P.Gj <= 30;
+    if (pl.allow_join && prm->candidates == 0 && P.lev_diag && P.R < (1u << 24) - 1) {
+        // Levenshtein: the join too (an eager call may still take the buckets,
+        // choose_candidates); the table and its class counts stay below 2^31
+        P.join_smax = (uint32_t)std::max(1, emax_same + 1);
+        P.join_classes = (uint32_t)P.dLmax + 2;
+        P.join = next_pow2(std::max<uint64_t>(2ull * P.join_smax * P.N, 1024)) * P.join_classes <= (1ull << 31);
+    }
     // with row chunks the uniques are numbered and the join's inserts run chunk
     // by chunk, while later chunks are still being copied
-    P.front_join = P.join && P.nchunks > 1;
+    P.front_join = P.join && P.hamming && P.nchunks > 1;
     if (P.hamming && P.RX == 2 && !P.join) {   // 2 x-entries per lane: segment join only
         P.RX = 4;
         P.TX = 128;
@@ -602,7 +613,7 @@ idb_status derive_plan(Pipeline &pl, const idb_params *prm) {
     }
     // segment join without a requested shape: 2 x-entries per lane, 512 y-entries
     // (its groups are mostly small: narrower x-chunks leave fewer lanes idle)
-    if (P.join && P.W == 1 && prm->tile_rx <= 0) {
+    if (P.join && P.hamming && P.W == 1 && prm->tile_rx <= 0) {
         P.RX = 2;
         P.TX = 64;
         if (prm->tile_ty <= 0) P.TY = 512;
@@ -670,7 +681,7 @@ idb_status alloc_fixed(Pipeline &pl) {
     TRY(ensure(c, bSigAnd, 16 * (P.nbins + 1)));
     TRY(ensure(c, bUClass, 4 * N1));
     TRY(ensure(c, bBpCount, 4 * (P.nbins + 1)));
-    TRY(ensure(c, bClsHist, 4 * 130));
+    TRY(ensure(c, bClsHist, 4 * 2 * kSchedBins));
     TRY(ensure(c, bCnt, 4 * N1));
     TRY(ensure(c, bUCore, 4 * N1));
     TRY(ensure(c, bParent, 4 * N1));
@@ -683,7 +694,11 @@ idb_status alloc_fixed(Pipeline &pl) {
         // keys: at most join_smax per unique; the table at load <= 1/2
         const uint64_t heads = (uint64_t)P.join_smax * N;
         const uint64_t jcap = next_pow2(std::max<uint64_t>(2 * heads, 1024));
-        TRY(ensure(c, bJnTab, (sizeof(unsigned long long) + sizeof(uint32_t)) * jcap));
+        TRY(ensure(c, bJnTab, (sizeof(unsigned long long) + sizeof(uint32_t) * P.join_classes) * jcap));
+        if (!P.hamming) {
+            TRY(ensure(c, bJnPos, 4 * (size_t)P.join_classes * jcap));
+            B.jn_pos = ptr<uint32_t>(c, bJnPos);
+        }
         TRY(ensure(c, bJnISlot, 16 * N1));
         TRY(ensure(c, bJnStart, 4 * jcap));         // group starts, per table slot
         TRY(ensure(c, bJnCur, 4 * (heads + 1)));    // rank of each (unique, segment) in its group
@@ -829,6 +844,49 @@ idb_status launch_front(Pipeline &pl, cudaStream_t s) {
     return IDB_OK;
 }
 
+// Unit shape of the edit-distance join: the largest of 64 x 256 down to 32 x 64
+// pairs that leaves about four units per resident warp (16 an SM), so that a
+// few dense groups do not end as one long unit each (20k rows, 0.6M pairs: 889 us
+// in 64 x 256 units).
+void set_join_shape(Plan &P, uint64_t pairs) {
+    const uint64_t want = pairs / ((uint64_t)sm_count() * 16 * 4);
+    P.RX = P.W == 1 && want >= 64 * 64 ? 2 : 1;
+    P.TX = 32 * P.RX;
+    P.TY = 64;
+    while (P.TY < 256 && (uint64_t)P.TX * P.TY * 2 <= want) P.TY *= 2;
+}
+
+// After launch_buckets of an eager call with the edit-distance join: entries are
+// allocated for the join, or for the buckets where those score fewer pairs.  A
+// join pair costs about what a bucket pair does (the same test; its hits a few
+// look-ups more), and the join scores fewer pairs unless most of them share
+// segments (tiny alphabets, or one dense family), so the buckets are only
+// counted when the join's pairs are many.
+idb_status choose_candidates(Pipeline &pl) {
+    idb_context *c = pl.c;
+    Plan &P = pl.P;
+    Buffers &B = pl.B;
+    cudaStream_t s = c->stream;
+    TRY(read_counters(pl));
+    if (P.join && !P.hamming && c->h_ctr->join_pairs > kJoinSurePairs) {
+        const uint32_t join_entries = c->h_ctr->n_entries;
+        const unsigned long long join_pairs = c->h_ctr->join_pairs;
+        P.join = false;
+        launch_buckets(P, B, s);
+        launch_bucket_pairs(P, B, s);
+        TRY(check_launch());
+        TRY(read_counters(pl));
+        if (join_pairs <= c->h_ctr->bucket_pairs) {
+            P.join = true;
+            c->h_ctr->n_entries = join_entries;
+            CU(cudaMemcpyAsync(&B.ctr->n_entries, &c->h_ctr->n_entries, sizeof(uint32_t),
+                               cudaMemcpyHostToDevice, s));
+        }
+    }
+    if (P.join && !P.hamming && pl.own_shape) set_join_shape(P, c->h_ctr->join_pairs);
+    return alloc_entries(pl, c->h_ctr->n_entries);
+}
+
 idb_status run_phases(Pipeline &pl, bool eager, bool stop_after_schedule = false) {
     idb_context *c = pl.c;
     Plan &P = pl.P;
@@ -843,10 +901,7 @@ idb_status run_phases(Pipeline &pl, bool eager, bool stop_after_schedule = false
     TRY(check_launch());
     record(pl, 1);
     launch_buckets(P, B, s);
-    if (eager) {
-        TRY(read_counters(pl));
-        TRY(alloc_entries(pl, c->h_ctr->n_entries));
-    }
+    if (eager) TRY(choose_candidates(pl));
     launch_fill(P, B, s);
     launch_binpairs(P, B, s);
     TRY(check_launch());
@@ -1777,8 +1832,7 @@ idb_status idb_autotune(idb_context *c, const idb_input *in, const idb_params *p
     // front and buckets once (independent of the unit shape)
     TRY(launch_front(pl, s));
     launch_buckets(P, B, s);
-    TRY(read_counters(pl));
-    TRY(alloc_entries(pl, c->h_ctr->n_entries));
+    TRY(choose_candidates(pl));
     launch_fill(P, B, s);
     TRY(check_launch());
     // candidate shapes

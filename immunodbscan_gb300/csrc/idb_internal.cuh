@@ -23,6 +23,7 @@ constexpr uint32_t kSmallSide = 32;
 // A bin paired with itself with at most kTinySide entries is a tiny bin pair:
 // one lane takes all of its pairs, 32 tiny bin pairs per warp at once.
 constexpr uint32_t kTinySide = 8;
+constexpr uint32_t kTinyPairs = kTinySide * (kTinySide - 1) / 2;
 // Hamming with eps <= kJoinMaxEps for every length uses the segment join: two
 // equal-length sequences within eps agree exactly on one of eps+1 segments.
 // At eps 3 the quarter-length segments make groups large enough that the
@@ -32,6 +33,12 @@ constexpr int kJoinMaxEps = 2;
 // Levenshtein with eps <= kLevDiagMaxEps at every admissible length pair uses the
 // diagonal test (bitops.cuh); above that its cost per pair grows with eps^2.
 constexpr int kLevDiagMaxEps = 3;
+constexpr uint32_t kSchedVariants = 16; // loops of the edit-distance kernel told apart by the schedule
+constexpr uint32_t kSchedBins = 64 * kSchedVariants;
+// Candidate pairs up to which an eager call takes the edit-distance join without
+// counting the buckets' pairs for comparison: scoring that many takes about as
+// long as the count (0.2 ms).
+constexpr unsigned long long kJoinSurePairs = 1ull << 27;
 constexpr int kMlpIn = 16;              // learned scheduler: features per bin pair
 constexpr int kMlpHidden = 64;          // two hidden layers of 64
 constexpr int kMlpParams = kMlpIn * kMlpHidden + kMlpHidden + kMlpHidden * kMlpHidden + kMlpHidden +
@@ -151,7 +158,9 @@ struct Counters {
     uint32_t n_core_edges;       // neighbour pairs with both ends core
     uint32_t n_jslots;           // segment join: table slots in use (the probed prefix)
     uint32_t chunk_uniques[kMaxRowChunks];   // uniques of each row chunk (numbered by chunk)
-    uint32_t n_groups;           // segment join: keys held by two or more uniques
+    uint32_t n_groups;           // segment join: bin pairs of the groups
+    unsigned long long join_pairs;    // edit-distance join: candidate pairs of its groups
+    unsigned long long bucket_pairs;  // pairs of the buckets (an upper bound), when compared with it
     uint32_t n_tiny;             // tiny bin pairs (one lane each), listed from the small list's end
     uint32_t tiny_cursor;        // their work queue head
 };
@@ -199,7 +208,11 @@ struct Plan {
     bool lev_diag = false;                        // Levenshtein by the diagonal test
     // records are bit planes (else one code byte per residue)
     bool planes() const { return fast && (hamming || lev_diag); }
-    bool join = false;                            // Hamming by segment join (eps <= kJoinMaxEps)
+    bool join = false;                            // candidates by segment join (Hamming with eps <=
+                                                  // kJoinMaxEps; Levenshtein by the diagonal test)
+    uint32_t join_classes = 1;                    // counts per table slot (Levenshtein: the indexed
+                                                  // uniques, then one per length gap and shift)
+    bool vj_meta = true;                          // side records of the join hold the V and J bits
     uint32_t join_smax = 1;                       // most segments of any length
     bool streamed = false;                        // neighbour pairs not stored: the
                                                   // distance work runs twice
@@ -266,13 +279,14 @@ struct Buffers {
     // many (unique, segment) entries hold each key, so that the passes over
     // the slots read 4 bytes per slot
     unsigned long long *jn_key = nullptr;           // [jn_mask+1]
-    uint32_t *jn_cnt = nullptr;                     // [jn_mask+1]
+    uint32_t *jn_cnt = nullptr;                     // [(jn_mask+1) * join_classes]
+    uint32_t *jn_pos = nullptr;                     // the same, Levenshtein: next entry of each class
     uint64_t jn_mask = 0;
     uint32_t *jn_islot = nullptr;                   // [4*N] slot of (unique, segment)
     uint32_t *jn_start = nullptr;                   // [jn_mask+1] first entry of a slot's group, kNone if none
     uint32_t *jn_bpidx = nullptr;                   // [jn_mask+1] bin pair of a slot's group
     uint32_t *jn_cur = nullptr;                     // [join_smax*N] rank of (unique, segment) in its group
-    uint32_t *cls_hist = nullptr;                   // [65]
+    uint32_t *cls_hist = nullptr;                   // [2*kSchedBins] schedule bins, then cursors
     float *pred = nullptr;                          // learned cost per bin pair
     // graph
     uint2 *edges = nullptr;                         // [cap_edges]
@@ -321,6 +335,12 @@ void launch_buckets(const Plan &P, const Buffers &B, cudaStream_t s);
 // inserts of every unique (chunk < 0) or of one row chunk's uniques
 void launch_join_init(const Plan &P, const Buffers &B, cudaStream_t s);
 void launch_join_insert(const Plan &P, const Buffers &B, int chunk, cudaStream_t s);
+// edit-distance join (k_lev_join.cu): table, look-ups and group places; entries; bin pairs
+void launch_lev_join(const Plan &P, const Buffers &B, cudaStream_t s);
+void launch_lev_join_fill(const Plan &P, const Buffers &B, cudaStream_t s);
+void launch_lev_join_binpairs(const Plan &P, const Buffers &B, cudaStream_t s);
+// after launch_buckets without the join: ctr->bucket_pairs
+void launch_bucket_pairs(const Plan &P, const Buffers &B, cudaStream_t s);
 void launch_binpairs(const Plan &P, const Buffers &B, cudaStream_t s);
 void launch_schedule(const Plan &P, const Buffers &B, cudaStream_t s);
 void launch_distance(const Plan &P, const Buffers &B, int grid, cudaStream_t s,

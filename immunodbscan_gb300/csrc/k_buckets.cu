@@ -24,8 +24,9 @@
 //
 // Hamming with eps <= 2 at every length takes its candidates from a segment
 // join instead (the k_join_* kernels below): groups of uniques that share one
-// whole segment of eps+1, which every neighbour pair does (pigeonhole).
-#include "idb_internal.cuh"
+// whole segment of eps+1, which every neighbour pair does (pigeonhole).  Edit
+// distances up to 3 have a join of their own (k_lev_join.cu).
+#include "records.cuh"
 
 namespace idb {
 
@@ -40,16 +41,6 @@ inline int grid_for(uint64_t n, int threads = kThreads) {
     if (g < 1) g = 1;
     return (int)g;
 }
-
-struct BinGeom {
-    uint32_t Gv, Gj, NL, Lmin, VW, JW, K;
-    __device__ __forceinline__ bool in_range(uint32_t L) const { return L >= Lmin && L - Lmin < NL; }
-    // sub-bucket index: ((((r*Gv + v)*Gj + j)*NL + L-Lmin)*K + class
-    __device__ __forceinline__ uint32_t bin(uint32_t r, uint32_t v, uint32_t j, uint32_t L,
-                                            uint32_t c) const {
-        return (((r * Gv + v) * Gj + j) * NL + (L - Lmin)) * K + c;
-    }
-};
 
 // genes of `bits` (first word) below gene index g
 __device__ __forceinline__ uint64_t below(uint64_t word0, uint32_t g) {
@@ -151,88 +142,6 @@ __global__ void k_bin_hist(BinGeom g, const Counters *__restrict__ ctr,
                     }
                 }
             }
-        }
-    }
-}
-
-// Record of one unique.
-//  planes (fast path; Hamming and the diagonal edit-distance test): Bp bit planes x W words; bit i of word
-//    p*W + i/32 is bit p of the code of residue i.  Hamming distance of two
-//    records = sum over words of popc(OR_p (x_p ^ y_p)).
-//  codes (other Levenshtein and the generic path): one code byte per residue.
-// Codes are a bijection of the byte values present, so equality of codes is
-// equality of bytes.
-// The record of one unique (fast paths: at most NR 16-byte words): bit planes
-// or code bytes, residues read 4 at a time.
-// Bit planes of one sequence (L <= 128): bit i of wd[p][w] is bit p of the
-// code of residue 32w + i; positions past L keep code 0.  Residues are read 4
-// at a time.
-__device__ __forceinline__ void build_planes(const uint8_t *s, uint32_t L, const uint8_t *cm,
-                                             uint32_t (&wd)[5][4]) {
-#pragma unroll
-    for (int p = 0; p < 5; ++p)
-#pragma unroll
-        for (int w = 0; w < 4; ++w) wd[p][w] = 0;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-        if (32u * w >= L) break;
-        uint32_t cw[8];
-        load_chunk32(s, L, (uint32_t)w, cw);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const uint32_t i0 = 32u * w + 4u * k;
-            const uint32_t v = cw[k];
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const uint32_t c = i0 + b < L ? (uint32_t)cm[(v >> (8 * b)) & 0xFFu] : 0u;
-#pragma unroll
-                for (int p = 0; p < 5; ++p) wd[p][w] |= ((c >> p) & 1u) << (4 * k + b);
-            }
-        }
-    }
-}
-
-template <int NR>
-__device__ __forceinline__ void build_small_record(const uint8_t *s, uint32_t L,
-                                                   const uint8_t *cm, int planes, uint32_t W,
-                                                   uint4 (&rec)[NR]) {
-    if (planes > 0) {
-        uint32_t wd[5][4];
-        build_planes(s, L, cm, wd);
-        // layout: word p*W + w
-        uint32_t flat[4 * NR];
-#pragma unroll
-        for (int k = 0; k < 4 * NR; ++k) flat[k] = 0;
-#pragma unroll
-        for (int p = 0; p < 5; ++p)
-#pragma unroll
-            for (int w = 0; w < 4; ++w)
-                if (p < planes && (uint32_t)w < W) {
-                    const uint32_t k = (uint32_t)p * W + w;
-#pragma unroll
-                    for (int kk = 0; kk < 4 * NR; ++kk)
-                        if ((uint32_t)kk == k) flat[kk] = wd[p][w];
-                }
-#pragma unroll
-        for (int q = 0; q < NR; ++q) rec[q] = make_uint4(flat[4 * q], flat[4 * q + 1], flat[4 * q + 2], flat[4 * q + 3]);
-    } else {
-        GlobalReader rd(s, L);
-#pragma unroll
-        for (int q = 0; q < NR; ++q) {
-            uint32_t wv[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const uint32_t i0 = q * 16 + e * 4;
-                const uint32_t v = i0 < L ? rd.next() : 0u;
-                uint32_t acc = 0;
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const uint32_t c = i0 + t < L ? (uint32_t)cm[(v >> (8 * t)) & 0xFFu] : 0u;
-                    acc |= c << (8 * t);
-                }
-                wv[e] = acc;
-            }
-            rec[q] = make_uint4(wv[0], wv[1], wv[2], wv[3]);
         }
     }
 }
@@ -416,12 +325,41 @@ __global__ void k_binpairs_fill(uint32_t nsub, PairGeom pg, const int16_t *__res
         visit_pairs<true>(sb, pg, eps_tab, bin_start, sig, out, bp_off[sb], cap_bp, err);
 }
 
+// Pairs of the buckets, before the signatures leave any out.
+__global__ void k_bucket_pairs(uint32_t nsub, PairGeom pg, const int16_t *__restrict__ eps_tab,
+                               const uint32_t *__restrict__ bin_start, unsigned long long *total) {
+    const uint32_t stride = gridDim.x * blockDim.x;
+    unsigned long long pairs = 0;
+    for (uint32_t sb = blockIdx.x * blockDim.x + threadIdx.x; sb < nsub; sb += stride) {
+        const unsigned long long nA = bin_start[sb + 1] - bin_start[sb];
+        if (nA == 0) continue;
+        const uint32_t b = sb / pg.K, li = b % pg.NL;
+        for (int g = 0; g <= pg.dLmax; ++g) {
+            if (!pair_ok(pg, eps_tab, li, g)) continue;
+            // the K classes of a bin are neighbours: from class c on for g = 0
+            const uint32_t first = (b + g) * pg.K;
+            const unsigned long long nB = bin_start[first + pg.K] - bin_start[g == 0 ? sb + 1 : first];
+            pairs += nA * nB + (g == 0 ? nA * (nA - 1) / 2 : 0);
+        }
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) pairs += __shfl_xor_sync(0xFFFFFFFFu, pairs, d);
+    if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(total, pairs);
+}
+
 // Schedule: heavy bin pairs first (counting sort on log2 of the cost, cost =
-// pairs for the static schedule or the predicted cost for the learned one).
+// pairs for the static schedule or the predicted cost for the learned one), and
+// among equals by (eps, length gap): the edit-distance kernel has a loop for each,
+// and warps that run the same one share the instruction cache.
+__device__ __forceinline__ uint32_t sched_bin(const BinPair &P, uint32_t cls, int by_loop) {
+    const uint32_t v = by_loop ? ((uint32_t)P.eps * 4 + (uint32_t)(P.lb - P.la)) & (kSchedVariants - 1) : 0u;
+    return (63 - cls) * kSchedVariants + v;
+}
+
 __global__ void k_cls_hist(const Counters *__restrict__ ctr, const BinPair *__restrict__ bp,
-                           const float *__restrict__ pred, uint32_t *__restrict__ hist) {
-    __shared__ uint32_t h[64];
-    if (threadIdx.x < 64) h[threadIdx.x] = 0;
+                           const float *__restrict__ pred, uint32_t *__restrict__ hist, int by_loop) {
+    __shared__ uint32_t h[kSchedBins];
+    for (uint32_t k = threadIdx.x; k < kSchedBins; k += blockDim.x) h[k] = 0;
     __syncthreads();
     const uint32_t n = ctr->n_binpairs;
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -431,10 +369,11 @@ __global__ void k_cls_hist(const Counters *__restrict__ ctr, const BinPair *__re
             const float c = fmaxf(pred[i], 1.0f);
             cls = min(63u, (uint32_t)(log2f(c) * 2.0f));
         }
-        atomicAdd(&h[63 - cls], 1u);
+        atomicAdd(&h[sched_bin(bp[i], cls, by_loop)], 1u);
     }
     __syncthreads();
-    if (threadIdx.x < 64 && h[threadIdx.x]) atomicAdd(&hist[threadIdx.x], h[threadIdx.x]);
+    for (uint32_t k = threadIdx.x; k < kSchedBins; k += blockDim.x)
+        if (h[k]) atomicAdd(&hist[k], h[k]);
 }
 
 __global__ void k_cls_scatter(const Counters *__restrict__ ctr, const BinPair *__restrict__ bp,
@@ -443,7 +382,7 @@ __global__ void k_cls_scatter(const Counters *__restrict__ ctr, const BinPair *_
                               uint32_t *__restrict__ units, uint32_t TX, uint32_t TY, uint32_t q,
                               int small_mode, uint32_t *__restrict__ small_list,
                               uint32_t *__restrict__ n_small, uint32_t *__restrict__ n_tiny,
-                              uint32_t small_cap) {
+                              uint32_t small_cap, int by_loop) {
     const uint32_t n = ctr->n_binpairs;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -453,21 +392,22 @@ __global__ void k_cls_scatter(const Counters *__restrict__ ctr, const BinPair *_
             const float c = fmaxf(pred[i], 1.0f);
             cls = min(63u, (uint32_t)(log2f(c) * 2.0f));
         }
-        // one cursor increment per class among the warp's active lanes
-        const uint32_t act = __activemask();
-        const uint32_t grp = __match_any_sync(act, cls);
+        // one cursor increment per bin among the warp's active lanes
+        const uint32_t act = __activemask(), bin = sched_bin(P, cls, by_loop);
+        const uint32_t grp = __match_any_sync(act, bin);
         const uint32_t lane = threadIdx.x & 31, leader = (uint32_t)__ffs(grp) - 1;
         uint32_t base = 0;
-        if (lane == leader) base = atomicAdd(&cursor[63 - cls], (uint32_t)__popc(grp));
+        if (lane == leader) base = atomicAdd(&cursor[bin], (uint32_t)__popc(grp));
         base = __shfl_sync(act, base, leader);
-        const uint32_t pos = start[63 - cls] + base + __popc(grp & ((1u << lane) - 1u));
+        const uint32_t pos = start[bin] + base + __popc(grp & ((1u << lane) - 1u));
         P.cls = (uint8_t)cls;
         out[pos] = P;
         uint64_t nu;
         if (small_mode && P.a_n <= kSmallSide && (P.same || P.b_n <= kSmallSide)) {
             nu = 0;                               // pair-parallel path, no tiled units
             // small bin pairs from the front of the list, tiny ones from its end
-            const bool tiny = P.same && P.a_n <= kTinySide;
+            // (mode 2, edit distances: also two bins with as few pairs)
+            const bool tiny = P.same ? P.a_n <= kTinySide : small_mode == 2 && P.a_n * P.b_n <= kTinyPairs;
             const uint32_t am = __activemask();
             const uint32_t tm = __ballot_sync(am, tiny), sm = am & ~tm;
             const uint32_t ld = (uint32_t)__ffs(am) - 1;
@@ -512,11 +452,6 @@ __global__ void k_set_unit_base(const Counters *__restrict__ ctr, BinPair *__res
 // only if its V sets and J sets intersect, so each neighbour pair appears once
 // and the pairs are exactly those of the bucket path.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t seg_count(const int16_t *eps_tab, uint32_t NL, uint32_t li) {
-    const int e = eps_tab[(size_t)li * NL + li];
-    return e < 0 ? 1u : (uint32_t)e + 1u;
-}
-
 // Key of segment k of a unique: repertoire (24 bits), length (8), segment (2)
 // and 30 bits of a hash of the segment's residue codes.  Codes are a bijection
 // of the bytes, so identical segments always share a key; two different
@@ -540,17 +475,6 @@ __device__ __forceinline__ unsigned long long seg_key(const uint32_t (&wd)[5][4]
     }
     return ((unsigned long long)r << 40) | ((unsigned long long)L << 32) |
            ((unsigned long long)k << 30) | (h >> 34);
-}
-
-// Slots of the join table in use: about 1.5 slots per possible key (join_smax
-// per unique), a power of two, at most the allocation.  The allocation is sized
-// for every row being unique; the uniques are counted on the device, so the
-// table a call probes (and clears) is the smaller one they need.
-__device__ __forceinline__ uint32_t join_mask(uint32_t nu, uint32_t smax, uint64_t cap_mask) {
-    const uint64_t want = max((3ull * smax * nu + 1) / 2, 1024ull);
-    uint64_t c = 1024;
-    while (c < want) c <<= 1;
-    return (uint32_t)min(c - 1, cap_mask);
 }
 
 // The probed prefix is sized by the unique count, or by `rows` (an upper
@@ -793,6 +717,10 @@ void launch_join_insert(const Plan &P, const Buffers &B, int chunk, cudaStream_t
 
 void launch_buckets(const Plan &P, const Buffers &B, cudaStream_t s) {
     BinGeom g{P.Gv, P.Gj, P.NL, P.Lmin, P.VW, P.JW, P.K};
+    if (P.join && !P.hamming) {
+        launch_lev_join(P, B, s);
+        return;
+    }
     if (P.join) {
         const uint64_t slots = B.jn_mask + 1;   // the allocation; the probed prefix is on the device
         if (!P.front_join) {                    // else the row chunks did these
@@ -821,6 +749,10 @@ void launch_buckets(const Plan &P, const Buffers &B, cudaStream_t s) {
 }
 
 void launch_fill(const Plan &P, const Buffers &B, cudaStream_t s) {
+    if (P.join && !P.hamming) {
+        launch_lev_join_fill(P, B, s);
+        return;
+    }
     if (P.join) {
         BinGeom g{P.Gv, P.Gj, P.NL, P.Lmin, P.VW, P.JW, P.K};
         const int planes = (int)P.B;
@@ -881,6 +813,10 @@ void launch_binpairs(const Plan &P, const Buffers &B, cudaStream_t s) {
 }
 
 void launch_binpairs_fill(const Plan &P, const Buffers &B, cudaStream_t s) {
+    if (P.join && !P.hamming) {
+        launch_lev_join_binpairs(P, B, s);
+        return;
+    }
     if (P.join) {
         BinGeom g{P.Gv, P.Gj, P.NL, P.Lmin, P.VW, P.JW, P.K};
         k_join_bp_fill<<<grid_wave(k_join_bp_fill, (B.jn_mask + 1) / 4, kThreads), kThreads, 0, s>>>(
@@ -895,18 +831,27 @@ void launch_binpairs_fill(const Plan &P, const Buffers &B, cudaStream_t s) {
                                                        &B.ctr->error);
 }
 
+void launch_bucket_pairs(const Plan &P, const Buffers &B, cudaStream_t s) {
+    PairGeom pg{P.NL, P.Lmin, P.Gv, P.Gj, P.K, P.dLmax, P.hamming, P.TX, P.TY, P.TY / P.TX};
+    const uint32_t nb = (uint32_t)P.nbins;
+    cudaMemsetAsync(&B.ctr->bucket_pairs, 0, sizeof(B.ctr->bucket_pairs), s);
+    k_bucket_pairs<<<grid_wave(k_bucket_pairs, nb, kThreads), kThreads, 0, s>>>(nb, pg, B.eps_tab, B.bin_hist,
+                                                                          &B.ctr->bucket_pairs);
+}
+
 void launch_schedule(const Plan &P, const Buffers &B, cudaStream_t s) {
     const uint32_t q = P.TY / P.TX;
     const float *pred = P.schedule == 1 ? B.pred : nullptr;
-    cudaMemsetAsync(B.cls_hist, 0, sizeof(uint32_t) * 130, s);
-    k_cls_hist<<<grid_for(P.cap_binpairs), kThreads, 0, s>>>(B.ctr, B.bp, pred, B.cls_hist);
-    scan_u32(B.cls_hist, B.cls_hist, 64, nullptr, nullptr, B.scan_part, B.scan_part_cap, s);
+    const int by_loop = P.lev_diag ? 1 : 0;
+    cudaMemsetAsync(B.cls_hist, 0, sizeof(uint32_t) * 2 * kSchedBins, s);
+    k_cls_hist<<<grid_for(P.cap_binpairs), kThreads, 0, s>>>(B.ctr, B.bp, pred, B.cls_hist, by_loop);
+    scan_u32(B.cls_hist, B.cls_hist, kSchedBins, nullptr, nullptr, B.scan_part, B.scan_part_cap, s);
     cudaMemsetAsync(&B.ctr->n_small, 0, 2 * sizeof(uint32_t), s);   // n_small, small_cursor
     cudaMemsetAsync(&B.ctr->n_tiny, 0, 2 * sizeof(uint32_t), s);    // n_tiny, tiny_cursor
     k_cls_scatter<<<grid_for(P.cap_binpairs), kThreads, 0, s>>>(
-        B.ctr, B.bp, pred, B.cls_hist, B.cls_hist + 64, B.bp_sorted, B.bp_units, P.TX, P.TY, q,
-        P.planes() ? 1 : 0, B.bp_small, &B.ctr->n_small, &B.ctr->n_tiny,
-        (uint32_t)P.cap_binpairs + 1u);
+        B.ctr, B.bp, pred, B.cls_hist, B.cls_hist + kSchedBins, B.bp_sorted, B.bp_units, P.TX, P.TY, q,
+        P.planes() ? (P.hamming ? 1 : 2) : 0, B.bp_small, &B.ctr->n_small, &B.ctr->n_tiny,
+        (uint32_t)P.cap_binpairs + 1u, by_loop);
     scan_u32(B.bp_units, B.bp_units, (uint32_t)P.cap_binpairs, &B.ctr->n_binpairs,
              &B.ctr->n_units, B.scan_part, B.scan_part_cap, s);
     k_set_unit_base<<<grid_for(P.cap_binpairs), kThreads, 0, s>>>(B.ctr, B.bp_sorted, B.bp_units);

@@ -368,6 +368,7 @@ static DistArgs make_args(const Plan &P, const Buffers &B) {
     a.small_list = B.bp_small;
     a.small_cap = (uint32_t)P.cap_binpairs + 1u;
     a.join = P.join ? 1 : 0;
+    a.vj_meta = P.vj_meta ? 1 : 0;
     a.sink = kSinkEdges;
     a.cnt = B.cnt;
     a.ucopies = B.ucopies;

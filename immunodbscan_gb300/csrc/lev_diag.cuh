@@ -21,6 +21,11 @@ namespace idb {
 
 namespace {
 
+// A unit with at most this many x-entries is scored pair by pair: a pair read from
+// L1 costs about twice a tiled one, and a tile would leave 3/4 of the lanes idle.
+constexpr uint32_t kThinX = 8;
+constexpr uint32_t kLevHitQ = 16;   // queued (y, hits) records per lane
+
 template <int BP, int W>
 struct LevShape {
     static constexpr int NW = BP * W;            // words per record
@@ -65,12 +70,168 @@ __device__ __noinline__ uint32_t lev_pair(const uint4 *xr, const uint4 *yr, uint
     return 1u;
 }
 
+// Is a pair of a segment-join group that is within eps to be emitted from this
+// group?  Its V and J sets must intersect, and the group's (segment k, shift)
+// must be the first, in the order of the look-ups (k_lev_join.cu), at which x
+// (the shorter; of two equal lengths the smaller unique id) holds a segment of
+// y.  P.v is the segment, P.j the segment count.  mx, my: side records.
+template <int BP, int W>
+__device__ __noinline__ bool lev_join_ok(const DistArgs &a, const BinPair &P, const uint4 *xr,
+                                         const uint4 *yr, const uint4 &mx, const uint4 &my) {
+    const int m = P.la, n = P.lb, gap = n - m, S = P.j, e = S - 1, kg = P.v;
+    int dg = 0;   // the group's shift
+    if (P.same) {
+        if (mx.w > my.w) { const uint4 *t = xr; xr = yr; yr = t; }
+    } else {
+        if (gap == 0 && mx.w >= my.w) return false;   // found from the other side (or itself)
+        dg = max(-kg, -gap - (e - kg)) + (int)(mx.z >> 30);
+    }
+    if (a.vj_meta) {
+        if (((mx.x & my.x) | (mx.y & my.y)) == 0 || (mx.z & my.z & 0x3FFFFFFFu) == 0) return false;
+    } else if (!vj_intersect(a, mx.w, my.w)) {
+        return false;
+    }
+    uint32_t x[BP * W], y[BP * W];
+    load_planes<BP, W>(xr, x);
+    load_planes<BP, W>(yr, y);
+    for (int k = 0; k <= kg; ++k) {
+        const int s = k * n / S, len = (k + 1) * n / S - s;
+        const int lo = max(-k, -gap - (e - k)), hi = min(k, e - k - gap);
+        for (int d = lo; d <= hi; ++d) {
+            const int pos = s + d;
+            if (pos < 0 || pos + len > m) continue;
+            uint32_t diff[W];
+#pragma unroll
+            for (int w = 0; w < W; ++w) diff[w] = 0;
+#pragma unroll
+            for (int p = 0; p < BP; ++p) {
+                uint32_t in[W], sh[W];
+#pragma unroll
+                for (int w = 0; w < W; ++w) in[w] = y[p * W + w];
+                shift_words<W>(in, -d, sh);            // bit i: y[i - d]
+#pragma unroll
+                for (int w = 0; w < W; ++w) diff[w] |= x[p * W + w] ^ sh[w];
+            }
+            uint32_t any = 0;
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                const int a0 = max(pos - 32 * w, 0), a1 = min(pos + len - 32 * w, 32);
+                if (a0 < a1) any |= diff[w] & (low_mask32(a1) & ~low_mask32(a0));
+            }
+            const bool here = k == kg && d == dg;
+            if (any == 0) return here;
+            if (here) return false;   // the key was shared by its hash only
+        }
+    }
+    return false;
+}
+
+template <int BP, int W>
+__device__ __forceinline__ bool lev_is_edge(const DistArgs &a, const BinPair &P, uint32_t xrow, uint32_t yrow,
+                                            const uint4 &mx, const uint4 &my) {
+    constexpr int R16 = LevShape<BP, W>::R16;
+    if (!a.join) return canonical_meta(a, P, mx, my);
+    return lev_join_ok<BP, W>(a, P, a.rec + (size_t)xrow * R16, a.rec + (size_t)yrow * R16, mx, my);
+}
+
 // A warp's shared memory.
 struct LevSlice {
     uint4 *sy;       // staged y-records, one shifted copy per diagonal
     uint4 *sym;      // y side records
     uint4 *sxm;      // x side records
     uint32_t *shq;   // deferred hits
+    uint32_t *seg;   // segment join: masks of the look-ups (LevLookups)
+};
+
+// Out of line: one copy for every unit loop.
+__device__ __noinline__ void lev_drain(const DistArgs &a, EdgeWriter &ew, const BinPair &P, const LevSlice &S,
+                                       uint32_t qn, int lane) {
+    drain_hits(a, ew, S.shq, qn, S.sxm, S.sym, lane, a.join && a.vj_meta,
+               [&](uint32_t r, uint32_t, const uint4 &my) {
+                   const uint4 mx = S.sxm[32 * r + lane];
+                   return a.join ? vj_intersect(a, mx.w, my.w) : canonical_meta(a, P, mx, my);
+               });
+}
+
+// The look-ups of a length pair (k_lev_join.cu) are the cells of the diagonal test:
+// segment k at shift delta is diagonal d = -delta, and x holds it iff the mask of
+// diagonal d has no bit in x's positions of the segment.  A unit keeps, in the
+// order of the look-ups, those position masks, then (equal lengths) the masks
+// of the unshifted segments for pairs taken the other way round.
+template <int E, int G, int W>
+struct LevLookups {
+    using Dg = LevDiags<E, G>;
+    static constexpr int count() {
+        int n = 0;
+        for (int k = 0; k <= E; ++k)
+            for (int d = G + Dg::lo; d >= -Dg::lo; --d) n += Dg::cell(d, k);
+        return n;
+    }
+    static constexpr int n = count();
+    static constexpr int words = (n + E + 1) * W;
+    // lanes write the masks; returns a bit per look-up that lies inside x
+    static __device__ __forceinline__ uint32_t fill(uint32_t *seg, int m, int len_y, int lane) {
+        uint32_t valid = 0;
+        int idx = 0;
+#pragma unroll
+        for (int k = 0; k <= E; ++k) {
+            const int s = k * len_y / (E + 1), t = (k + 1) * len_y / (E + 1);
+#pragma unroll
+            for (int d = G + Dg::lo; d >= -Dg::lo; --d) {
+                if (!Dg::cell(d, k)) continue;
+                const int a = s - d, b = t - d;
+                if (a >= 0 && b <= m) valid |= 1u << idx;
+#pragma unroll
+                for (int w = 0; w < W; ++w)
+                    if (lane == w) seg[idx * W + w] = word_mask(a, b, w);
+                ++idx;
+            }
+#pragma unroll
+            for (int w = 0; w < W; ++w)
+                if (lane == w) seg[(n + k) * W + w] = word_mask(s, t, w);
+        }
+        return valid;
+    }
+    // bits of word w at positions [a, b)
+    static __device__ __forceinline__ uint32_t word_mask(int a, int b, int w) {
+        const int a0 = min(max(a - 32 * w, 0), 32), b0 = min(max(b - 32 * w, 0), 32);
+        return low_mask32(b0) & ~low_mask32(a0);
+    }
+    // number of the first look-up of segment kg
+    static __device__ __forceinline__ uint32_t base(int kg) {
+        uint32_t n = 0;
+#pragma unroll
+        for (int k = 0; k < E; ++k)
+#pragma unroll
+            for (int d = G + Dg::lo; d >= -Dg::lo; --d)
+                if (Dg::cell(d, k) && k < kg) ++n;
+        return n;
+    }
+    // Emitted here: of the look-ups that hold (valid: lies inside x), the group's
+    // own is the first.  D: the pair's mismatch masks.
+    static __device__ __forceinline__ bool first(const uint32_t (&D)[Dg::n][W], const uint32_t *seg,
+                                                 uint32_t valid, uint32_t own, bool swapped) {
+        uint32_t holds = 0;
+        int idx = 0;
+#pragma unroll
+        for (int k = 0; k <= E; ++k)
+#pragma unroll
+            for (int d = G + Dg::lo; d >= -Dg::lo; --d) {
+                if (!Dg::cell(d, k)) continue;
+                uint32_t any = 0;
+#pragma unroll
+                for (int w = 0; w < W; ++w) {
+                    if (G == 0 && d != 0)
+                        any |= (swapped ? D[(G == 0 ? -d : d) + Dg::lo][w] : D[d + Dg::lo][w]) &
+                               seg[(swapped ? n + k : idx) * W + w];
+                    else
+                        any |= D[d + Dg::lo][w] & seg[idx * W + w];
+                }
+                if (any == 0) holds |= 1u << idx;
+                ++idx;
+            }
+        return ((holds & valid) & (0xFFFFFFFFu >> (31 - own))) == 1u << own;
+    }
 };
 
 // One tiled unit: 32*RX x-entries in registers against the unit's y-entries.
@@ -82,8 +243,21 @@ __device__ __forceinline__ void lev_unit(const DistArgs &a, EdgeWriter &ew, cons
     constexpr int NW = Sh::NW;
     constexpr int Y16 = (Dg::n * NW + 3) / 4;    // 16-byte words of a staged y
     static_assert(Y16 <= Sh::YMax, "staged y-record size");
+    using Lk = LevLookups<E, G, W>;
     const bool same = U.P.same != 0;
     uint32_t x[RX][NW], vmask[RX];
+    // segment join: the group's look-up, plus a per-entry shift for the classes
+    // that looked it up (the group's own uniques: no shift, the middle one)
+    const int kg = U.P.v;
+    const uint32_t own = Lk::base(kg) + (same ? (uint32_t)min(kg, E - kg) : 0u);
+    const uint32_t valid = a.join ? Lk::fill(S.seg, U.P.la, U.P.lb, lane) : 0u;
+    // Segment join: may a pair within eps be emitted from this group?  (V and J
+    // sets intersect; of equal lengths the smaller id looks the larger one up.)
+    auto join_edge = [&](const uint32_t (&D)[Dg::n][W], const uint4 &mx, const uint4 &my) {
+        if (a.vj_meta && (((mx.x & my.x) | (mx.y & my.y)) == 0 || (mx.z & my.z & 0x3FFFFFFFu) == 0)) return false;
+        if (G == 0 && !same && mx.w >= my.w) return false;
+        return Lk::first(D, S.seg, valid, own + (same ? 0u : mx.z >> 30), G == 0 && same && mx.w > my.w);
+    };
 #pragma unroll
     for (int r = 0; r < RX; ++r) {
         const uint32_t xi = (uint32_t)r * 32 + lane;
@@ -126,10 +300,39 @@ __device__ __forceinline__ void lev_unit(const DistArgs &a, EdgeWriter &ew, cons
         // x-entries before them; they come first in the chunk
         uint32_t tdiag = 0;
         if (same && U.ybase + yb < U.xbase + U.nx) tdiag = min(nb, U.xbase + U.nx - (U.ybase + yb));
-        auto is_edge = [&](uint32_t r, uint32_t, const uint4 &my) {
-            return canonical_meta(a, U.P, S.sxm[32 * r + lane], my);
-        };
         uint32_t qn = 0;
+        // Segment join: the queued pairs that are emitted from this group.  Checked
+        // here and not in the loop below, where one hit in a warp would make all of
+        // it wait for the check (2M rows, 0.15e9 neighbours: 9.2 ms in the loop).
+        auto flush = [&]() {
+            __syncwarp();
+            if (a.join)
+                for (uint32_t k = 0; k < qn; ++k) {
+                    const uint32_t e = S.shq[k * 32 + lane], t = e >> 8;
+                    const uint4 my = S.sym[t];
+                    const uint32_t *ys = reinterpret_cast<const uint32_t *>(S.sy + t * Y16);
+                    uint32_t keep = 0;
+#pragma unroll
+                    for (int r = 0; r < RX; ++r)
+                        if ((e >> r) & 1u) {
+                            uint32_t D[Dg::n][W];
+#pragma unroll
+                            for (int q = 0; q < Dg::n; ++q)
+#pragma unroll
+                                for (int w = 0; w < W; ++w) {
+                                    uint32_t d = x[r][w] ^ ys[q * NW + w];
+#pragma unroll
+                                    for (int p = 1; p < BP; ++p) d |= x[r][p * W + w] ^ ys[q * NW + p * W + w];
+                                    D[q][w] = d;
+                                }
+                            keep |= (uint32_t)join_edge(D, S.sxm[32 * r + lane], my) << r;
+                        }
+                    S.shq[k * 32 + lane] = (t << 8) | keep;
+                }
+            lev_drain(a, ew, U.P, S, qn, lane);
+            qn = 0;
+            __syncwarp();
+        };
         for (uint32_t t = 0; t < nb; ++t) {
             uint32_t y[4 * Y16];
 #pragma unroll
@@ -160,18 +363,12 @@ __device__ __forceinline__ void lev_unit(const DistArgs &a, EdgeWriter &ew, cons
             }
             uint32_t hit = 0;
 #pragma unroll
-            for (int r = 0; r < RX; ++r) hit |= (uint32_t)(sc[r] == 0) << r;
+            for (int r = 0; r < RX; ++r)
+                hit |= (uint32_t)(sc[r] == 0) << r;
             if (hit) S.shq[qn++ * 32 + lane] = (t << 8) | hit;
-            if (__any_sync(0xFFFFFFFFu, qn == (uint32_t)kHitQ)) {
-                __syncwarp();
-                drain_hits(a, ew, S.shq, qn, S.sxm, S.sym, lane, false, is_edge);
-                qn = 0;
-                __syncwarp();
-            }
-        }
-        if (__any_sync(0xFFFFFFFFu, qn)) {
-            __syncwarp();
-            drain_hits(a, ew, S.shq, qn, S.sxm, S.sym, lane, false, is_edge);
+            // one flush in the code: the queue is full, or the batch ends
+            const bool end = t + 1 == nb;
+            if (__any_sync(0xFFFFFFFFu, qn == kLevHitQ || (end && qn))) flush();
         }
     }
     __syncwarp();
@@ -183,6 +380,32 @@ __device__ __forceinline__ void lev_unit_rx(const DistArgs &a, EdgeWriter &ew, c
                                             const LevSlice &S, int lane, uint64_t &pairs) {
     if (RX > 1 && U.nx <= 32) lev_unit<BP, W, 1, E, G>(a, ew, U, S, lane, pairs);
     else lev_unit<BP, W, RX, E, G>(a, ew, U, S, lane, pairs);
+}
+
+// Pairs of nx x-entries with ny y-entries (same: pairs of the nx entries), lanes
+// taking pairs and reading their records from L1.
+template <int BP, int W>
+__device__ __forceinline__ void lev_pair_block(const DistArgs &a, EdgeWriter &ew, const BinPair &P, bool same,
+                                               uint32_t xstart, uint32_t nx, uint32_t ystart, uint32_t ny,
+                                               int lane) {
+    constexpr int R16 = LevShape<BP, W>::R16;
+    const uint32_t npairs = same ? nx * (nx - 1) / 2 : nx * ny;
+    for (uint32_t b0 = 0; b0 < npairs; b0 += 1024) {
+        uint32_t rmask = 0;           // bit i: the lane's pair of round i is an edge
+        for (uint32_t p0 = b0; p0 < min(npairs, b0 + 1024); p0 += 32) {
+            const uint32_t p = p0 + lane;
+            if (p >= npairs) break;
+            uint32_t i, j;
+            small_pair(p, same, nx, i, j);
+            const uint32_t xrow = xstart + i, yrow = ystart + j;
+            if (lev_pair<BP, W>(a.rec + (size_t)xrow * R16, a.rec + (size_t)yrow * R16, (uint32_t)P.eps,
+                                (uint32_t)(P.lb - P.la)) == 0 &&
+                lev_is_edge<BP, W>(a, P, xrow, yrow, __ldg(a.meta + xrow), __ldg(a.meta + yrow)))
+                rmask |= 1u << ((p0 - b0) >> 5);
+        }
+        __syncwarp();
+        emit_pair_bits(a, ew, lane, rmask, b0 + (uint32_t)lane, 32u, same, nx, xstart, ystart);
+    }
 }
 
 // Small bin pairs (at most kSmallSide entries a side): a warp each, lanes take
@@ -221,27 +444,15 @@ __device__ __forceinline__ void lev_small_all(const DistArgs &a, EdgeWriter &ew,
             const uint32_t n = P.a_n, npairs = same ? n * (n - 1) / 2 : n * P.b_n;
             const uint32_t ystart = same ? P.a_start : P.b_start;
             if (lane == 0) pairs += npairs;
-            uint32_t rmask = 0;           // bit i: the lane's pair of round i is an edge
-            for (uint32_t p0 = 0; p0 < npairs; p0 += 32) {
-                const uint32_t p = p0 + lane;
-                if (p >= npairs) break;
-                uint32_t i, j;
-                small_pair(p, same, n, i, j);
-                if (lev_pair<BP, W>(a.rec + (size_t)(P.a_start + i) * R16,
-                                    a.rec + (size_t)(ystart + j) * R16, (uint32_t)P.eps,
-                                    (uint32_t)(P.lb - P.la)) == 0 &&
-                    canonical_meta(a, P, __ldg(a.meta + P.a_start + i), __ldg(a.meta + ystart + j)))
-                    rmask |= 1u << (p0 >> 5);
-            }
-            __syncwarp();
-            emit_pair_bits(a, ew, lane, rmask, (uint32_t)lane, 32u, same, n, P.a_start, ystart);
+            lev_pair_block<BP, W>(a, ew, P, same, P.a_start, n, ystart, P.b_n, lane);
             if (a.bp_cycles && lane == 0)
                 atomicAdd(&a.bp_cycles[idx], (unsigned long long)(clock64() - t0));
         }
     }
 }
 
-// Tiny bin pairs: one lane takes every pair of one of them, 32 at a time.
+// Tiny bin pairs (at most kTinyPairs pairs): one lane takes every pair of one of
+// them, 32 at a time.
 template <int BP, int W>
 __device__ __forceinline__ void lev_tiny_all(const DistArgs &a, EdgeWriter &ew, int lane,
                                              uint64_t &pairs) {
@@ -261,20 +472,23 @@ __device__ __forceinline__ void lev_tiny_all(const DistArgs &a, EdgeWriter &ew, 
             idx = a.small_list[a.small_cap - 1u - (s0 + (uint32_t)lane)];
             P = a.bp[idx];
         }
-        const uint32_t n = P.a_n, np = n * (n - 1) / 2;
+        const bool same = P.same != 0;
+        const uint32_t n = P.a_n, np = same ? n * (n - 1) / 2 : n * P.b_n;
+        const uint32_t ystart = same ? P.a_start : P.b_start;
         pairs += np;
-        static_assert(kTinySide * (kTinySide - 1) / 2 <= 32, "tiny pair mask");
-        const uint4 *rec = a.rec + (size_t)P.a_start * R16;
+        static_assert(kTinyPairs <= 32, "tiny pair mask");
         uint32_t emask = 0;
         for (uint32_t p = 0; p < np; ++p) {
             uint32_t i, j;
-            small_pair(p, true, n, i, j);
-            if (lev_pair<BP, W>(rec + (size_t)i * R16, rec + (size_t)j * R16, (uint32_t)P.eps, 0u) == 0 &&
-                canonical_meta(a, P, __ldg(a.meta + P.a_start + i), __ldg(a.meta + P.a_start + j)))
+            small_pair(p, same, n, i, j);
+            const uint32_t xrow = P.a_start + i, yrow = ystart + j;
+            if (lev_pair<BP, W>(a.rec + (size_t)xrow * R16, a.rec + (size_t)yrow * R16, (uint32_t)P.eps,
+                                (uint32_t)(P.lb - P.la)) == 0 &&
+                lev_is_edge<BP, W>(a, P, xrow, yrow, __ldg(a.meta + xrow), __ldg(a.meta + yrow)))
                 emask |= 1u << p;
         }
         __syncwarp();
-        emit_pair_bits(a, ew, lane, emask, 0u, 1u, true, n, P.a_start, P.a_start);
+        emit_pair_bits(a, ew, lane, emask, 0u, 1u, same, n, P.a_start, ystart);
         if (a.bp_cycles) {   // the batch's cycles, shared out by pairs
             const uint32_t tot = __reduce_add_sync(0xFFFFFFFFu, np);
             const unsigned long long dt = (unsigned long long)(clock64() - t0);
@@ -285,20 +499,28 @@ __device__ __forceinline__ void lev_tiny_all(const DistArgs &a, EdgeWriter &ew, 
 
 template <int BP, int W, int RX>
 __global__ void __launch_bounds__(kWarps * 32, (W <= 2 ? 4 : 3))
-k_lev_diag(DistArgs a) {
+k_lev_diag(const __grid_constant__ DistArgs a) {
     using Sh = LevShape<BP, W>;
     __shared__ uint4 sy[kWarps][Sh::YB * Sh::YMax];
     __shared__ uint4 sym[kWarps][Sh::YB];
     __shared__ uint4 sxm[kWarps][32 * RX];
-    __shared__ uint32_t shq[kWarps][kHitQ * 32];
+    __shared__ uint32_t shq[kWarps][kLevHitQ * 32];
+    __shared__ uint32_t seg[kWarps][LevLookups<3, 0, W>::words];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t n_units = a.ctr->n_units, n_bp = a.ctr->n_binpairs;
-    const LevSlice S{sy[wid], sym[wid], sxm[wid], shq[wid]};
+    const LevSlice S{sy[wid], sym[wid], sxm[wid], shq[wid], seg[wid]};
     EdgeWriter ew;
     ew.init();
     uint64_t pairs = 0;
     Unit U;
     while (next_unit(a, n_units, n_bp, lane, U)) {
+        if (!U.P.same && U.nx <= kThinX) {   // too few x-entries for the lanes: pair by pair
+            if (lane == 0) pairs += (uint64_t)U.nx * U.ny;
+            lev_pair_block<BP, W>(a, ew, U.P, false, U.P.a_start + U.xbase, U.nx,
+                                  U.P.b_start + U.ybase, U.ny, lane);
+            log_unit(a, U, lane);
+            continue;
+        }
         switch ((uint32_t)U.P.eps * 4 + (uint32_t)(U.P.lb - U.P.la)) {
             case 0: lev_unit_rx<BP, W, RX, 0, 0>(a, ew, U, S, lane, pairs); break;
             case 4: lev_unit_rx<BP, W, RX, 1, 0>(a, ew, U, S, lane, pairs); break;

@@ -60,7 +60,9 @@ typedef struct idb_params {
     int32_t  schedule;         /* 0 = static (pair-count) order, 1 = learned       */
     int32_t  tile_rx;          /* x-entries per lane of a work unit (0 = default)  */
     int32_t  tile_ty;          /* y-entries of a work unit (0 = default)           */
-    int32_t  candidates;       /* 0 = automatic (Hamming eps <= 2: segment join),
+    int32_t  candidates;       /* 0 = automatic (Hamming eps <= 2 and edit distance
+                                  eps <= 3: segment join, unless the buckets
+                                  hold fewer pairs than an edit-distance join),
                                   1 = every admissible pair of the buckets        */
     int32_t  edge_memory_mb;   /* device memory for the neighbour-pair list:
                                   0 = as much as the pairs need; > 0 = at most this
@@ -126,8 +128,9 @@ typedef struct idb_stats {
                                   (0 when eps <= 3 everywhere: those pairs are
                                   decided without a recurrence over columns)      */
     uint32_t candidates;       /* 0: every admissible pair of the buckets scored;
-                                  1: Hamming segment join (eps <= 2 at every
-                                  length): only pairs sharing a whole segment    */
+                                  1: segment join (Hamming eps <= 2, edit distance
+                                  eps <= 3 at every length): only pairs sharing a
+                                  whole segment                                   */
     uint32_t streamed;         /* 1: neighbour pairs were not stored (two sweeps;
                                   core_edges is not counted)                      */
 } idb_stats;
