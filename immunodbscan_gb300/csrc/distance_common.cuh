@@ -36,7 +36,7 @@ struct DistArgs {
     uint32_t sink;
     uint32_t *cnt;                   // copies-weighted neighbour counts (count sweep)
     const uint32_t *ucopies;
-    const uint32_t *ucore;           // core flags (grow sweep)
+    const uint32_t *ecopies;         // the same per entry
     uint32_t *parent;                // union-find forest (grow sweep)
     uint32_t *bmin;                  // minimum core neighbour of a non-core unique
 };
@@ -51,7 +51,7 @@ void launch_lev_diag_5(const Plan &P, const DistArgs &a, int grid, cudaStream_t 
 namespace {
 
 constexpr int kWarps = 4;            // warps per block
-constexpr int kYB = 64;              // y-records staged per batch
+constexpr int kYB = 32;              // y-records staged per batch (a lane's hits: one word)
 
 // Streamed mode, for neighbour graphs larger than the edge memory allowed: the
 // distance work runs twice and no pair is stored.  The count sweep adds each
@@ -62,33 +62,31 @@ constexpr int kYB = 64;              // y-records staged per batch
 // same border rule as the edge-list path).  Both are order-independent.
 __device__ __forceinline__ uint32_t sweep_find(uint32_t *p, uint32_t x) {
     volatile uint32_t *vp = p;
-    while (true) {   // parent[y] <= y: x strictly decreases
+    while (true) {   // parent[y] <= y of a core y: x strictly decreases
         const uint32_t px = vp[x];
-        if (px == x) return x;
+        if (px >= x) return px == x ? x : kNone;   // kNone: not a core's parent
         const uint32_t ppx = vp[px];
-        if (ppx == px) return px;
+        if (ppx >= px) return ppx == px ? px : kNone;
         vp[x] = ppx;   // path halving
         x = ppx;
     }
 }
 
 __device__ __noinline__ void sink_streamed(const DistArgs &a, uint32_t lo, uint32_t hi) {
-    if (a.sink == kSinkCount) {
-        atomicAdd(&a.cnt[lo], __ldg(&a.ucopies[hi]));
-        atomicAdd(&a.cnt[hi], __ldg(&a.ucopies[lo]));
+    // parents carry the core flag; equal ones (stale or not) are one component
+    const uint32_t plo = __ldcg(a.parent + lo), phi = __ldcg(a.parent + hi);
+    const uint32_t nlo = plo & kNonCore, nhi = phi & kNonCore;
+    if (nlo != nhi) {
+        atomicMin(&a.bmin[nlo ? lo : hi], nlo ? hi : lo);
         return;
     }
-    const uint32_t clo = a.ucore[lo], chi = a.ucore[hi];
-    if (clo != chi) {
-        atomicMin(&a.bmin[clo ? hi : lo], clo ? lo : hi);
-        return;
-    }
-    if (!clo) return;
-    uint32_t x = lo, y = hi, it = 0;
+    if (nlo || plo == phi) return;
+    uint32_t x = plo, y = phi, it = 0;
     for (; it < kSpinCap; ++it) {
         uint32_t rx = sweep_find(a.parent, x), ry = sweep_find(a.parent, y);
         if (rx == ry) break;
         if (rx < ry) { const uint32_t t = rx; rx = ry; ry = t; }
+        if (rx == kNone) { it = kSpinCap; break; }
         if (atomicCAS(&a.parent[rx], rx, ry) == rx) break;   // hook the larger root
         x = rx;
         y = ry;
@@ -100,9 +98,20 @@ __device__ __noinline__ void sink_streamed(const DistArgs &a, uint32_t lo, uint3
 __device__ __forceinline__ void put_edge(const DistArgs &a, uint64_t slot, uint32_t lo, uint32_t hi) {
     if (a.sink == kSinkEdges) {
         if (slot < a.cap_edges) a.edges[slot] = make_uint2(lo, hi);
-    } else {
+    } else if (a.sink == kSinkGrow) {
         sink_streamed(a, lo, hi);
     }
+}
+
+// Copies-weighted counts (rule S5) of one neighbour pair (copies clo, chi), and a
+// smaller neighbour for the larger id (any one will do, so a plain store): the
+// forest the unions start from (k_core).
+__device__ __forceinline__ void count_pair(const DistArgs &a, uint32_t lo, uint32_t hi, uint32_t clo,
+                                           uint32_t chi) {
+    if (a.sink == kSinkGrow) return;
+    atomicAdd(&a.cnt[lo], chi);
+    atomicAdd(&a.cnt[hi], clo);
+    a.parent[hi] = lo;
 }
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
@@ -144,7 +153,10 @@ struct EdgeWriter {
             if ((uint64_t)b + kEdgeChunk > a.cap_edges && lane == 0)
                 atomicOr(&a.ctr->error, kErrEdgeOverflow);
         }
-        if (ok) put_edge(a, base + fill + __popc(m & lanemask_lt()), lo, hi);
+        if (ok) {
+            put_edge(a, base + fill + __popc(m & lanemask_lt()), lo, hi);
+            count_pair(a, lo, hi, __ldg(&a.ucopies[lo]), __ldg(&a.ucopies[hi]));
+        }
         fill += n;
         written += n;
     }
@@ -306,38 +318,17 @@ __device__ __forceinline__ void small_pair(uint32_t p, bool same, uint32_t n, ui
     }
 }
 
-// Bulk append of a lane's edges given as bits: bit b stands for pair index
-// p0 + stride*b of a small or tiny bin pair (i, j from the pair index; the
-// unique ids from the side records).  Warp-uniform.
-__device__ __forceinline__ void emit_pair_bits(const DistArgs &a, EdgeWriter &ew, int lane,
-                                               uint32_t bits, uint32_t p0, uint32_t stride,
-                                               bool same, uint32_t n, uint32_t xstart,
-                                               uint32_t ystart) {
-    const uint32_t c = (uint32_t)__popc(bits);
-    uint32_t incl = c;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-        if (lane >= d) incl += t;
-    }
-    const uint32_t T = __shfl_sync(0xFFFFFFFFu, incl, 31);
-    if (T == 0) return;
-    const EdgeWriter::Bulk bk = ew.reserve(a, lane, T);
-    uint32_t k = incl - c;
-    for (uint32_t b = bits; b; b &= b - 1) {
-        const uint32_t p = p0 + stride * ((uint32_t)__ffs(b) - 1u);
-        uint32_t i, j;
-        small_pair(p, same, n, i, j);
-        const uint32_t ux = __ldg(&a.meta[xstart + i].w), uy = __ldg(&a.meta[ystart + j].w);
-        put_edge(a, ew.slot_of(bk, k++), min(ux, uy), max(ux, uy));
-    }
-}
-
-// Small bin pairs of a warp: the warp claims kSmallBatch schedule positions
+// Small bin pairs of a warp: the warp claims up to kSmallBatch schedule positions
 // with one atomic, each lane loads one of their bin pairs, and while one bin
 // pair is scored the next one's records are prefetched into L1 (a small bin
 // pair is otherwise a chain of dependent loads: position, bin pair, records).
+// When there are fewer than two claims a warp, the claims get smaller instead,
+// so that no warp works through a chain while others have nothing.
 constexpr uint32_t kSmallBatch = 16;
+
+__device__ __forceinline__ uint32_t small_batch(uint32_t n_small) {
+    return min(kSmallBatch, max(1u, n_small / (2u * gridDim.x * kWarps)));
+}
 
 __device__ __forceinline__ BinPair shfl_binpair(const BinPair &p, int src) {
     static_assert(sizeof(BinPair) % 4 == 0, "BinPair words");
@@ -354,56 +345,190 @@ __device__ __forceinline__ BinPair shfl_binpair(const BinPair &p, int src) {
 __device__ __forceinline__ void prefetch_l1(const void *p) {
     asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
-// Deferred hits: the tiled loops only record, per lane, (y index in the staged
-// chunk, hit bits) in a small shared-memory queue; the queue is drained here when
-// a lane's queue is full or the chunk ends, with every lane taking part.
-constexpr int kHitQ = 8;   // queued (y, hits) records per lane
 constexpr uint32_t kOff = 0x40000000u;   // score of a masked x-entry (never a hit)
 
-// The queue holds (y index in the chunk, hit bits) per lane.  Hits are
-// compacted over the whole warp before they are written: each lane first keeps
-// the bits of its own queue that are edges (check(r, t, my): x-entry 32 r + lane
-// against y-entry t of the chunk, whose side record is my; `decided`: the
-// hits were checked when they were queued), then one warp scan gives every
-// lane its place in one bulk append.
-template <typename Check>
-__device__ __forceinline__ void drain_hits(const DistArgs &a, EdgeWriter &ew, uint32_t *q,
-                                           uint32_t qn, const uint4 *xm, const uint4 *ym, int lane,
-                                           bool decided, Check check) {
-    uint32_t c = 0;
-    for (uint32_t k = 0; k < qn; ++k) {
-        const uint32_t e = q[k * 32 + lane];
-        uint32_t keep = e & 0xFFu;
-        if (!decided) {
-            const uint32_t t = e >> 8;
-            const uint4 my = ym[t];
-            for (uint32_t b = keep; b; b &= b - 1) {
-                const uint32_t r = (uint32_t)__ffs(b) - 1u;
-                if (!check(r, t, my)) keep &= ~(1u << r);
-            }
-            q[k * 32 + lane] = (t << 8) | keep;
-        }
-        c += (uint32_t)__popc(keep);
+// What a tiled unit keeps of its entries in the warp's shared memory.
+struct TileSlice {
+    uint4 *xm, *ym;          // side records of the x-entries and of the batch's y-entries
+    uint32_t *xcp, *ycp;     // their copies
+    uint32_t *xs, *ys;       // sums of the neighbours' copies (ys: small bin pairs only)
+
+    __device__ __forceinline__ void begin_x(const DistArgs &a, uint32_t i, uint32_t entry) const {
+        xm[i] = __ldg(a.meta + entry);
+        xcp[i] = __ldg(a.ecopies + entry);
+        xs[i] = 0u;
     }
+    __device__ __forceinline__ void begin_y(const DistArgs &a, uint32_t t, uint32_t entry) const {
+        ym[t] = __ldg(a.meta + entry);
+        ycp[t] = __ldg(a.ecopies + entry);
+    }
+    // after the unit's last batch: one count update per x-entry
+    __device__ __forceinline__ void end_x(const DistArgs &a, uint32_t n, int lane) const {
+        __syncwarp();
+        for (uint32_t i = (uint32_t)lane; i < n; i += 32)
+            if (xs[i]) atomicAdd(&a.cnt[xm[i].w], xs[i]);
+        __syncwarp();
+    }
+};
+
+// 32 x 32 bit transpose over the warp: bit k of lane i becomes bit i of lane k.
+__device__ __forceinline__ uint32_t transpose32(uint32_t m, int lane) {
+    uint32_t mask = 0x0000FFFFu;
+#pragma unroll
+    for (int j = 16; j; j >>= 1, mask ^= mask << j) {
+        const uint32_t o = __shfl_xor_sync(0xFFFFFFFFu, m, j);
+        m = (lane & j) ? (m & ~mask) | ((o & ~mask) >> j) : (m & mask) | ((o & mask) << j);
+    }
+    return m;
+}
+
+// The neighbour pairs of a batch: bit t of hits[r] = x-entry 32 r + lane with
+// y-entry t.  One bulk append for the warp, and the counts of both sides: a
+// lane's hits give its x-entries' sums, the transposed bits the y-entries',
+// so that an entry costs one count update per unit or batch instead of one per
+// pair (a pass over the edge list afterwards took 1.8 ms for 0.15e9 pairs,
+// nearly all of it atomics).  Most entries have one copy: a sum is a popcount
+// plus what the others add.  Out of line: one copy for every unit loop.
+template <int RX>
+__device__ __noinline__ void emit_batch(const DistArgs &a, EdgeWriter &ew, const TileSlice &T,
+                                        const uint32_t (&hits)[RX], uint32_t nb, int lane) {
+    uint32_t c = 0;
+#pragma unroll
+    for (int r = 0; r < RX; ++r) c += (uint32_t)__popc(hits[r]);
     uint32_t incl = c;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
         const uint32_t n = __shfl_up_sync(0xFFFFFFFFu, incl, d);
         if (lane >= d) incl += n;
     }
-    const uint32_t T = __shfl_sync(0xFFFFFFFFu, incl, 31);
-    if (T == 0) return;
-    const EdgeWriter::Bulk bk = ew.reserve(a, lane, T);
-    uint32_t i = incl - c;
-    for (uint32_t k = 0; k < qn; ++k) {
-        const uint32_t e = q[k * 32 + lane];
-        const uint32_t uy = ym[e >> 8].w;
-        for (uint32_t b = e & 0xFFu; b; b &= b - 1) {
-            const uint32_t r = (uint32_t)__ffs(b) - 1u;
-            const uint32_t ux = xm[32 * r + lane].w;
+    const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    if (total == 0) return;
+    const EdgeWriter::Bulk bk = ew.reserve(a, lane, total);
+    const bool count = a.sink != kSinkGrow;
+    const uint32_t uy_lane = (uint32_t)lane < nb ? T.ym[lane].w : 0u;
+    const uint32_t ymult = __ballot_sync(0xFFFFFFFFu, (uint32_t)lane < nb && T.ycp[lane] > 1);
+    uint32_t i = incl - c, ysum = 0, yhint = kNone;
+#pragma unroll
+    for (int r = 0; r < RX; ++r) {
+        const uint32_t h = hits[r], x = 32u * r + (uint32_t)lane;
+        if (!__any_sync(0xFFFFFFFFu, h)) continue;
+        const uint32_t ux = T.xm[x].w;
+        for (uint32_t b = h; b; b &= b - 1) {
+            const uint32_t uy = T.ym[__ffs(b) - 1].w;
             put_edge(a, ew.slot_of(bk, i++), min(ux, uy), max(ux, uy));
         }
+        if (!count) continue;
+        if (h) {
+            uint32_t s = (uint32_t)__popc(h);
+            for (uint32_t b = h & ymult; b; b &= b - 1) s += T.ycp[__ffs(b) - 1] - 1u;
+            T.xs[x] += s;
+            const uint32_t uy = T.ym[__ffs(h) - 1].w;
+            if (uy < ux) a.parent[ux] = uy;
+        }
+        const uint32_t m = transpose32(h, lane);
+        const uint32_t xmult = __ballot_sync(0xFFFFFFFFu, T.xcp[x] > 1);
+        if (m) {
+            ysum += (uint32_t)__popc(m);
+            for (uint32_t b = m & xmult; b; b &= b - 1) ysum += T.xcp[32 * r + __ffs(b) - 1] - 1u;
+            yhint = min(yhint, T.xm[32 * r + __ffs(m) - 1].w);
+        }
     }
+    if (ysum) {
+        atomicAdd(&a.cnt[uy_lane], ysum);
+        if (yhint < uy_lane) a.parent[uy_lane] = yhint;
+    }
+}
+
+// Inclusive sum over the lanes, and the total.
+__device__ __forceinline__ uint32_t warp_incl_sum(uint32_t v, int lane, uint32_t *total) {
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t n = __shfl_up_sync(0xFFFFFFFFu, v, d);
+        if (lane >= d) v += n;
+    }
+    *total = __shfl_sync(0xFFFFFFFFu, v, 31);
+    return v;
+}
+
+// The neighbour pairs of a small bin pair (n x-entries, m y-entries, at most 32
+// each; same: pairs of the n): bit k of a lane's word is pair lane + 32 k.  One
+// bulk append; the counts are summed in shared memory, one update per entry.
+__device__ __noinline__ void emit_pair_bits(const DistArgs &a, EdgeWriter &ew, const TileSlice &T, int lane,
+                                            uint32_t bits, bool same, uint32_t n, uint32_t m,
+                                            uint32_t xstart, uint32_t ystart) {
+    const uint32_t c = (uint32_t)__popc(bits);
+    uint32_t total;
+    const uint32_t incl = warp_incl_sum(c, lane, &total);
+    if (total == 0) return;
+    const EdgeWriter::Bulk bk = ew.reserve(a, lane, total);
+    const bool count = a.sink != kSinkGrow;
+    __syncwarp();
+    if ((uint32_t)lane < n) T.begin_x(a, lane, xstart + lane);
+    if (!same && (uint32_t)lane < m) {
+        T.begin_y(a, lane, ystart + lane);
+        T.ys[lane] = 0u;
+    }
+    __syncwarp();
+    const uint4 *ym = same ? T.xm : T.ym;
+    const uint32_t *ycp = same ? T.xcp : T.ycp;
+    uint32_t *ys = same ? T.xs : T.ys;
+    uint32_t k = incl - c;
+    for (uint32_t b = bits; b; b &= b - 1) {
+        const uint32_t p = (uint32_t)lane + 32u * ((uint32_t)__ffs(b) - 1u);
+        uint32_t i, j;
+        small_pair(p, same, n, i, j);
+        const uint32_t ux = T.xm[i].w, uy = ym[j].w, lo = min(ux, uy), hi = max(ux, uy);
+        put_edge(a, ew.slot_of(bk, k++), lo, hi);
+        if (count) {
+            atomicAdd(&T.xs[i], ycp[j]);
+            atomicAdd(&ys[j], T.xcp[i]);
+            a.parent[hi] = lo;     // any smaller neighbour (k_core)
+        }
+    }
+    T.end_x(a, n, lane);
+    if (!same && (uint32_t)lane < m && T.ys[lane]) atomicAdd(&a.cnt[T.ym[lane].w], T.ys[lane]);
+    __syncwarp();
+}
+
+// The neighbour pairs of the lanes' own tiny bin pairs (an entry of the bin with
+// another; bit of pair (i, j) as in small_pair): every pair is a constant bit,
+// so ids, copies and sums stay in registers and an entry costs one count update.
+__device__ __noinline__ void emit_tiny_bits(const DistArgs &a, EdgeWriter &ew, int lane, uint32_t bits,
+                                            uint32_t n, uint32_t start) {
+    const uint32_t c = (uint32_t)__popc(bits);
+    uint32_t total;
+    const uint32_t incl = warp_incl_sum(c, lane, &total);
+    if (total == 0) return;
+    const EdgeWriter::Bulk bk = ew.reserve(a, lane, total);
+    if (bits == 0) return;
+    const bool count = a.sink != kSinkGrow;
+    uint32_t k = incl - c;
+    uint32_t uid[kTinySide], cp[kTinySide], sum[kTinySide], hint[kTinySide];
+#pragma unroll
+    for (uint32_t i = 0; i < kTinySide; ++i) {
+        uid[i] = i < n ? __ldg(&a.meta[start + i].w) : 0u;
+        cp[i] = i < n ? __ldg(&a.ecopies[start + i]) : 0u;
+        sum[i] = 0u;
+        hint[i] = kNone;
+    }
+#pragma unroll
+    for (uint32_t j = 1; j < kTinySide; ++j)
+#pragma unroll
+        for (uint32_t i = 0; i < j; ++i)
+            if ((bits >> (j * (j - 1) / 2 + i)) & 1u) {
+                put_edge(a, ew.slot_of(bk, k++), min(uid[i], uid[j]), max(uid[i], uid[j]));
+                sum[i] += cp[j];
+                sum[j] += cp[i];
+                hint[i] = min(hint[i], uid[j]);
+                hint[j] = min(hint[j], uid[i]);
+            }
+    if (!count) return;
+#pragma unroll
+    for (uint32_t i = 0; i < kTinySide; ++i)
+        if (sum[i]) {
+            atomicAdd(&a.cnt[uid[i]], sum[i]);
+            if (hint[i] < uid[i]) a.parent[uid[i]] = hint[i];
+        }
 }
 
 template <typename K>

@@ -45,8 +45,8 @@ __device__ __forceinline__ bool join_meta_ok(const uint4 &mx, const uint4 &my, c
 // the two records by shuffles.  Canonicity of a hit is decided from the side
 // records (global loads: hits are rare).
 template <int BP, int W, int EM, bool JN>
-__device__ __forceinline__ void hamming_small(const DistArgs &a, EdgeWriter &ew, const BinPair &P,
-                                              uint32_t idx, int lane, uint64_t &pairs) {
+__device__ __forceinline__ void hamming_small(const DistArgs &a, EdgeWriter &ew, const TileSlice &T,
+                                              const BinPair &P, uint32_t idx, int lane, uint64_t &pairs) {
     constexpr int NW = BP * W;
     constexpr int R16 = (NW + 3) / 4;
     const long long t0 = a.bp_cycles ? clock64() : 0;
@@ -111,22 +111,22 @@ __device__ __forceinline__ void hamming_small(const DistArgs &a, EdgeWriter &ew,
         }
     }
     // every round's edges of the lane, one bulk append for the warp
-    emit_pair_bits(a, ew, lane, rmask, (uint32_t)lane, 32u, same, n, P.a_start, ystart);
+    emit_pair_bits(a, ew, T, lane, rmask, same, n, m, P.a_start, ystart);
     if (a.bp_cycles && lane == 0)
         atomicAdd(&a.bp_cycles[idx], (unsigned long long)(clock64() - t0));
 }
 
 template <int BP, int W, int EM, bool JN>
-__device__ __forceinline__ void hamming_small_all(const DistArgs &a, EdgeWriter &ew, int lane,
-                                                  uint64_t &pairs) {
+__device__ __forceinline__ void hamming_small_all(const DistArgs &a, EdgeWriter &ew, const TileSlice &T,
+                                                  int lane, uint64_t &pairs) {
     constexpr int R16 = (BP * W + 3) / 4;
-    const uint32_t n_small = a.ctr->n_small;
+    const uint32_t n_small = a.ctr->n_small, batch = small_batch(n_small);
     for (;;) {
         uint32_t s0 = 0;
-        if (lane == 0) s0 = atomicAdd(&a.ctr->small_cursor, kSmallBatch);
+        if (lane == 0) s0 = atomicAdd(&a.ctr->small_cursor, batch);
         s0 = __shfl_sync(0xFFFFFFFFu, s0, 0);
         if (s0 >= n_small) break;
-        const uint32_t cnt = min(kSmallBatch, n_small - s0);
+        const uint32_t cnt = min(batch, n_small - s0);
         uint32_t myidx = 0;
         BinPair myP;
         memset(&myP, 0, sizeof(BinPair));
@@ -145,7 +145,7 @@ __device__ __forceinline__ void hamming_small_all(const DistArgs &a, EdgeWriter 
                 if (!ns && (uint32_t)lane < nm) prefetch_l1(a.rec + (size_t)(nb + lane) * R16);
             }
             const BinPair P = shfl_binpair(myP, (int)g);
-            hamming_small<BP, W, EM, JN>(a, ew, P, __shfl_sync(0xFFFFFFFFu, myidx, g), lane, pairs);
+            hamming_small<BP, W, EM, JN>(a, ew, T, P, __shfl_sync(0xFFFFFFFFu, myidx, g), lane, pairs);
         }
     }
 }
@@ -211,7 +211,9 @@ __device__ __forceinline__ void hamming_tiny_all(const DistArgs &a, EdgeWriter &
             emask |= (uint32_t)ok << p;
         }
         // pass 2: one bulk append for the warp
-        emit_pair_bits(a, ew, lane, emask, 0u, 1u, true, n, P.a_start, P.a_start);
+        __syncwarp();
+        emit_tiny_bits(a, ew, lane, emask, n, P.a_start);
+        __syncwarp();
         if (a.bp_cycles) {
             // the batch's cycles, shared out by pairs (every lane takes part in
             // the reduction; lanes past the list's end hold n = 0)
@@ -229,15 +231,15 @@ __device__ __forceinline__ void hamming_tiny_all(const DistArgs &a, EdgeWriter &
 template <int BP, int W, int RX, int EM, bool FULL, bool JN>
 __device__ __forceinline__ void hamming_unit_y(const DistArgs &a, EdgeWriter &ew, const Unit &U,
                                                const uint32_t (&x)[RX][BP * W],
-                                               const uint32_t (&vmask)[RX], uint32_t valid,
-                                               uint4 *sy, uint4 *sym, uint4 *sxm, uint32_t *shq,
+                                               uint32_t valid, uint4 *sy, const TileSlice &T,
                                                const uint32_t *sseg, int lane) {
     constexpr int NW = BP * W;
     constexpr int R16 = (NW + 3) / 4;
     const uint32_t rb = (U.nx + 31) >> 5;   // r-blocks holding entries
     const uint32_t jk = U.P.v;              // segment join: the group's segment
     // a pair is a hit iff its score <= thr (score: d&(d-1) for eps 1, d for
-    // eps 0, the popcount otherwise); masked entries score >= kOff
+    // eps 0, the popcount otherwise); masked entries score >= kOff.  Lanes past
+    // the unit's end hold a copy of its first entry; their hits are dropped.
     const uint32_t thr = EM == 0 ? (uint32_t)max(U.P.eps, 0) : 0u;
     const bool neg = EM == 0 && U.P.eps < 0;       // no pair can be a neighbour
     const uint32_t same = U.P.same;
@@ -248,9 +250,11 @@ __device__ __forceinline__ void hamming_unit_y(const DistArgs &a, EdgeWriter &ew
         const uint32_t nb = min((uint32_t)kYB, U.ny - yb);
         const uint4 *src = a.rec + (size_t)(yrow0 + yb) * R16;
         for (uint32_t t = lane; t < nb * R16; t += 32) sy[t] = __ldg(src + t);
-        for (uint32_t t = lane; t < nb; t += 32) sym[t] = __ldg(a.meta + yrow0 + yb + t);
+        if ((uint32_t)lane < nb) T.begin_y(a, lane, yrow0 + yb + lane);
         __syncwarp();
-        uint32_t qn = 0;
+        uint32_t hits[RX];                // bit t: a hit with y-entry t of the batch
+#pragma unroll
+        for (int r = 0; r < RX; ++r) hits[r] = 0u;
         // y-entries inside the unit's own x range (same bin) need the mask of the
         // x-entries before them; they come first in the chunk (y ascending, all
         // after xbase), the rest pair with every x-entry of the unit
@@ -276,7 +280,7 @@ __device__ __forceinline__ void hamming_unit_y(const DistArgs &a, EdgeWriter &ew
                     uint32_t d = x[r][0] ^ y[0];
 #pragma unroll
                     for (int p = 1; p < BP; ++p) d |= x[r][p] ^ y[p];
-                    sc[r] = (EM == 2 ? d : (EM == 1 ? (d & (d - 1u)) : (uint32_t)__popc(d))) | vmask[r];
+                    sc[r] = (EM == 2 ? d : (EM == 1 ? (d & (d - 1u)) : (uint32_t)__popc(d)));
                 } else {
                     uint32_t dist = 0;
 #pragma unroll
@@ -286,15 +290,15 @@ __device__ __forceinline__ void hamming_unit_y(const DistArgs &a, EdgeWriter &ew
                         for (int p = 1; p < BP; ++p) d |= x[r][p * W + w] ^ y[p * W + w];
                         dist += __popc(d);
                     }
-                    sc[r] = dist | vmask[r];
+                    sc[r] = dist;
                 }
             }
         };
         auto record = [&](uint32_t t, const uint32_t (&sc)[RX]) {
             // with exact signatures a hit outside its canonical bin is dropped
             // here: sig_x & sig_y must be empty
-            const uint4 ym = sym[t];
-            uint32_t hit = 0;
+            const uint4 ym = T.ym[t];
+            const uint32_t bit = 1u << t;
 #pragma unroll
             for (int r = 0; r < RX; ++r)
                 if (sc[r] <= thr) {
@@ -303,7 +307,7 @@ __device__ __forceinline__ void hamming_unit_y(const DistArgs &a, EdgeWriter &ew
                         // segment join: V and J sets intersect, the group's
                         // segment is identical and no lower one is (masks of
                         // segment kk, word w at sseg[4 kk + w])
-                        const uint4 m = sxm[32 * r + lane];
+                        const uint4 m = T.xm[32 * r + lane];
                         ok = ((m.x & ym.x) | (m.y & ym.y)) != 0 && (m.z & ym.z & 0x3FFFFFFFu) != 0;
                         if (ok) {
                             const uint32_t *yw = reinterpret_cast<const uint32_t *>(sy + t * R16);
@@ -322,27 +326,11 @@ __device__ __forceinline__ void hamming_unit_y(const DistArgs &a, EdgeWriter &ew
                                  (jk < 3 || l2 != 0);
                         }
                     } else if (a.sig_exact) {
-                        const uint4 m = sxm[32 * r + lane];
+                        const uint4 m = T.xm[32 * r + lane];
                         ok = ((m.x & ym.x) | (m.y & ym.y) | (m.z & ym.z)) == 0;
                     }
-                    hit |= (uint32_t)ok << r;
+                    if (ok) hits[r] |= bit;
                 }
-            hit &= valid;
-            if (hit) shq[qn++ * 32 + lane] = (t << 8) | hit;
-        };
-        // hits are queued in pair order (the diagonal part masks x-entries from y
-        // on), and the join and exact signatures are checked as they are queued
-        const bool decided = JN || a.sig_exact;
-        auto is_edge = [&](uint32_t r, uint32_t, const uint4 &my) {
-            return canonical(a, U.P, sxm[32 * r + lane].w, my.w);
-        };
-        auto drain_if_full = [&](uint32_t room) {
-            if (__any_sync(0xFFFFFFFFu, qn + room > (uint32_t)kHitQ)) {
-                __syncwarp();
-                drain_hits(a, ew, shq, qn, sxm, sym, lane, decided, is_edge);
-                qn = 0;
-                __syncwarp();
-            }
         };
         for (uint32_t t = 0; t < tdiag; ++t) {
             uint32_t sc[RX];
@@ -355,7 +343,6 @@ __device__ __forceinline__ void hamming_unit_y(const DistArgs &a, EdgeWriter &ew
 #pragma unroll
             for (int r = 1; r < RX; ++r) z = min(z, sc[r]);
             if (z <= thr) record(t, sc);
-            drain_if_full(1);
         }
         uint32_t t = tdiag;
         for (; t + 1 < nb; t += 2) {      // two y-entries per step: twice the chains
@@ -367,7 +354,6 @@ __device__ __forceinline__ void hamming_unit_y(const DistArgs &a, EdgeWriter &ew
             for (int r = 1; r < RX; ++r) { za = min(za, sa[r]); zb = min(zb, sb[r]); }
             if (za <= thr) record(t, sa);
             if (zb <= thr) record(t + 1, sb);
-            drain_if_full(2);
         }
         if (t < nb) {
             uint32_t sc[RX];
@@ -377,9 +363,20 @@ __device__ __forceinline__ void hamming_unit_y(const DistArgs &a, EdgeWriter &ew
             for (int r = 1; r < RX; ++r) z = min(z, sc[r]);
             if (z <= thr) record(t, sc);
         }
-        if (__any_sync(0xFFFFFFFFu, qn)) {
-            __syncwarp();
-            drain_hits(a, ew, shq, qn, sxm, sym, lane, decided, is_edge);
+        uint32_t any = 0;
+#pragma unroll
+        for (int r = 0; r < RX; ++r) {
+            if (!((valid >> r) & 1u)) hits[r] = 0u;
+            any |= hits[r];
+        }
+        if (__any_sync(0xFFFFFFFFu, any)) {
+            if (!JN && !a.sig_exact) {   // wide gene lists: the bin of the lowest common genes only
+#pragma unroll
+                for (int r = 0; r < RX; ++r)
+                    for (uint32_t b = hits[r]; b; b &= b - 1)
+                        if (!canonical(a, U.P, T.xm[32 * r + lane].w, T.ym[__ffs(b) - 1].w)) hits[r] &= ~(b & (0u - b));
+            }
+            emit_batch<RX>(a, ew, T, hits, nb, lane);
         }
         __syncwarp();
     }
@@ -391,31 +388,31 @@ __device__ __forceinline__ void hamming_unit_y(const DistArgs &a, EdgeWriter &ew
 // ---------------------------------------------------------------------------
 template <int BP, int W, int RX, int EM, bool JN>
 __global__ void __launch_bounds__(kWarps * 32, (W == 1 && RX <= 2 ? 6 : (W == 1 && RX <= 4 ? 5 : 4)))
-k_hamming(DistArgs a) {
+k_hamming(const __grid_constant__ DistArgs a) {
     constexpr int NW = BP * W;                 // words per record used
     constexpr int R16 = (NW + 3) / 4;          // 16-byte words per record
     __shared__ uint4 sy[kWarps][kYB * R16];
     __shared__ uint4 sym[kWarps][kYB];            // y side records
     __shared__ uint4 sxm[kWarps][32 * RX];        // x side records
-    __shared__ uint32_t shq[kWarps][kHitQ * 32];  // deferred hits
     __shared__ uint32_t sseg[kWarps][16];         // segment join: masks of segment kk, word w
-    static_assert(RX <= 8 && kYB < (1 << 24), "hit record layout");
+    __shared__ uint32_t scp[kWarps][2 * 32 * RX + 2 * kYB];   // copies and sums (TileSlice)
+    static_assert(RX <= 8 && kYB <= 32, "hit words");
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t n_units = a.ctr->n_units, n_bp = a.ctr->n_binpairs;
+    const TileSlice T{sxm[wid], sym[wid], scp[wid], scp[wid] + 2 * 32 * RX, scp[wid] + 32 * RX,
+                      scp[wid] + 2 * 32 * RX + kYB};
     EdgeWriter ew;
     ew.init();
     uint64_t pairs = 0;
     Unit U;
     while (next_unit(a, n_units, n_bp, lane, U)) {
         uint32_t x[RX][NW];
-        uint32_t vmask[RX];          // kOff for x-entries outside the unit
         uint32_t valid = 0;
 #pragma unroll
         for (int r = 0; r < RX; ++r) {
             const uint32_t xi = (uint32_t)r * 32 + lane;
             const bool ok = xi < U.nx;
             valid |= (uint32_t)ok << r;
-            vmask[r] = ok ? 0u : kOff;
             const uint4 *src = a.rec + (size_t)(U.P.a_start + U.xbase + (ok ? xi : 0)) * R16;
 #pragma unroll
             for (int q = 0; q < R16; ++q) {
@@ -426,7 +423,7 @@ k_hamming(DistArgs a) {
                     if (4 * q + e < NW) x[r][4 * q + e] = w4[e];
             }
             if (ok) pairs += unit_pairs(U, U.xbase + xi);
-            sxm[wid][xi] = __ldg(a.meta + U.P.a_start + U.xbase + (ok ? xi : 0));
+            T.begin_x(a, xi, U.P.a_start + U.xbase + (ok ? xi : 0));
         }
         if (JN && lane < 16) {
             // segment kk = lane / 4 of length la split into j segments, word w = lane % 4
@@ -443,15 +440,14 @@ k_hamming(DistArgs a) {
         }
         __syncwarp();
         if (U.nx == (uint32_t)(32 * RX))
-            hamming_unit_y<BP, W, RX, EM, true, JN>(a, ew, U, x, vmask, valid, sy[wid], sym[wid], sxm[wid],
-                                                shq[wid], sseg[wid], lane);
+            hamming_unit_y<BP, W, RX, EM, true, JN>(a, ew, U, x, valid, sy[wid], T, sseg[wid], lane);
         else
-            hamming_unit_y<BP, W, RX, EM, false, JN>(a, ew, U, x, vmask, valid, sy[wid], sym[wid],
-                                                 sxm[wid], shq[wid], sseg[wid], lane);
+            hamming_unit_y<BP, W, RX, EM, false, JN>(a, ew, U, x, valid, sy[wid], T, sseg[wid], lane);
+        T.end_x(a, U.nx, lane);
         log_unit(a, U, lane);
     }
     // then the small bin pairs (they also fill the tail of the tiled work)
-    hamming_small_all<BP, W, EM, JN>(a, ew, lane, pairs);
+    hamming_small_all<BP, W, EM, JN>(a, ew, T, lane, pairs);
     hamming_tiny_all<BP, W, EM, JN>(a, ew, lane, pairs);
     finish(a, ew, pairs, lane);
 }

@@ -71,7 +71,7 @@ enum BufId {
     bBpSorted, bBpUnits, bClsHist, bPred, bEdges, bCnt, bUCore,
     bParent, bBMin, bRootFlag, bUidFirst, bDepth, bScanPart, bClone, bCore, bCopies, bUniques,
     bCtr, bVTab, bJTab, bSigAnd, bUClass, bEntMeta, bCallAux, bCallTab, bCallRef, bCallTodo, bBpSmall,
-    bJnTab, bJnISlot, bJnStart, bJnCur, bJnBpIdx, bJnPos, bNumBufs
+    bJnTab, bJnISlot, bJnStart, bJnCur, bJnBpIdx, bJnPos, bEntCopies, bNumBufs
 };
 
 }  // namespace
@@ -739,6 +739,8 @@ idb_status alloc_entries(Pipeline &pl, uint64_t n_entries) {
     TRY(ensure(c, bEntUid, 4 * pl.P.cap_entries));
     TRY(ensure(c, bEntRec, (size_t)pl.P.RS * pl.P.cap_entries));
     TRY(ensure(c, bEntMeta, 16 * pl.P.cap_entries));
+    TRY(ensure(c, bEntCopies, 4 * pl.P.cap_entries));
+    pl.B.ent_copies = ptr<uint32_t>(c, bEntCopies);
     pl.B.ent_meta = ptr<uint4>(c, bEntMeta);
     pl.B.ent_uid = ptr<uint32_t>(c, bEntUid);
     pl.B.ent_rec = ptr<uint4>(c, bEntRec);
@@ -933,6 +935,7 @@ idb_status run_phases(Pipeline &pl, bool eager, bool stop_after_schedule = false
         if (!eager) break;
         TRY(read_counters(pl));
         const Counters &h = *c->h_ctr;
+        P.union_sample = h.edge_reserved >= kUnionSampleMin;
         if (!(h.error & kErrEdgeOverflow)) break;
         // grow to the exact requirement and sweep again, or stream
         const uint64_t need = (uint64_t)h.edge_reserved + 64ull * kEdgeChunk * 1024;

@@ -9,12 +9,16 @@
 namespace idb {
 
 constexpr uint32_t kNone = 0xFFFFFFFFu;
+constexpr uint32_t kNonCore = 0x80000000u;   // in a union-find parent: the unique is not core
+                                             // (unique ids stay below 2^31)
 constexpr int kMaxGeneWords = 8;        // 512 reference genes per gene column
 constexpr int kFastMaxCodes = 32;       // alphabet of the fast (bit-plane) path
 constexpr int kFastMaxWords = 4;        // 128 residues on the fast path
 constexpr int kGenericMaxLen = 1024;    // Levenshtein on the generic path
 constexpr int kDepthMax = 50;           // tree-depth histogram cap (cuda/PSDBSCAN.hcu:1029)
 constexpr uint32_t kEdgeChunk = 256;    // edge slots reserved per warp at a time
+constexpr uint32_t kUnionSample = 32;   // long edge lists: this fraction of them is merged first
+constexpr uint32_t kUnionSampleMin = 1u << 20;   // edge slots from which they are
 constexpr uint32_t kSpinCap = 1u << 22; // bound of every device-side retry loop
 constexpr int kMaxRowChunks = 8;        // host columns uploaded in at most this many row chunks
 // Bin pairs with at most kSmallSide entries on each side (Hamming fast path) are
@@ -216,6 +220,7 @@ struct Plan {
     uint32_t join_smax = 1;                       // most segments of any length
     bool streamed = false;                        // neighbour pairs not stored: the
                                                   // distance work runs twice
+    bool union_sample = false;                    // unions start with a sample of the edges
     uint64_t edge_budget = 0;                     // bytes for the edge list (0: no limit)
     // row chunks of the front end: host columns arrive chunk by chunk and the
     // gene-bitset and duplicate kernels of chunk k wait only for its rows
@@ -269,6 +274,7 @@ struct Buffers {
     unsigned long long *sig_and = nullptr;          // [2*nbins] AND of V / J signatures
     uint32_t *ent_uid = nullptr;                    // [cap_entries]
     uint4 *ent_meta = nullptr;                      // [cap_entries] {sigV lo, sigV hi, sigJ, uid}
+    uint32_t *ent_copies = nullptr;                 // [cap_entries] copies of the entry's unique
     uint4 *ent_rec = nullptr;                       // [cap_entries * RS/16]
     uint32_t *bp_count = nullptr;                   // [nbins+1]
     BinPair *bp = nullptr, *bp_sorted = nullptr;    // [cap_binpairs]
@@ -346,6 +352,8 @@ void launch_schedule(const Plan &P, const Buffers &B, cudaStream_t s);
 void launch_distance(const Plan &P, const Buffers &B, int grid, cudaStream_t s,
                      uint32_t sink = kSinkEdges);
 void launch_count_admissible(const Plan &P, const Buffers &B, cudaStream_t s);
+// counts, forest and border minima before a distance sweep that counts
+void launch_graph_init(const Plan &P, const Buffers &B, cudaStream_t s);
 // core_out: when set, the row core flags are written right after the core
 // marking and the event is recorded there (an external record node in a
 // captured graph), so their copy to the host can start before the labels.

@@ -160,7 +160,8 @@ k_bin_fill(BinGeom g, const Counters *__restrict__ ctr,
                            const int64_t *__restrict__ seq_off, const uint8_t *__restrict__ codemap,
                            const uint32_t *__restrict__ bin_start, uint32_t *__restrict__ cursor,
                            uint32_t *__restrict__ ent_uid, uint4 *__restrict__ ent_rec,
-                           uint4 *__restrict__ ent_meta,
+                           uint4 *__restrict__ ent_meta, const uint32_t *__restrict__ ucopies,
+                           uint32_t *__restrict__ ent_copies,
                            uint32_t rs16, int planes, uint32_t W, uint64_t cap_entries,
                            uint32_t *err) {
     __shared__ uint8_t cm[256];
@@ -169,7 +170,7 @@ k_bin_fill(BinGeom g, const Counters *__restrict__ ctr,
     const uint32_t nu = ctr->n_uniques;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < nu; u += stride) {
-        const uint32_t row = urow[u], L = ulen[u], r = urep[u];
+        const uint32_t row = urow[u], L = ulen[u], r = urep[u], copies = ucopies[u];
         if (!g.in_range(L)) continue;
         const uint8_t *s = seq + seq_off[row];
         // the record depends on the unique only: build it once (registers when it
@@ -210,6 +211,7 @@ k_bin_fill(BinGeom g, const Counters *__restrict__ ctr,
                                              __popc(grp & ((1u << lane) - 1u));
                         if (pos >= cap_entries) { atomicOr(err, kErrEntryOverflow); continue; }
                         ent_uid[pos] = u;
+                        ent_copies[pos] = copies;
                         // side record: signature below (v, j) and the unique id
                         ent_meta[pos] = make_uint4((uint32_t)sv, (uint32_t)(sv >> 32), (uint32_t)sj, u);
                         uint4 *dst = ent_rec + pos * rs16;
@@ -622,7 +624,8 @@ k_join_fill(BinGeom g, const Counters *__restrict__ ctr, const uint32_t *__restr
             const uint64_t *__restrict__ vbits, const uint64_t *__restrict__ jbits,
             const uint32_t *__restrict__ start,
             const uint32_t *__restrict__ irank, uint32_t smax, uint4 *__restrict__ ent_rec,
-            uint4 *__restrict__ ent_meta, int planes, uint32_t W, uint64_t cap_entries,
+            uint4 *__restrict__ ent_meta, const uint32_t *__restrict__ ucopies,
+            uint32_t *__restrict__ ent_copies, int planes, uint32_t W, uint64_t cap_entries,
             uint32_t *err) {
     __shared__ uint8_t cm[256];
     for (int k = threadIdx.x; k < 256; k += blockDim.x) cm[k] = codemap[k];
@@ -648,6 +651,7 @@ k_join_fill(BinGeom g, const Counters *__restrict__ ctr, const uint32_t *__restr
             const uint64_t vb = vbits[(size_t)row * g.VW];
             const uint32_t jb = (uint32_t)jbits[(size_t)row * g.JW];
             ent_meta[pos] = make_uint4((uint32_t)vb, (uint32_t)(vb >> 32), jb | (k << 30), u);
+            ent_copies[pos] = ucopies[u];
             uint4 *dst = ent_rec + pos * RSC;
 #pragma unroll
             for (int q = 0; q < RSC; ++q) dst[q] = rec[q];
@@ -760,7 +764,7 @@ void launch_fill(const Plan &P, const Buffers &B, cudaStream_t s) {
             kern<<<grid_wave(kern, P.N, kThreads), kThreads, 0, s>>>(g, B.ctr, B.urow, B.ulen, B.seq, B.seq_off,
                                                      B.codemap, B.eps_tab, B.jn_islot, B.vbits,
                                                      B.jbits, B.jn_start, B.jn_cur, P.join_smax,
-                                                     B.ent_rec, B.ent_meta, planes, P.W,
+                                                     B.ent_rec, B.ent_meta, B.ucopies, B.ent_copies, planes, P.W,
                                                      P.cap_entries, &B.ctr->error);
         };
         switch (P.RS / 16) {   // Hamming fast path: 1..8 words of bit planes
@@ -783,7 +787,7 @@ void launch_fill(const Plan &P, const Buffers &B, cudaStream_t s) {
     auto go = [&](auto kern) {
         kern<<<grid_wave(kern, P.N, kThreads), kThreads, 0, s>>>(
             g, B.ctr, B.urow, B.ulen, B.urep, B.uclass, B.sig_and, B.vbits, B.jbits, B.seq, B.seq_off,
-            B.codemap, B.bin_hist, B.bin_cursor, B.ent_uid, B.ent_rec, B.ent_meta, rs16, planes, P.W,
+            B.codemap, B.bin_hist, B.bin_cursor, B.ent_uid, B.ent_rec, B.ent_meta, B.ucopies, B.ent_copies, rs16, planes, P.W,
             P.cap_entries, &B.ctr->error);
     };
     switch (rs16) {

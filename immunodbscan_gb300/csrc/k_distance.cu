@@ -372,7 +372,7 @@ static DistArgs make_args(const Plan &P, const Buffers &B) {
     a.sink = kSinkEdges;
     a.cnt = B.cnt;
     a.ucopies = B.ucopies;
-    a.ucore = B.ucore;
+    a.ecopies = B.ent_copies;
     a.parent = B.parent;
     a.bmin = B.bmin;
     return a;
@@ -398,6 +398,7 @@ void launch_distance(const Plan &P, const Buffers &B, int grid, cudaStream_t s, 
         a.edges = nullptr;
         a.cap_edges = ~0ull;
     }
+    if (sink != kSinkGrow) launch_graph_init(P, B, s);   // a repeated sweep counts anew
     cudaMemsetAsync(&B.ctr->unit_cursor, 0, sizeof(uint32_t), s);
     cudaMemsetAsync(&B.ctr->small_cursor, 0, sizeof(uint32_t), s);
     cudaMemsetAsync(&B.ctr->tiny_cursor, 0, sizeof(uint32_t), s);

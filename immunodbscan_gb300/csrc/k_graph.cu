@@ -13,7 +13,7 @@
 //  tree depths       cuda/PSDBSCAN.hcu:154-177, 1020-1040
 //
 // Here the neighbour pairs found by the distance kernel form an edge list.
-// Counts are accumulated per edge; core-core edges are merged by unions that
+// Counts come with it (PairSums, count_pair); core-core edges are merged by unions that
 // hook the larger root under the smaller one with atomicCAS while find()
 // halves paths, so every component's root is its minimum core index, as in the
 // reference.  In the same pass every core-to-non-core edge offers its core end
@@ -54,27 +54,19 @@ __global__ void k_graph_init(const Counters *__restrict__ ctr, const uint32_t *_
     }
 }
 
-// count pass: copies-weighted neighbour counts (S5)
-__global__ void k_count(const Counters *__restrict__ ctr, uint64_t cap, const uint2 *__restrict__ edges,
-                        const uint32_t *__restrict__ ucopies, uint32_t *__restrict__ cnt) {
-    const uint32_t ne = edge_slots(ctr, cap);
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += stride) {
-        const uint2 ed = edges[e];
-        if (ed.x == kNone) continue;
-        atomicAdd(&cnt[ed.x], ucopies[ed.y]);
-        atomicAdd(&cnt[ed.y], ucopies[ed.x]);
-    }
-}
-
+// Core flags (S5) and the forest the unions start from: every core is its own
+// root, or under the smaller neighbour the distance kernel left in its parent
+// when that is core too (such an edge is a union); a non-core unique is marked.
 __global__ void k_core(const Counters *__restrict__ ctr0, Counters *ctr, const uint32_t *__restrict__ cnt,
-                       uint32_t min_pts, uint32_t *__restrict__ ucore) {
+                       uint32_t min_pts, uint32_t *__restrict__ ucore, uint32_t *parent) {
     const uint32_t nu = ctr0->n_uniques;
     const uint32_t stride = gridDim.x * blockDim.x;
     uint32_t local = 0;
     for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < nu; u += stride) {
         const uint32_t c = cnt[u] >= min_pts;
         ucore[u] = c;
+        const uint32_t p = parent[u];
+        parent[u] = !c ? u | kNonCore : (p != u && cnt[p] < min_pts ? u : p);
         local += c;
     }
 #pragma unroll
@@ -86,41 +78,94 @@ __device__ __forceinline__ uint32_t uf_find(uint32_t *p, uint32_t x) {
     volatile uint32_t *vp = p;
     while (true) {   // parent[y] <= y always, so x strictly decreases: terminates
         const uint32_t px = vp[x];
-        if (px == x) return x;
+        if (px >= x) return px == x ? x : kNone;   // kNone: not a core's parent
         const uint32_t ppx = vp[px];
-        if (ppx == px) return px;
+        if (ppx >= px) return ppx == px ? px : kNone;
         vp[x] = ppx;           // path halving
         x = ppx;
     }
 }
 
-// Core-core edges are merged (S6); an edge with one core end offers the core
-// to its non-core end, which keeps the minimum (the border rule).
-__global__ void k_union(Counters *ctr, uint64_t cap, const uint2 *__restrict__ edges,
-                        const uint32_t *__restrict__ ucore, uint32_t *parent,
-                        uint32_t *__restrict__ bmin) {
-    const uint32_t ne = edge_slots(ctr, cap);
+__device__ __forceinline__ void uf_merge(Counters *ctr, uint32_t *parent, uint32_t a, uint32_t b) {
+    uint32_t it = 0;
+    for (; it < kSpinCap; ++it) {
+        uint32_t ra = uf_find(parent, a), rb = uf_find(parent, b);
+        if (ra == rb) break;
+        if (ra < rb) { const uint32_t t = ra; ra = rb; rb = t; }
+        if (ra == kNone) { it = kSpinCap; break; }
+        // hook the larger root under the smaller one
+        if (atomicCAS(&parent[ra], ra, rb) == ra) break;
+        a = ra;
+        b = rb;
+    }
+    if (it == kSpinCap) atomicOr(&ctr->error, kErrUnionStall);
+}
+
+// Long edge lists: from that forest and the core-core edges of every
+// kUnionSample-th slot, each followed by k_flatten (every core at its root), the
+// pass over all edges finds nearly every pair already under one parent (dense
+// components are connected by a small part of their edges), instead of millions
+// of edges hooking and walking the same few trees at once.
+__global__ void __launch_bounds__(kThreads)
+k_union_sample(Counters *ctr, uint64_t cap, const uint2 *__restrict__ edges, uint32_t *parent) {
+    const uint32_t ne = edge_slots(ctr, cap) / kUnionSample;
     const uint32_t stride = gridDim.x * blockDim.x;
-    uint32_t n_cc = 0;
-    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += stride) {
-        const uint2 ed = edges[e];
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ne; i += stride) {
+        const uint2 ed = edges[(uint64_t)i * kUnionSample + kUnionSample / 2];
         if (ed.x == kNone) continue;
-        const uint32_t cx = ucore[ed.x], cy = ucore[ed.y];
-        if (cx != cy) { atomicMin(&bmin[cx ? ed.y : ed.x], cx ? ed.x : ed.y); continue; }
-        if (!cx) continue;
-        ++n_cc;
-        uint32_t a = ed.x, b = ed.y;
-        uint32_t it = 0;
-        for (; it < kSpinCap; ++it) {
-            uint32_t ra = uf_find(parent, a), rb = uf_find(parent, b);
-            if (ra == rb) break;
-            if (ra < rb) { const uint32_t t = ra; ra = rb; rb = t; }
-            // hook the larger root under the smaller one
-            if (atomicCAS(&parent[ra], ra, rb) == ra) break;
-            a = ra;
-            b = rb;
+        const uint32_t px = __ldcg(parent + ed.x), py = __ldcg(parent + ed.y);
+        if (((px | py) & kNonCore) || px == py) continue;
+        // neighbouring slots hold edges of one group: one merge per pair of trees
+        const unsigned long long key = ((unsigned long long)px << 32) | py;
+        const uint32_t grp = __match_any_sync(__activemask(), key);
+        if ((threadIdx.x & 31) == (uint32_t)__ffs(grp) - 1) uf_merge(ctr, parent, px, py);
+    }
+}
+
+__global__ void k_flatten(const Counters *__restrict__ ctr, uint32_t *parent) {
+    const uint32_t nu = ctr->n_uniques;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    volatile uint32_t *vp = parent;
+    for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < nu; u += stride) {
+        uint32_t r = vp[u];
+        if (r & kNonCore) continue;
+        uint32_t pr = vp[r];
+        while (pr < r) { r = pr; pr = vp[r]; }   // strictly decreasing, terminates
+        vp[u] = r;
+    }
+}
+
+// Core-core edges are merged (S6); an edge with one core end offers the core
+// to its non-core end, which keeps the minimum (the border rule).  A parent
+// carries its unique's core flag (kNonCore), so one load per end decides the
+// border edges and the core ones already under one parent; these loads may be
+// served from L1 (a stale parent is an ancestor too, and two equal ones still
+// mean one component).  Four edges' loads in flight per thread.
+__global__ void __launch_bounds__(kThreads)
+k_union(Counters *ctr, uint64_t cap, const uint2 *__restrict__ edges, uint32_t *parent,
+        uint32_t *__restrict__ bmin) {
+    const uint32_t ne = edge_slots(ctr, cap) & ~3u;   // reserved in chunks of 256
+    const uint64_t stride = 4ull * gridDim.x * blockDim.x;
+    uint32_t n_cc = 0;
+    for (uint64_t e0 = 4ull * (blockIdx.x * blockDim.x + threadIdx.x); e0 < ne; e0 += stride) {
+        const uint4 v0 = __ldcs(reinterpret_cast<const uint4 *>(edges + e0));
+        const uint4 v1 = __ldcs(reinterpret_cast<const uint4 *>(edges + e0 + 2));
+        const uint2 ed[4] = {{v0.x, v0.y}, {v0.z, v0.w}, {v1.x, v1.y}, {v1.z, v1.w}};
+        uint32_t px[4], py[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const bool pad = ed[k].x == kNone;
+            px[k] = pad ? kNonCore : parent[ed[k].x];
+            py[k] = pad ? kNonCore : parent[ed[k].y];
         }
-        if (it == kSpinCap) atomicOr(&ctr->error, kErrUnionStall);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t nx = px[k] & kNonCore, ny = py[k] & kNonCore;
+            if (nx != ny) { atomicMin(&bmin[nx ? ed[k].x : ed[k].y], nx ? ed[k].y : ed[k].x); continue; }
+            if (nx) continue;
+            ++n_cc;
+            if (px[k] != py[k]) uf_merge(ctr, parent, px[k], py[k]);
+        }
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) n_cc += __shfl_xor_sync(0xFFFFFFFFu, n_cc, d);
@@ -171,7 +216,7 @@ __global__ void k_compress(const Counters *__restrict__ ctr, const uint32_t *__r
         uint32_t r = u;
         if (ucore[u]) {
             uint32_t pr = vp[r];
-            while (pr != r) {   // parent[y] <= y: strictly decreasing, terminates
+            while (pr < r) {   // parent[y] <= y: strictly decreasing, terminates
                 r = pr;
                 pr = vp[r];
             }
@@ -233,18 +278,27 @@ __global__ void k_uniques_out(const Counters *__restrict__ ctr, const uint32_t *
 
 }  // namespace
 
+void launch_graph_init(const Plan &P, const Buffers &B, cudaStream_t s) {
+    k_graph_init<<<grid_wave(k_graph_init, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ucopies, B.cnt, B.parent, B.bmin);
+}
+
 void launch_graph(const Plan &P, const Buffers &B, bool trees, cudaStream_t s, cudaEvent_t core_out) {
     const uint64_t ecap = P.cap_edges;
     const int gu = grid_for(P.N);
-    k_graph_init<<<grid_wave(k_graph_init, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ucopies, B.cnt, B.parent, B.bmin);
-    k_count<<<grid_wave(k_count, ecap, kThreads), kThreads, 0, s>>>(B.ctr, ecap, B.edges, B.ucopies, B.cnt);
-    k_core<<<grid_wave(k_core, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ctr, B.cnt, P.min_pts, B.ucore);
+    k_core<<<grid_wave(k_core, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ctr, B.cnt, P.min_pts, B.ucore, B.parent);
     if (core_out) {   // the row core flags now, and an event for their copy
         launch_outputs(P, B, s, kOutCore);
         cudaEventRecordWithFlags(core_out, s, cudaEventRecordExternal);
     }
     // unions of core-core edges; each non-core unique keeps its minimum core neighbour
-    k_union<<<grid_wave(k_union, ecap, kThreads), kThreads, 0, s>>>(B.ctr, ecap, B.edges, B.ucore, B.parent, B.bmin);
+    if (P.union_sample) {
+        k_flatten<<<grid_wave(k_flatten, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.parent);
+        // few threads: with a full wave in flight most of them try to hook the same
+        // few trees at once, and those atomics go one by one (21M edges: 533 us)
+        k_union_sample<<<2 * sm_count(), kThreads, 0, s>>>(B.ctr, ecap, B.edges, B.parent);
+        k_flatten<<<grid_wave(k_flatten, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.parent);
+    }
+    k_union<<<grid_wave(k_union, ecap / 4, kThreads), kThreads, 0, s>>>(B.ctr, ecap, B.edges, B.parent, B.bmin);
     if (trees) {
         cudaMemsetAsync(B.depth_hist, 0, sizeof(uint32_t) * (kDepthMax + 1), s);
         k_depth<<<gu, kThreads, 0, s>>>(P.N, B.row2uid, B.urow, B.ucore, B.bmin, B.parent,
@@ -263,9 +317,8 @@ void launch_graph(const Plan &P, const Buffers &B, bool trees, cudaStream_t s, c
 // core neighbour; depths, compression and labels as above.  The sweep-local
 // statistics are cleared between the sweeps so that they count one sweep.
 void launch_streamed_sweeps(const Plan &P, const Buffers &B, cudaStream_t s) {
-    k_graph_init<<<grid_wave(k_graph_init, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ucopies, B.cnt, B.parent, B.bmin);
     launch_distance(P, B, 0, s, kSinkCount);
-    k_core<<<grid_wave(k_core, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ctr, B.cnt, P.min_pts, B.ucore);
+    k_core<<<grid_wave(k_core, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ctr, B.cnt, P.min_pts, B.ucore, B.parent);
     cudaMemsetAsync(&B.ctr->pairs_evaluated, 0, sizeof(B.ctr->pairs_evaluated), s);
     cudaMemsetAsync(&B.ctr->n_edges, 0, sizeof(B.ctr->n_edges), s);
     cudaMemsetAsync(&B.ctr->edge_reserved, 0, sizeof(B.ctr->edge_reserved), s);

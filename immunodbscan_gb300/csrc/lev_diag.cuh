@@ -24,7 +24,6 @@ namespace {
 // A unit with at most this many x-entries is scored pair by pair: a pair read from
 // L1 costs about twice a tiled one, and a tile would leave 3/4 of the lanes idle.
 constexpr uint32_t kThinX = 8;
-constexpr uint32_t kLevHitQ = 16;   // queued (y, hits) records per lane
 
 template <int BP, int W>
 struct LevShape {
@@ -33,7 +32,7 @@ struct LevShape {
     static constexpr int YMax = NW;              // 16-byte words of a staged y (4 diagonals)
     // y-records staged per batch, so that a block's static shared memory stays
     // below 48 KB
-    static constexpr int YB = NW <= 8 ? 64 : (NW <= 15 ? 32 : 16);
+    static constexpr int YB = NW <= 15 ? kYB : 16;
 };
 
 template <int BP, int W>
@@ -137,21 +136,9 @@ __device__ __forceinline__ bool lev_is_edge(const DistArgs &a, const BinPair &P,
 // A warp's shared memory.
 struct LevSlice {
     uint4 *sy;       // staged y-records, one shifted copy per diagonal
-    uint4 *sym;      // y side records
-    uint4 *sxm;      // x side records
-    uint32_t *shq;   // deferred hits
     uint32_t *seg;   // segment join: masks of the look-ups (LevLookups)
+    TileSlice T;
 };
-
-// Out of line: one copy for every unit loop.
-__device__ __noinline__ void lev_drain(const DistArgs &a, EdgeWriter &ew, const BinPair &P, const LevSlice &S,
-                                       uint32_t qn, int lane) {
-    drain_hits(a, ew, S.shq, qn, S.sxm, S.sym, lane, a.join && a.vj_meta,
-               [&](uint32_t r, uint32_t, const uint4 &my) {
-                   const uint4 mx = S.sxm[32 * r + lane];
-                   return a.join ? vj_intersect(a, mx.w, my.w) : canonical_meta(a, P, mx, my);
-               });
-}
 
 // The look-ups of a length pair (k_lev_join.cu) are the cells of the diagonal test:
 // segment k at shift delta is diagonal d = -delta, and x holds it iff the mask of
@@ -245,7 +232,7 @@ __device__ __forceinline__ void lev_unit(const DistArgs &a, EdgeWriter &ew, cons
     static_assert(Y16 <= Sh::YMax, "staged y-record size");
     using Lk = LevLookups<E, G, W>;
     const bool same = U.P.same != 0;
-    uint32_t x[RX][NW], vmask[RX];
+    uint32_t x[RX][NW];
     // segment join: the group's look-up, plus a per-entry shift for the classes
     // that looked it up (the group's own uniques: no shift, the middle one)
     const int kg = U.P.v;
@@ -263,9 +250,8 @@ __device__ __forceinline__ void lev_unit(const DistArgs &a, EdgeWriter &ew, cons
         const uint32_t xi = (uint32_t)r * 32 + lane;
         const bool ok = xi < U.nx;
         const uint32_t row = U.P.a_start + U.xbase + (ok ? xi : 0);
-        vmask[r] = ok ? 0u : kOff;
         load_planes<BP, W>(a.rec + (size_t)row * Sh::R16, x[r]);
-        S.sxm[xi] = __ldg(a.meta + row);
+        S.T.begin_x(a, xi, row);
         if (ok) pairs += unit_pairs(U, U.xbase + xi);
     }
     const uint32_t yrow0 = (same ? U.P.a_start : U.P.b_start) + U.ybase;
@@ -293,46 +279,16 @@ __device__ __forceinline__ void lev_unit(const DistArgs &a, EdgeWriter &ew, cons
 #pragma unroll
             for (int k = 0; k < Y16; ++k)
                 S.sy[t * Y16 + k] = make_uint4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
-            S.sym[t] = __ldg(a.meta + yrow0 + yb + t);
+            S.T.begin_y(a, t, yrow0 + yb + t);
         }
         __syncwarp();
         // y-entries inside the unit's own x range (same bin) need the mask of the
         // x-entries before them; they come first in the chunk
         uint32_t tdiag = 0;
         if (same && U.ybase + yb < U.xbase + U.nx) tdiag = min(nb, U.xbase + U.nx - (U.ybase + yb));
-        uint32_t qn = 0;
-        // Segment join: the queued pairs that are emitted from this group.  Checked
-        // here and not in the loop below, where one hit in a warp would make all of
-        // it wait for the check (2M rows, 0.15e9 neighbours: 9.2 ms in the loop).
-        auto flush = [&]() {
-            __syncwarp();
-            if (a.join)
-                for (uint32_t k = 0; k < qn; ++k) {
-                    const uint32_t e = S.shq[k * 32 + lane], t = e >> 8;
-                    const uint4 my = S.sym[t];
-                    const uint32_t *ys = reinterpret_cast<const uint32_t *>(S.sy + t * Y16);
-                    uint32_t keep = 0;
+        uint32_t hits[RX];                // bit t: within eps of y-entry t of the batch
 #pragma unroll
-                    for (int r = 0; r < RX; ++r)
-                        if ((e >> r) & 1u) {
-                            uint32_t D[Dg::n][W];
-#pragma unroll
-                            for (int q = 0; q < Dg::n; ++q)
-#pragma unroll
-                                for (int w = 0; w < W; ++w) {
-                                    uint32_t d = x[r][w] ^ ys[q * NW + w];
-#pragma unroll
-                                    for (int p = 1; p < BP; ++p) d |= x[r][p * W + w] ^ ys[q * NW + p * W + w];
-                                    D[q][w] = d;
-                                }
-                            keep |= (uint32_t)join_edge(D, S.sxm[32 * r + lane], my) << r;
-                        }
-                    S.shq[k * 32 + lane] = (t << 8) | keep;
-                }
-            lev_drain(a, ew, U.P, S, qn, lane);
-            qn = 0;
-            __syncwarp();
-        };
+        for (int r = 0; r < RX; ++r) hits[r] = 0u;
         for (uint32_t t = 0; t < nb; ++t) {
             uint32_t y[4 * Y16];
 #pragma unroll
@@ -353,7 +309,7 @@ __device__ __forceinline__ void lev_unit(const DistArgs &a, EdgeWriter &ew, cons
                         for (int p = 1; p < BP; ++p) d |= x[r][p * W + w] ^ y[q * NW + p * W + w];
                         D[q][w] = d;
                     }
-                sc[r] = lev_diag<W, E, G>(D) | vmask[r];
+                sc[r] = lev_diag<W, E, G>(D);
             }
             if (t < tdiag) {
                 const uint32_t nact = U.ybase + yb + t - U.xbase;   // x-entries before y
@@ -361,17 +317,50 @@ __device__ __forceinline__ void lev_unit(const DistArgs &a, EdgeWriter &ew, cons
                 for (int r = 0; r < RX; ++r)
                     if ((uint32_t)r * 32 + lane >= nact) sc[r] |= kOff;
             }
-            uint32_t hit = 0;
 #pragma unroll
             for (int r = 0; r < RX; ++r)
-                hit |= (uint32_t)(sc[r] == 0) << r;
-            if (hit) S.shq[qn++ * 32 + lane] = (t << 8) | hit;
-            // one flush in the code: the queue is full, or the batch ends
-            const bool end = t + 1 == nb;
-            if (__any_sync(0xFFFFFFFFu, qn == kLevHitQ || (end && qn))) flush();
+                if (sc[r] == 0) hits[r] |= 1u << t;
+        }
+        uint32_t any = 0;
+#pragma unroll
+        for (int r = 0; r < RX; ++r) {    // lanes past the unit's end hold a copy of its first entry
+            if ((uint32_t)r * 32 + lane >= U.nx) hits[r] = 0u;
+            any |= hits[r];
+        }
+        if (__any_sync(0xFFFFFFFFu, any)) {
+            // Which hits are emitted here.  Checked per batch, not in the loop
+            // above, where one hit in a warp would make all of it wait for the
+            // check (2M rows, 0.15e9 neighbours: 9.2 against 7.4 ms).
+#pragma unroll
+            for (int r = 0; r < RX; ++r) {
+                const uint4 mx = S.T.xm[32 * r + lane];
+                for (uint32_t b = hits[r]; b; b &= b - 1) {
+                    const uint32_t t = (uint32_t)__ffs(b) - 1u;
+                    const uint4 my = S.T.ym[t];
+                    bool ok;
+                    if (a.join) {
+                        const uint32_t *ys = reinterpret_cast<const uint32_t *>(S.sy + t * Y16);
+                        uint32_t D[Dg::n][W];
+#pragma unroll
+                        for (int q = 0; q < Dg::n; ++q)
+#pragma unroll
+                            for (int w = 0; w < W; ++w) {
+                                uint32_t d = x[r][w] ^ ys[q * NW + w];
+#pragma unroll
+                                for (int p = 1; p < BP; ++p) d |= x[r][p * W + w] ^ ys[q * NW + p * W + w];
+                                D[q][w] = d;
+                            }
+                        ok = join_edge(D, mx, my) && (a.vj_meta || vj_intersect(a, mx.w, my.w));
+                    } else {
+                        ok = canonical_meta(a, U.P, mx, my);
+                    }
+                    if (!ok) hits[r] &= ~(1u << t);
+                }
+            }
+            emit_batch<RX>(a, ew, S.T, hits, nb, lane);
         }
     }
-    __syncwarp();
+    S.T.end_x(a, U.nx, lane);
 }
 
 // A unit whose x-chunk fills at most one 32-lane block takes the one-block loop.
@@ -382,45 +371,43 @@ __device__ __forceinline__ void lev_unit_rx(const DistArgs &a, EdgeWriter &ew, c
     else lev_unit<BP, W, RX, E, G>(a, ew, U, S, lane, pairs);
 }
 
-// Pairs of nx x-entries with ny y-entries (same: pairs of the nx entries), lanes
-// taking pairs and reading their records from L1.
+// Pairs of n x-entries with m y-entries, at most 32 each (same: pairs of the n),
+// lanes taking pairs and reading their records from L1.
 template <int BP, int W>
-__device__ __forceinline__ void lev_pair_block(const DistArgs &a, EdgeWriter &ew, const BinPair &P, bool same,
-                                               uint32_t xstart, uint32_t nx, uint32_t ystart, uint32_t ny,
-                                               int lane) {
+__device__ __forceinline__ void lev_pair_block(const DistArgs &a, EdgeWriter &ew, const TileSlice &T,
+                                               const BinPair &P, bool same, uint32_t xstart, uint32_t n,
+                                               uint32_t ystart, uint32_t m, int lane) {
     constexpr int R16 = LevShape<BP, W>::R16;
-    const uint32_t npairs = same ? nx * (nx - 1) / 2 : nx * ny;
-    for (uint32_t b0 = 0; b0 < npairs; b0 += 1024) {
-        uint32_t rmask = 0;           // bit i: the lane's pair of round i is an edge
-        for (uint32_t p0 = b0; p0 < min(npairs, b0 + 1024); p0 += 32) {
-            const uint32_t p = p0 + lane;
-            if (p >= npairs) break;
-            uint32_t i, j;
-            small_pair(p, same, nx, i, j);
-            const uint32_t xrow = xstart + i, yrow = ystart + j;
-            if (lev_pair<BP, W>(a.rec + (size_t)xrow * R16, a.rec + (size_t)yrow * R16, (uint32_t)P.eps,
-                                (uint32_t)(P.lb - P.la)) == 0 &&
-                lev_is_edge<BP, W>(a, P, xrow, yrow, __ldg(a.meta + xrow), __ldg(a.meta + yrow)))
-                rmask |= 1u << ((p0 - b0) >> 5);
-        }
-        __syncwarp();
-        emit_pair_bits(a, ew, lane, rmask, b0 + (uint32_t)lane, 32u, same, nx, xstart, ystart);
+    const uint32_t npairs = same ? n * (n - 1) / 2 : n * m;
+    uint32_t rmask = 0;           // bit i: the lane's pair of round i is an edge
+    for (uint32_t p0 = 0; p0 < npairs; p0 += 32) {
+        const uint32_t p = p0 + lane;
+        if (p >= npairs) break;
+        uint32_t i, j;
+        small_pair(p, same, n, i, j);
+        const uint32_t xrow = xstart + i, yrow = ystart + j;
+        if (lev_pair<BP, W>(a.rec + (size_t)xrow * R16, a.rec + (size_t)yrow * R16, (uint32_t)P.eps,
+                            (uint32_t)(P.lb - P.la)) == 0 &&
+            lev_is_edge<BP, W>(a, P, xrow, yrow, __ldg(a.meta + xrow), __ldg(a.meta + yrow)))
+            rmask |= 1u << (p0 >> 5);
     }
+    __syncwarp();
+    emit_pair_bits(a, ew, T, lane, rmask, same, n, m, xstart, ystart);
 }
 
 // Small bin pairs (at most kSmallSide entries a side): a warp each, lanes take
 // pairs and read their records from L1 (the next bin pair's are prefetched).
 template <int BP, int W>
-__device__ __forceinline__ void lev_small_all(const DistArgs &a, EdgeWriter &ew, int lane,
+__device__ __forceinline__ void lev_small_all(const DistArgs &a, EdgeWriter &ew, const TileSlice &T, int lane,
                                               uint64_t &pairs) {
     constexpr int R16 = LevShape<BP, W>::R16;
-    const uint32_t n_small = a.ctr->n_small;
+    const uint32_t n_small = a.ctr->n_small, batch = small_batch(n_small);
     for (;;) {
         uint32_t s0 = 0;
-        if (lane == 0) s0 = atomicAdd(&a.ctr->small_cursor, kSmallBatch);
+        if (lane == 0) s0 = atomicAdd(&a.ctr->small_cursor, batch);
         s0 = __shfl_sync(0xFFFFFFFFu, s0, 0);
         if (s0 >= n_small) break;
-        const uint32_t cnt = min(kSmallBatch, n_small - s0);
+        const uint32_t cnt = min(batch, n_small - s0);
         uint32_t myidx = 0;
         BinPair myP;
         memset(&myP, 0, sizeof(BinPair));
@@ -444,7 +431,7 @@ __device__ __forceinline__ void lev_small_all(const DistArgs &a, EdgeWriter &ew,
             const uint32_t n = P.a_n, npairs = same ? n * (n - 1) / 2 : n * P.b_n;
             const uint32_t ystart = same ? P.a_start : P.b_start;
             if (lane == 0) pairs += npairs;
-            lev_pair_block<BP, W>(a, ew, P, same, P.a_start, n, ystart, P.b_n, lane);
+            lev_pair_block<BP, W>(a, ew, T, P, same, P.a_start, n, ystart, P.b_n, lane);
             if (a.bp_cycles && lane == 0)
                 atomicAdd(&a.bp_cycles[idx], (unsigned long long)(clock64() - t0));
         }
@@ -488,7 +475,20 @@ __device__ __forceinline__ void lev_tiny_all(const DistArgs &a, EdgeWriter &ew, 
                 emask |= 1u << p;
         }
         __syncwarp();
-        emit_pair_bits(a, ew, lane, emask, 0u, 1u, same, n, P.a_start, ystart);
+        // two bins: their pairs one by one (few: most tiny groups are one bin's)
+        emit_tiny_bits(a, ew, lane, same ? emask : 0u, n, P.a_start);
+        __syncwarp();
+        uint32_t rest = same ? 0u : emask;
+        for (uint32_t it = 0; it < kTinyPairs && __any_sync(0xFFFFFFFFu, rest); ++it) {
+            uint32_t ux = 0, uy = 0;
+            if (rest) {
+                const uint32_t p = (uint32_t)__ffs(rest) - 1u;
+                ux = __ldg(&a.meta[P.a_start + p % n].w);
+                uy = __ldg(&a.meta[ystart + p / n].w);
+            }
+            ew.append(a, lane, rest != 0, min(ux, uy), max(ux, uy));
+            rest &= rest - 1;
+        }
         if (a.bp_cycles) {   // the batch's cycles, shared out by pairs
             const uint32_t tot = __reduce_add_sync(0xFFFFFFFFu, np);
             const unsigned long long dt = (unsigned long long)(clock64() - t0);
@@ -502,13 +502,15 @@ __global__ void __launch_bounds__(kWarps * 32, (W <= 2 ? 4 : 3))
 k_lev_diag(const __grid_constant__ DistArgs a) {
     using Sh = LevShape<BP, W>;
     __shared__ uint4 sy[kWarps][Sh::YB * Sh::YMax];
-    __shared__ uint4 sym[kWarps][Sh::YB];
+    __shared__ uint4 sym[kWarps][32];
     __shared__ uint4 sxm[kWarps][32 * RX];
-    __shared__ uint32_t shq[kWarps][kLevHitQ * 32];
     __shared__ uint32_t seg[kWarps][LevLookups<3, 0, W>::words];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t n_units = a.ctr->n_units, n_bp = a.ctr->n_binpairs;
-    const LevSlice S{sy[wid], sym[wid], sxm[wid], shq[wid], seg[wid]};
+    __shared__ uint32_t scp[kWarps][2 * 32 * RX + 2 * 32];   // copies and sums (TileSlice)
+    const LevSlice S{sy[wid], seg[wid],
+                     {sxm[wid], sym[wid], scp[wid], scp[wid] + 2 * 32 * RX, scp[wid] + 32 * RX,
+                      scp[wid] + 2 * 32 * RX + 32}};
     EdgeWriter ew;
     ew.init();
     uint64_t pairs = 0;
@@ -516,8 +518,9 @@ k_lev_diag(const __grid_constant__ DistArgs a) {
     while (next_unit(a, n_units, n_bp, lane, U)) {
         if (!U.P.same && U.nx <= kThinX) {   // too few x-entries for the lanes: pair by pair
             if (lane == 0) pairs += (uint64_t)U.nx * U.ny;
-            lev_pair_block<BP, W>(a, ew, U.P, false, U.P.a_start + U.xbase, U.nx,
-                                  U.P.b_start + U.ybase, U.ny, lane);
+            for (uint32_t y = 0; y < U.ny; y += 32)
+                lev_pair_block<BP, W>(a, ew, S.T, U.P, false, U.P.a_start + U.xbase, U.nx,
+                                      U.P.b_start + U.ybase + y, min(32u, U.ny - y), lane);
             log_unit(a, U, lane);
             continue;
         }
@@ -535,7 +538,7 @@ k_lev_diag(const __grid_constant__ DistArgs a) {
         }
         log_unit(a, U, lane);
     }
-    lev_small_all<BP, W>(a, ew, lane, pairs);
+    lev_small_all<BP, W>(a, ew, S.T, lane, pairs);
     lev_tiny_all<BP, W>(a, ew, lane, pairs);
     finish(a, ew, pairs, lane);
 }
