@@ -855,7 +855,7 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
 
 // exclusive block scan of one value per thread; returns prefix, *sum = total
 __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *sum) {
-    __shared__ uint32_t wsum[32];
+    __shared__ uint32_t wsum[33];   // warps before each warp, and the block's total
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nw = blockDim.x >> 5;
     uint32_t inc = warp_incl_scan(v);
@@ -865,11 +865,11 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *sum) {
         uint32_t w = lane < nw ? wsum[lane] : 0u;
         uint32_t wi = warp_incl_scan(w);
         if (lane < nw) wsum[lane] = wi - w;
-        if (lane == nw - 1) wsum[31] = wi;
+        if (lane == nw - 1) wsum[32] = wi;
     }
     __syncthreads();
     uint32_t res = inc - v + wsum[wid];
-    *sum = wsum[31];
+    *sum = wsum[32];
     __syncthreads();
     return res;
 }

@@ -76,3 +76,24 @@ def test_workload4_relative_only(gpu_ctx):
     w = synth.workload(4, scale=0.01)
     w.abs_eps = -1
     _check(gpu_ctx, w, "workload4@0.01 relative")
+
+
+def test_unique_numbering_past_992_tiles(gpu_ctx):
+    """4.1M distinct rows: the device-wide scan has more than 992 tiles of 4,096
+    values, so the last warp of the block that scans the tiles' sums takes part.
+    Every row is its own unique and its own cluster, numbered by row."""
+    n = 4_100_000
+    aa = np.frombuffer(synth.AA, np.uint8)
+    blob = np.empty((n, 6), np.uint8)
+    for k in range(6):
+        blob[:, k] = aa[(np.arange(n) // 20 ** k) % 20]
+    w = synth.from_strings([b"A"], [b"IGHV1*01"], [b"IGHJ1*01"], [b"IGHV1*"], [b"IGHJ1*"], abs_eps=0,
+                           min_pts=1, use_hamming=True)
+    w.seq_blob, w.seq_off = blob.reshape(-1), np.arange(n + 1, dtype=np.int64) * 6
+    for name, call in (("v", w.v_blob), ("j", w.j_blob)):
+        setattr(w, name + "_blob", np.tile(call, n))
+        setattr(w, name + "_off", np.arange(n + 1, dtype=np.int64) * len(call))
+    w.rep_off = np.array([0, n], np.uint32)
+    g = cluster_workload(w, gpu_ctx)
+    assert g.n_uniques == n and np.all(g.copies == 1)
+    assert np.array_equal(g.clone_id, np.arange(1, n + 1, dtype=np.uint32))
