@@ -70,7 +70,7 @@ enum BufId {
     bURow, bUCopies, bULen, bURep, bBinHist, bBinCursor, bEntUid, bEntRec, bBpCount, bBp,
     bBpSorted, bBpUnits, bClsHist, bPred, bEdges, bCnt, bUCore,
     bParent, bBMin, bRootFlag, bUidFirst, bDepth, bScanPart, bClone, bCore, bCopies, bUniques,
-    bCtr, bVTab, bJTab, bSigAnd, bUClass, bEntMeta, bCallAux, bCallTab, bCallRef, bCallTodo, bBpSmall,
+    bCtr, bVTab, bJTab, bSigAnd, bUClass, bEntMeta, bCallTab, bCallRef, bCallTodo, bBpSmall,
     bJnTab, bJnISlot, bJnStart, bJnCur, bJnBpIdx, bJnPos, bEntCopies, bNumBufs
 };
 
@@ -340,10 +340,6 @@ struct Pipeline {
     }
 };
 
-void record(Pipeline &pl, int k) {
-    if (pl.timing) launch_stamp(&pl.B.ctr->stamp[k], pl.c->stream);
-}
-
 // phase durations from the device time stamps (ms)
 void phase_times(const Counters &h, idb_stats *st) {
     for (int k = 0; k < 5; ++k)
@@ -430,7 +426,6 @@ idb_status stage_inputs_and_survey(Pipeline &pl, const idb_input *in, bool host_
     TRY(ensure(c, bCtr, sizeof(Counters)));
     B.ctr = ptr<Counters>(c, bCtr);
     CU(cudaMemsetAsync(B.ctr, 0, sizeof(Counters), s));
-    CU(cudaMemsetAsync(&B.ctr->lmin, 0xFF, sizeof(uint32_t), s));   // min starts at max
     // staging buffers of host columns (device columns are read in place)
     auto place = [&](const char *src, const int64_t *off, BufId bid, BufId oid,
                      const uint8_t **dst, const int64_t **doff) -> idb_status {
@@ -492,7 +487,7 @@ idb_status stage_inputs_and_survey(Pipeline &pl, const idb_input *in, bool host_
     P.JW = P.Gj > 64 ? (P.Gj + 63) / 64 : 1;
     if (P.Gv == 0) P.Gv = 1;   // a V column with an empty reference list: all bitsets 0
     if (P.Gj == 0) P.Gj = 1;
-    record(pl, 0);
+    B.timing = pl.timing;
     launch_survey(P, B, s);
     TRY(check_launch());
     CU(cudaMemcpyAsync(c->h_ctr, B.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s));
@@ -523,7 +518,7 @@ idb_status derive_plan(Pipeline &pl, const idb_params *prm) {
     P.schedule = prm->schedule;
     P.streamed = prm->edge_memory_mb < 0;
     P.edge_budget = prm->edge_memory_mb > 0 ? (uint64_t)prm->edge_memory_mb << 20 : 0;
-    P.Lmin = P.N ? h.lmin : 0;
+    P.Lmin = P.N ? ~h.lmin_inv : 0;
     P.Lmax = P.N ? h.lmax : 0;
     if (P.Lmin > P.Lmax) P.Lmin = P.Lmax;
     if (P.Lmax > 65535) return fail(IDB_ERR_UNSUPPORTED, "sequences longer than 65535 bytes");
@@ -636,14 +631,13 @@ idb_status alloc_call_scratch(idb_context *c, Buffers &B, uint64_t N) {
     TRY(ensure(c, bCallTab, 2 * 8 * slots));
     TRY(ensure(c, bCallRef, 2 * 4 * N));
     TRY(ensure(c, bCallTodo, 2 * 4 * N));
-    TRY(ensure(c, bCallAux, 2 * 4 * kMaxRowChunks));
     for (int k = 0; k < 2; ++k) {
         CallScratch &cs = B.call[k];
         cs.tab = ptr<unsigned long long>(c, bCallTab) + k * slots;
         cs.mask = (uint32_t)(slots - 1);
         cs.ref = ptr<uint32_t>(c, bCallRef) + k * N;
         cs.todo = ptr<uint32_t>(c, bCallTodo) + k * N;
-        cs.ntodo = ptr<uint32_t>(c, bCallAux) + k * kMaxRowChunks;
+        cs.ntodo = B.ctr->call_todo + k * kMaxRowChunks;
     }
     return IDB_OK;
 }
@@ -713,6 +707,7 @@ idb_status alloc_fixed(Pipeline &pl) {
     }
     B.scan_part_cap = scan_part_needed(std::max<uint64_t>(scan_n, 1u << 20));
     TRY(ensure(c, bScanPart, 4 * (size_t)B.scan_part_cap));
+    CU(cudaMemsetAsync(c->buf[bScanPart].p, 0, sizeof(uint32_t), c->stream));   // the scans' counter
     B.vbits = ptr<uint64_t>(c, bVBits); B.jbits = ptr<uint64_t>(c, bJBits);
     B.slot = ptr<uint32_t>(c, bSlot); B.rep_row = ptr<uint32_t>(c, bRepRow);
     B.flag = ptr<uint32_t>(c, bFlag); B.uid_of_row = ptr<uint32_t>(c, bUidOfRow);
@@ -759,6 +754,7 @@ idb_status alloc_binpairs(Pipeline &pl, uint64_t n_bp) {
     if (need > pl.B.scan_part_cap) {
         pl.B.scan_part_cap = (uint32_t)need;
         TRY(ensure(c, bScanPart, 4 * (size_t)need));
+        CU(cudaMemsetAsync(c->buf[bScanPart].p, 0, sizeof(uint32_t), c->stream));
         pl.B.scan_part = ptr<uint32_t>(c, bScanPart);
     }
     pl.B.bp = ptr<BinPair>(c, bBp);
@@ -901,7 +897,6 @@ idb_status run_phases(Pipeline &pl, bool eager, bool stop_after_schedule = false
         CU(cudaEventRecordWithFlags(c->ev_out[0], s, cudaEventRecordExternal));
     }
     TRY(check_launch());
-    record(pl, 1);
     launch_buckets(P, B, s);
     if (eager) TRY(choose_candidates(pl));
     launch_fill(P, B, s);
@@ -918,7 +913,6 @@ idb_status run_phases(Pipeline &pl, bool eager, bool stop_after_schedule = false
     }
     launch_schedule(P, B, s);
     TRY(check_launch());
-    record(pl, 2);
     if (stop_after_schedule) return IDB_OK;
     // The neighbour pairs go to an edge list for the graph phase, unless they
     // would take more than the edge memory allowed (or than the device has):
@@ -958,16 +952,12 @@ idb_status run_phases(Pipeline &pl, bool eager, bool stop_after_schedule = false
     if (P.streamed) {
         launch_streamed_sweeps(P, B, s);
         TRY(check_launch());
-        record(pl, 3);
         launch_streamed_labels(P, B, pl.trees, s);
     } else {
-        record(pl, 3);
         launch_graph(P, B, pl.trees, s, pl.early_out ? c->ev_out[1] : nullptr);
     }
-    record(pl, 4);
     launch_outputs(P, B, s, pl.early_out ? kOutClone : kOutAll);
     TRY(check_launch());
-    record(pl, 5);
     return IDB_OK;
 }
 
@@ -1116,8 +1106,7 @@ idb_status host_plan_capture(Pipeline &pl) {
     pl.early_out = !pl.P.streamed;
     CU(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(pl.B.ctr, 0, sizeof(Counters), s);
-    cudaMemsetAsync(&pl.B.ctr->lmin, 0xFF, sizeof(uint32_t), s);
-    record(pl, 0);
+    pl.B.timing = pl.timing;
     cudaStreamWaitEvent(s, c->ev_seq, cudaEventWaitExternal);
     launch_survey(pl.P, pl.B, s);
     idb_status st = run_phases(pl, false);
@@ -1492,9 +1481,8 @@ idb_status idb_batch_plan(idb_context *c, const idb_input *in, const idb_params 
     CU(cudaStreamSynchronize(s));
     CU(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(pl.B.ctr, 0, sizeof(Counters), s);
-    cudaMemsetAsync(&pl.B.ctr->lmin, 0xFF, sizeof(uint32_t), s);
     pl.timing = true;   // time-stamp kernels between the phases
-    record(pl, 0);
+    pl.B.timing = pl.timing;
     launch_survey(pl.P, pl.B, s);
     idb_status st = run_phases(pl, false);
     cudaGraph_t g = nullptr;
@@ -1593,6 +1581,9 @@ idb_status idb_diag_gene_bits(idb_context *c, const char *calls, const int64_t *
     pl.c = c;
     Plan &P = pl.P;
     Buffers &B = pl.B;
+    TRY(ensure(c, bCtr, sizeof(Counters)));
+    B.ctr = ptr<Counters>(c, bCtr);
+    CU(cudaMemsetAsync(B.ctr, 0, sizeof(Counters), c->stream));
     P.N = n_rows;
     P.no_v = false;
     P.Gv = n_genes;
@@ -1861,7 +1852,6 @@ idb_status idb_autotune(idb_context *c, const idb_input *in, const idb_params *p
     // one shape and schedule order: bin pairs, the order, then the distance
     // kernel three times (best of the three)
     auto time_shape = [&](Plan Q, float *ms_out) -> idb_status {
-        CU(cudaMemsetAsync(&B.ctr->n_binpairs, 0, 4, s));
         launch_binpairs(Q, B, s);
         TRY(read_counters(pl));
         pl.P = Q;

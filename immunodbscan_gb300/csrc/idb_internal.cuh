@@ -84,6 +84,18 @@ struct GeneMatcher {
 };
 
 #ifdef __CUDACC__
+// Phase time stamps: the device's global nanosecond timer, written by the first
+// thread of a phase's first kernel (a kernel of its own per stamp cost six
+// launches a call).
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+__device__ __forceinline__ void stamp_begin(unsigned long long *dst) {
+    if (dst && blockIdx.x == 0 && threadIdx.x == 0) *dst = global_ns();
+}
+
 // Sequential reader of a byte string in global memory, 4 bytes per step.  It
 // loads only the aligned 4-byte words that hold bytes of the string (so no load
 // leaves the string's pages) and joins neighbours with a funnel shift; bytes
@@ -138,7 +150,7 @@ __device__ __forceinline__ void load_chunk32(const uint8_t *p, uint32_t L, uint3
 
 // Device-resident counters of one clustering call (one struct, zeroed first).
 struct Counters {
-    uint32_t lmax, lmin;
+    uint32_t lmax, lmin_inv;     // longest sequence, and ~(shortest)
     uint32_t used[8];            // 256-bit byte-presence map of the sequences
     uint32_t n_uniques;
     uint32_t n_entries;
@@ -162,7 +174,7 @@ struct Counters {
     uint32_t n_core_edges;       // neighbour pairs with both ends core
     uint32_t n_jslots;           // segment join: table slots in use (the probed prefix)
     uint32_t chunk_uniques[kMaxRowChunks];   // uniques of each row chunk (numbered by chunk)
-    uint32_t n_groups;           // segment join: bin pairs of the groups
+    uint32_t call_todo[2 * kMaxRowChunks];   // rows that compute their own bitset, per column and chunk
     unsigned long long join_pairs;    // edit-distance join: candidate pairs of its groups
     unsigned long long bucket_pairs;  // pairs of the buckets (an upper bound), when compared with it
     uint32_t n_tiny;             // tiny bin pairs (one lane each), listed from the small list's end
@@ -177,7 +189,6 @@ struct Counters {
 struct BinPair {
     uint32_t a_start, a_n;      // x entries [a_start, a_start+a_n)
     uint32_t b_start, b_n;      // y entries
-    uint32_t unit_base;         // first work unit (exclusive scan, schedule order)
     uint32_t ncx;               // x chunks
     uint16_t la, lb;            // lengths of the two bins
     uint16_t v, j;              // the bins' V gene and J gene
@@ -186,7 +197,7 @@ struct BinPair {
     uint8_t cls;                // schedule class
     uint32_t cost_lo;           // predicted cost (pairs or learned), low 32 bits
 };
-static_assert(sizeof(BinPair) == 40, "BinPair layout");
+static_assert(sizeof(BinPair) == 36, "BinPair layout");
 
 // Host-side plan of one call (everything the kernels need as constants).
 struct Plan {
@@ -312,6 +323,8 @@ struct Buffers {
     uint32_t *copies = nullptr;
     uint32_t *uniques = nullptr;
     Counters *ctr = nullptr;
+    bool timing = false;                            // the phases write their time stamps
+    unsigned long long *stamp(int k) const { return timing ? &ctr->stamp[k] : nullptr; }
     // per bin-pair timing log (optional)
     unsigned long long *bp_cycles = nullptr;
     uint32_t *bp_hits = nullptr;
@@ -320,7 +333,6 @@ struct Buffers {
 // ---- launchers (each enqueues on `s`, never synchronises) ----
 void launch_survey(const Plan &P, const Buffers &B, cudaStream_t s);
 void launch_check_plan(const Plan &P, const Buffers &B, cudaStream_t s);
-void launch_stamp(unsigned long long *dst, cudaStream_t s);
 // The front end runs by row chunks [chunk_row[k], chunk_row[k+1]): the two
 // init launchers once, then per chunk launch_gene_bits (V, then J) and
 // launch_dedupe_rows, then launch_dedupe_final over all rows.

@@ -64,7 +64,9 @@ __device__ __forceinline__ bool same_group(const uint64_t *vbits, const uint64_t
 __global__ void k_group_insert(BinGeom g, Counters *ctr, const uint32_t *__restrict__ urow,
                                const uint32_t *__restrict__ ulen, const uint32_t *__restrict__ urep,
                                const uint64_t *__restrict__ vbits, const uint64_t *__restrict__ jbits,
-                               uint32_t *table, uint32_t *tcount, uint32_t *uslot, uint64_t mask) {
+                               uint32_t *table, uint32_t *tcount, uint32_t *uslot, uint64_t mask,
+                               unsigned long long *stamp) {
+    stamp_begin(stamp);
     const uint32_t nu = ctr->n_uniques;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < nu; u += stride) {
@@ -291,7 +293,6 @@ __device__ __forceinline__ uint32_t visit_pairs(uint32_t sb, const PairGeom &pg,
                 const uint32_t rest = b / pg.NL;
                 BinPair P;
                 P.a_start = a0; P.a_n = nA; P.b_start = b0; P.b_n = nB;
-                P.unit_base = 0;
                 P.ncx = (nA + pg.TX - 1) / pg.TX;
                 P.la = (uint16_t)(pg.Lmin + li); P.lb = (uint16_t)(pg.Lmin + li + g);
                 P.v = (uint16_t)((rest / pg.Gj) % pg.Gv); P.j = (uint16_t)(rest % pg.Gj);
@@ -358,8 +359,10 @@ __device__ __forceinline__ uint32_t sched_bin(const BinPair &P, uint32_t cls, in
     return (63 - cls) * kSchedVariants + v;
 }
 
-__global__ void k_cls_hist(const Counters *__restrict__ ctr, const BinPair *__restrict__ bp,
+__global__ void k_cls_hist(Counters *ctr, const BinPair *__restrict__ bp,
                            const float *__restrict__ pred, uint32_t *__restrict__ hist, int by_loop) {
+    if (blockIdx.x == 0 && threadIdx.x == 0)   // the lists k_cls_scatter fills
+        ctr->n_small = ctr->small_cursor = ctr->n_tiny = ctr->tiny_cursor = 0;
     __shared__ uint32_t h[kSchedBins];
     for (uint32_t k = threadIdx.x; k < kSchedBins; k += blockDim.x) h[k] = 0;
     __syncthreads();
@@ -434,15 +437,6 @@ __global__ void k_cls_scatter(const Counters *__restrict__ ctr, const BinPair *_
     }
 }
 
-__global__ void k_set_unit_base(const Counters *__restrict__ ctr, BinPair *__restrict__ bp,
-                                const uint32_t *__restrict__ base) {
-    const uint32_t n = ctr->n_binpairs;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-        bp[i].unit_base = base[i];
-}
-
-
 // ---------------------------------------------------------------------------
 // Segment join (Hamming, eps(L,L) <= kJoinMaxEps for every length).  Split a
 // sequence of length L into S = eps+1 segments [k*L/S, (k+1)*L/S): two
@@ -483,9 +477,14 @@ __device__ __forceinline__ unsigned long long seg_key(const uint32_t (&wd)[5][4]
 // bound) when the inserts run by row chunk, before the count is known.
 __global__ void k_join_clear(Counters *ctr, uint32_t smax, uint64_t cap_mask,
                              unsigned long long *__restrict__ key, uint32_t *__restrict__ cnt,
-                             uint32_t rows) {
+                             uint32_t rows, unsigned long long *stamp) {
+    stamp_begin(stamp);
     const uint32_t n = join_mask(rows ? rows : ctr->n_uniques, smax, cap_mask) + 1u;
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctr->n_jslots = n;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        ctr->n_jslots = n;
+        ctr->n_entries = 0;
+        ctr->n_binpairs = 0;
+    }
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         key[i] = ~0ull;
@@ -562,7 +561,8 @@ k_join_insert(BinGeom g, Counters *ctr, const uint32_t *__restrict__ urow,
 // rows: 1.472 against 1.456 ms a call).  Four slots per thread (16-byte loads and stores).
 __global__ void __launch_bounds__(256)
 k_join_groups(Counters *ctr, const uint32_t *__restrict__ tcnt, uint32_t *__restrict__ start,
-              uint32_t *__restrict__ bpidx) {
+              uint32_t *__restrict__ bpidx, unsigned long long *stamp) {
+    stamp_begin(stamp);
     __shared__ uint2 s_w[8];
     __shared__ uint2 s_base;
     const uint32_t ns = ctr->n_jslots;   // a power of two >= 1024: whole blocks of slots
@@ -593,7 +593,7 @@ k_join_groups(Counters *ctr, const uint32_t *__restrict__ tcnt, uint32_t *__rest
                 tg += x.x;
                 te += x.y;
             }
-            if (tg) s_base = make_uint2(atomicAdd(&ctr->n_groups, tg), atomicAdd(&ctr->n_entries, te));
+            if (tg) s_base = make_uint2(atomicAdd(&ctr->n_binpairs, tg), atomicAdd(&ctr->n_entries, te));
         }
         __syncthreads();
         uint32_t idx = s_base.x + s_w[wid].x + gi - groups, pos = s_base.y + s_w[wid].y + ei - entries;
@@ -660,10 +660,6 @@ k_join_fill(BinGeom g, const Counters *__restrict__ ctr, const uint32_t *__restr
     }
 }
 
-__global__ void k_join_nbp(Counters *ctr) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) ctr->n_binpairs = ctr->n_groups;
-}
-
 // One bin pair (a group against itself) per key held by two or more uniques:
 // a sequential pass over the probed prefix of the table.
 __global__ void k_join_bp_fill(BinGeom g, const Counters *__restrict__ ctr,
@@ -688,7 +684,6 @@ __global__ void k_join_bp_fill(BinGeom g, const Counters *__restrict__ ctr,
             const uint32_t li = L - g.Lmin;
             BinPair P;
             P.a_start = s0; P.a_n = c; P.b_start = s0; P.b_n = c;
-            P.unit_base = 0;
             P.ncx = (c + TX - 1) / TX;
             P.la = (uint16_t)L; P.lb = (uint16_t)L;
             P.v = (uint16_t)((key >> 30) & 3u);                   // segment of the group
@@ -705,9 +700,9 @@ __global__ void k_join_bp_fill(BinGeom g, const Counters *__restrict__ ctr,
 }  // namespace
 
 void launch_join_init(const Plan &P, const Buffers &B, cudaStream_t s) {
-    cudaMemsetAsync(&B.ctr->n_groups, 0, sizeof(uint32_t), s);
     k_join_clear<<<grid_wave(k_join_clear, B.jn_mask + 1, kThreads), kThreads, 0, s>>>(
-        B.ctr, P.join_smax, B.jn_mask, B.jn_key, B.jn_cnt, P.front_join ? P.N : 0u);
+        B.ctr, P.join_smax, B.jn_mask, B.jn_key, B.jn_cnt, P.front_join ? P.N : 0u,
+        P.front_join ? nullptr : B.stamp(1));
 }
 
 void launch_join_insert(const Plan &P, const Buffers &B, int chunk, cudaStream_t s) {
@@ -731,9 +726,8 @@ void launch_buckets(const Plan &P, const Buffers &B, cudaStream_t s) {
             launch_join_init(P, B, s);
             launch_join_insert(P, B, -1, s);
         }
-        cudaMemsetAsync(&B.ctr->n_entries, 0, sizeof(uint32_t), s);
         k_join_groups<<<grid_wave(k_join_groups, slots / 4, kThreads), kThreads, 0, s>>>(
-            B.ctr, B.jn_cnt, B.jn_start, B.jn_bpidx);
+            B.ctr, B.jn_cnt, B.jn_start, B.jn_bpidx, P.front_join ? B.stamp(1) : nullptr);
         return;
     }
     const uint32_t nb = (uint32_t)P.nbins;
@@ -742,7 +736,7 @@ void launch_buckets(const Plan &P, const Buffers &B, cudaStream_t s) {
     cudaMemsetAsync(B.tcount, 0, sizeof(uint32_t) * (B.table_mask + 1), s);
     k_group_insert<<<grid_wave(k_group_insert, P.N, kThreads), kThreads, 0, s>>>(g, B.ctr, B.urow, B.ulen, B.urep, B.vbits,
                                                        B.jbits, B.table, B.tcount, B.slot,
-                                                       B.table_mask);
+                                                       B.table_mask, B.stamp(1));
     k_group_class<<<grid_wave(k_group_class, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.slot, B.tcount, P.K, P.big_group,
                                                       B.uclass);
     cudaMemsetAsync(B.bin_hist, 0, sizeof(uint32_t) * (P.nbins + 1), s);
@@ -804,10 +798,7 @@ void launch_fill(const Plan &P, const Buffers &B, cudaStream_t s) {
 }
 
 void launch_binpairs(const Plan &P, const Buffers &B, cudaStream_t s) {
-    if (P.join) {
-        k_join_nbp<<<1, 32, 0, s>>>(B.ctr);
-        return;
-    }
+    if (P.join) return;   // counted with the groups
     PairGeom pg{P.NL, P.Lmin, P.Gv, P.Gj, P.K, P.dLmax, P.hamming, P.TX, P.TY, P.TY / P.TX};
     const uint32_t nb = (uint32_t)P.nbins;
     k_binpairs_count<<<grid_for(nb), kThreads, 0, s>>>(nb, pg, B.eps_tab, B.bin_hist, B.sig_and,
@@ -850,15 +841,12 @@ void launch_schedule(const Plan &P, const Buffers &B, cudaStream_t s) {
     cudaMemsetAsync(B.cls_hist, 0, sizeof(uint32_t) * 2 * kSchedBins, s);
     k_cls_hist<<<grid_for(P.cap_binpairs), kThreads, 0, s>>>(B.ctr, B.bp, pred, B.cls_hist, by_loop);
     scan_u32(B.cls_hist, B.cls_hist, kSchedBins, nullptr, nullptr, B.scan_part, B.scan_part_cap, s);
-    cudaMemsetAsync(&B.ctr->n_small, 0, 2 * sizeof(uint32_t), s);   // n_small, small_cursor
-    cudaMemsetAsync(&B.ctr->n_tiny, 0, 2 * sizeof(uint32_t), s);    // n_tiny, tiny_cursor
     k_cls_scatter<<<grid_for(P.cap_binpairs), kThreads, 0, s>>>(
         B.ctr, B.bp, pred, B.cls_hist, B.cls_hist + kSchedBins, B.bp_sorted, B.bp_units, P.TX, P.TY, q,
         P.planes() ? (P.hamming ? 1 : 2) : 0, B.bp_small, &B.ctr->n_small, &B.ctr->n_tiny,
         (uint32_t)P.cap_binpairs + 1u, by_loop);
     scan_u32(B.bp_units, B.bp_units, (uint32_t)P.cap_binpairs, &B.ctr->n_binpairs,
              &B.ctr->n_units, B.scan_part, B.scan_part_cap, s);
-    k_set_unit_base<<<grid_for(P.cap_binpairs), kThreads, 0, s>>>(B.ctr, B.bp_sorted, B.bp_units);
 }
 
 }  // namespace idb

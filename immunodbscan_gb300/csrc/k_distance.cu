@@ -398,10 +398,13 @@ void launch_distance(const Plan &P, const Buffers &B, int grid, cudaStream_t s, 
         a.edges = nullptr;
         a.cap_edges = ~0ull;
     }
-    if (sink != kSinkGrow) launch_graph_init(P, B, s);   // a repeated sweep counts anew
-    cudaMemsetAsync(&B.ctr->unit_cursor, 0, sizeof(uint32_t), s);
-    cudaMemsetAsync(&B.ctr->small_cursor, 0, sizeof(uint32_t), s);
-    cudaMemsetAsync(&B.ctr->tiny_cursor, 0, sizeof(uint32_t), s);
+    if (sink != kSinkGrow) {   // the work queues too; a repeated sweep counts anew
+        launch_graph_init(P, B, s);
+    } else {
+        cudaMemsetAsync(&B.ctr->unit_cursor, 0, sizeof(uint32_t), s);
+        cudaMemsetAsync(&B.ctr->small_cursor, 0, sizeof(uint32_t), s);
+        cudaMemsetAsync(&B.ctr->tiny_cursor, 0, sizeof(uint32_t), s);
+    }
     if (!P.fast) {
         if (P.hamming) run(k_generic<true>, a, 0, grid, s);
         else run(k_generic<false>, a, 0, grid, s);

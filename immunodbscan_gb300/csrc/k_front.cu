@@ -33,7 +33,8 @@ __device__ __forceinline__ uint32_t rep_of_row(const uint32_t *rep_off, uint32_t
 // Survey: sequence length range and the set of byte values present.
 // ---------------------------------------------------------------------------
 __global__ void k_survey(const uint8_t *__restrict__ seq, const int64_t *__restrict__ off,
-                         uint32_t N, Counters *ctr) {
+                         uint32_t N, Counters *ctr, unsigned long long *stamp) {
+    stamp_begin(stamp);
     __shared__ uint32_t used[8];
     __shared__ uint32_t smax, smin;
     if (threadIdx.x < 8) used[threadIdx.x] = 0;
@@ -110,7 +111,7 @@ __global__ void k_survey(const uint8_t *__restrict__ seq, const int64_t *__restr
     if (threadIdx.x < 8 && used[threadIdx.x]) atomicOr(&ctr->used[threadIdx.x], used[threadIdx.x]);
     if (threadIdx.x == 0) {
         atomicMax(&ctr->lmax, smax);
-        atomicMin(&ctr->lmin, smin);
+        atomicMax(&ctr->lmin_inv, ~smin);
     }
 }
 
@@ -841,6 +842,14 @@ __global__ void k_uniques_finish(uint32_t nchunks, Counters *ctr, const uint32_t
 // ---------------------------------------------------------------------------
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;
+constexpr uint32_t kScanOneTile = 4096;
+// One block scans up to this many values: 4 rounds of its 1,024 threads take
+// about as long as the second launch of the other form (10k values: 5.5 us; three
+// launches took 10 us).
+constexpr uint32_t kScanSmall = 16384;
+// Tiles whose sums the last block of the reduction scans; more take a launch of
+// 1,024 threads.
+constexpr uint32_t kScanFuse = 2048;
 constexpr uint32_t kScanTile = kScanThreads * kScanItems;
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
@@ -874,9 +883,35 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *sum) {
     return res;
 }
 
+// Up to kScanSmall values: one block, kScanOneTile of them at a time.
+__global__ void __launch_bounds__(1024)
+k_scan_one(const uint32_t *in, uint32_t *out, uint32_t n_host, const uint32_t *n_dev, uint32_t *total_out) {
+    const uint32_t n = n_dev ? min(*n_dev, n_host) : n_host;
+    uint32_t carry = 0;
+    for (uint32_t base = 0; base < n; base += kScanOneTile) {
+        const uint32_t i0 = base + 4 * threadIdx.x;
+        uint32_t v[4], s = 0, total;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            v[k] = i0 + k < n ? in[i0 + k] : 0u;
+            s += v[k];
+        }
+        uint32_t pre = carry + block_excl_scan(s, &total);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (i0 + k < n) out[i0 + k] = pre;
+            pre += v[k];
+        }
+        carry += total;
+    }
+    if (threadIdx.x == 0 && total_out) *total_out = carry;
+}
+
+// Sums of the tiles; with `fuse` the last block to finish also scans them (done:
+// a counter that is 0 between scans).
 __global__ void __launch_bounds__(kScanThreads)
 k_scan_reduce(const uint32_t *__restrict__ in, uint32_t n_host, const uint32_t *n_dev,
-              uint32_t *__restrict__ part) {
+              uint32_t *part, uint32_t *done, int fuse, uint32_t *total_out) {
     const uint32_t n = n_dev ? min(*n_dev, n_host) : n_host;
     const uint64_t base = (uint64_t)blockIdx.x * kScanTile;
     uint32_t s = 0;
@@ -887,6 +922,27 @@ k_scan_reduce(const uint32_t *__restrict__ in, uint32_t n_host, const uint32_t *
     uint32_t total;
     block_excl_scan(s, &total);
     if (threadIdx.x == 0) part[blockIdx.x] = total;
+    if (!fuse) return;
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    uint32_t carry = 0;
+    for (uint32_t b0 = 0; b0 < gridDim.x; b0 += kScanThreads) {
+        const uint32_t b = b0 + threadIdx.x;
+        const uint32_t v = b < gridDim.x ? __ldcg(part + b) : 0u;
+        const uint32_t pre = carry + block_excl_scan(v, &total);
+        if (b < gridDim.x) part[b] = pre;
+        carry += total;
+    }
+    if (threadIdx.x == 0) {
+        if (total_out) *total_out = carry;
+        *done = 0u;
+    }
 }
 
 __global__ void __launch_bounds__(1024)
@@ -953,14 +1009,6 @@ k_scan_down(const uint32_t *in, uint32_t *out, uint32_t n_host, const uint32_t *
     }
 }
 
-// Phase time stamps: the device's global nanosecond timer, written by a
-// one-thread kernel between phases (works inside a captured graph).
-__global__ void k_stamp(unsigned long long *dst) {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    *dst = t;
-}
-
 // A replayed plan is only valid while lengths and byte values stay inside the
 // ones it was built for.
 struct PlanShape {
@@ -971,7 +1019,7 @@ struct PlanShape {
 __global__ void k_check_plan(PlanShape ps, Counters *ctr) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     uint32_t err = 0;
-    if (ctr->lmax > ps.lmax || ctr->lmin < ps.lmin) err |= kErrLength;
+    if (ctr->lmax > ps.lmax || ~ctr->lmin_inv < ps.lmin) err |= kErrLength;
     for (int k = 0; k < 8; ++k)
         if (ctr->used[k] & ~ps.used[k]) err |= kErrAlphabet;
     if (err) atomicOr(&ctr->error, err);
@@ -988,7 +1036,8 @@ inline int grid_for(uint64_t n, int threads = kThreads) {
 }  // namespace
 
 // ---------------------------------------------------------------------------
-uint32_t scan_part_needed(uint64_t n) { return (uint32_t)((n + kScanTile - 1) / kScanTile + 1); }
+// part[0] is the reduction's counter (0 between scans), the tiles' sums follow.
+uint32_t scan_part_needed(uint64_t n) { return (uint32_t)((n + kScanTile - 1) / kScanTile + 2); }
 
 void scan_u32(const uint32_t *in, uint32_t *out, uint32_t n, const uint32_t *n_dev,
               uint32_t *total, uint32_t *part, uint32_t part_cap, cudaStream_t s) {
@@ -998,13 +1047,16 @@ void scan_u32(const uint32_t *in, uint32_t *out, uint32_t n, const uint32_t *n_d
         return;
     }
     (void)part_cap;
+    if (n <= kScanSmall) {
+        k_scan_one<<<1, 1024, 0, s>>>(in, out, n, n_dev, total);
+        return;
+    }
     const int vec = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
-    k_scan_reduce<<<nb, kScanThreads, 0, s>>>(in, n, n_dev, part);
-    k_scan_parts<<<1, 1024, 0, s>>>(part, nb, total);
-    k_scan_down<<<nb, kScanThreads, 0, s>>>(in, out, n, n_dev, part, vec);
+    const bool fuse = nb <= kScanFuse;
+    k_scan_reduce<<<nb, kScanThreads, 0, s>>>(in, n, n_dev, part + 1, part, fuse, total);
+    if (!fuse) k_scan_parts<<<1, 1024, 0, s>>>(part + 1, nb, total);
+    k_scan_down<<<nb, kScanThreads, 0, s>>>(in, out, n, n_dev, part + 1, vec);
 }
-
-void launch_stamp(unsigned long long *dst, cudaStream_t s) { k_stamp<<<1, 1, 0, s>>>(dst); }
 
 void launch_check_plan(const Plan &P, const Buffers &B, cudaStream_t s) {
     PlanShape ps;
@@ -1017,7 +1069,7 @@ void launch_check_plan(const Plan &P, const Buffers &B, cudaStream_t s) {
 }
 
 void launch_survey(const Plan &P, const Buffers &B, cudaStream_t s) {
-    k_survey<<<grid_wave(k_survey, P.N, kThreads), kThreads, 0, s>>>(B.seq, B.seq_off, P.N, B.ctr);
+    k_survey<<<grid_wave(k_survey, P.N, kThreads), kThreads, 0, s>>>(B.seq, B.seq_off, P.N, B.ctr, B.stamp(0));
 }
 
 void launch_const_strings(uint8_t *blob, int64_t *off, uint32_t N, cudaStream_t s) {
@@ -1030,9 +1082,11 @@ void launch_call_init(const Plan &P, const Buffers &B, bool v_column, cudaStream
         k_gene_bits_const<<<grid_for(P.N), kThreads, 0, s>>>(P.N, bits);
         return;
     }
+    // both columns' tables are neighbours: one clear for the two
+    const bool both = !P.no_v && !P.no_j;
+    if (both && !v_column) return;
     const CallScratch &cs = B.call[v_column ? 0 : 1];
-    cudaMemsetAsync(cs.tab, 0xFF, sizeof(unsigned long long) * ((size_t)cs.mask + 1), s);
-    cudaMemsetAsync(cs.ntodo, 0, sizeof(uint32_t) * kMaxRowChunks, s);
+    cudaMemsetAsync(cs.tab, 0xFF, sizeof(unsigned long long) * ((size_t)cs.mask + 1) * (both ? 2 : 1), s);
 }
 
 void launch_gene_bits(const Plan &P, const Buffers &B, bool v_column, uint32_t chunk, cudaStream_t s) {

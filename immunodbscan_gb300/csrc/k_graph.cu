@@ -42,9 +42,12 @@ __device__ __forceinline__ uint32_t edge_slots(const Counters *ctr, uint64_t cap
     return (uint32_t)(r < cap ? r : cap);
 }
 
-__global__ void k_graph_init(const Counters *__restrict__ ctr, const uint32_t *__restrict__ ucopies,
+__global__ void k_graph_init(Counters *ctr, const uint32_t *__restrict__ ucopies,
                              uint32_t *__restrict__ cnt, uint32_t *__restrict__ parent,
-                             uint32_t *__restrict__ bmin) {
+                             uint32_t *__restrict__ bmin, unsigned long long *stamp) {
+    stamp_begin(stamp);
+    if (blockIdx.x == 0 && threadIdx.x == 0)   // the distance kernel's work queues
+        ctr->unit_cursor = ctr->small_cursor = ctr->tiny_cursor = 0;
     const uint32_t nu = ctr->n_uniques;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < nu; u += stride) {
@@ -58,7 +61,9 @@ __global__ void k_graph_init(const Counters *__restrict__ ctr, const uint32_t *_
 // root, or under the smaller neighbour the distance kernel left in its parent
 // when that is core too (such an edge is a union); a non-core unique is marked.
 __global__ void k_core(const Counters *__restrict__ ctr0, Counters *ctr, const uint32_t *__restrict__ cnt,
-                       uint32_t min_pts, uint32_t *__restrict__ ucore, uint32_t *parent) {
+                       uint32_t min_pts, uint32_t *__restrict__ ucore, uint32_t *parent,
+                       unsigned long long *stamp) {
+    stamp_begin(stamp);
     const uint32_t nu = ctr0->n_uniques;
     const uint32_t stride = gridDim.x * blockDim.x;
     uint32_t local = 0;
@@ -208,7 +213,9 @@ __global__ void k_depth(uint32_t N, const uint32_t *__restrict__ row2uid, const 
 // node pointing at an inner ancestor.  Each thread writes only its own node,
 // and the roots no longer change, so every write is final.
 __global__ void k_compress(const Counters *__restrict__ ctr, const uint32_t *__restrict__ ucore,
-                           uint32_t *parent, uint32_t *__restrict__ rootflag) {
+                           uint32_t *parent, uint32_t *__restrict__ rootflag, uint32_t N,
+                           unsigned long long *stamp) {
+    stamp_begin(stamp);
     const uint32_t nu = ctr->n_uniques;
     const uint32_t stride = gridDim.x * blockDim.x;
     volatile uint32_t *vp = parent;
@@ -224,6 +231,8 @@ __global__ void k_compress(const Counters *__restrict__ ctr, const uint32_t *__r
         }
         rootflag[u] = ucore[u] && r == u;
     }
+    // the scan runs over [0, N]: nothing past the uniques
+    for (uint64_t u = (uint64_t)nu + blockIdx.x * blockDim.x + threadIdx.x; u <= N; u += stride) rootflag[u] = 0u;
 }
 
 __global__ void k_labels(const Counters *__restrict__ ctr, const uint32_t *__restrict__ ucore,
@@ -249,7 +258,9 @@ __global__ void k_rows_out(uint32_t N, uint32_t min_pts, const uint32_t *__restr
                            const uint32_t *__restrict__ urow, const uint32_t *__restrict__ ucopies,
                            const uint32_t *__restrict__ ucore, const uint32_t *__restrict__ ulabel,
                            uint32_t *__restrict__ clone_id, int32_t *__restrict__ core,
-                           uint32_t *__restrict__ copies, Counters *ctr, uint32_t what) {
+                           uint32_t *__restrict__ copies, Counters *ctr, uint32_t what,
+                           unsigned long long *stamp) {
+    if (what & kOutClone) stamp_begin(stamp);
     const uint32_t stride = gridDim.x * blockDim.x;
     uint32_t noise = 0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += stride) {
@@ -267,6 +278,10 @@ __global__ void k_rows_out(uint32_t N, uint32_t min_pts, const uint32_t *__restr
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) noise += __shfl_xor_sync(0xFFFFFFFFu, noise, d);
     if ((threadIdx.x & 31) == 0 && noise) atomicAdd(&ctr->n_noise_rows, noise);
+    if (stamp && (what & kOutClone)) {   // the call's end: the last block's
+        __syncthreads();
+        if (threadIdx.x == 0) atomicMax(stamp + 1, global_ns());
+    }
 }
 
 __global__ void k_uniques_out(const Counters *__restrict__ ctr, const uint32_t *__restrict__ urow,
@@ -279,13 +294,13 @@ __global__ void k_uniques_out(const Counters *__restrict__ ctr, const uint32_t *
 }  // namespace
 
 void launch_graph_init(const Plan &P, const Buffers &B, cudaStream_t s) {
-    k_graph_init<<<grid_wave(k_graph_init, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ucopies, B.cnt, B.parent, B.bmin);
+    k_graph_init<<<grid_wave(k_graph_init, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ucopies, B.cnt, B.parent, B.bmin, B.stamp(2));
 }
 
 void launch_graph(const Plan &P, const Buffers &B, bool trees, cudaStream_t s, cudaEvent_t core_out) {
     const uint64_t ecap = P.cap_edges;
     const int gu = grid_for(P.N);
-    k_core<<<grid_wave(k_core, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ctr, B.cnt, P.min_pts, B.ucore, B.parent);
+    k_core<<<grid_wave(k_core, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ctr, B.cnt, P.min_pts, B.ucore, B.parent, B.stamp(3));
     if (core_out) {   // the row core flags now, and an event for their copy
         launch_outputs(P, B, s, kOutCore);
         cudaEventRecordWithFlags(core_out, s, cudaEventRecordExternal);
@@ -304,8 +319,7 @@ void launch_graph(const Plan &P, const Buffers &B, bool trees, cudaStream_t s, c
         k_depth<<<gu, kThreads, 0, s>>>(P.N, B.row2uid, B.urow, B.ucore, B.bmin, B.parent,
                                          B.depth_hist);
     }
-    cudaMemsetAsync(B.rootflag, 0, sizeof(uint32_t) * ((size_t)P.N + 1), s);
-    k_compress<<<grid_wave(k_compress, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ucore, B.parent, B.rootflag);
+    k_compress<<<grid_wave(k_compress, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ucore, B.parent, B.rootflag, P.N, nullptr);
     scan_u32(B.rootflag, B.rootflag, P.N + 1, nullptr, &B.ctr->n_clusters, B.scan_part,
              B.scan_part_cap, s);
     k_labels<<<grid_wave(k_labels, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ucore, B.parent, B.bmin, B.rootflag, B.urep,
@@ -318,7 +332,7 @@ void launch_graph(const Plan &P, const Buffers &B, bool trees, cudaStream_t s, c
 // statistics are cleared between the sweeps so that they count one sweep.
 void launch_streamed_sweeps(const Plan &P, const Buffers &B, cudaStream_t s) {
     launch_distance(P, B, 0, s, kSinkCount);
-    k_core<<<grid_wave(k_core, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ctr, B.cnt, P.min_pts, B.ucore, B.parent);
+    k_core<<<grid_wave(k_core, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ctr, B.cnt, P.min_pts, B.ucore, B.parent, nullptr);
     cudaMemsetAsync(&B.ctr->pairs_evaluated, 0, sizeof(B.ctr->pairs_evaluated), s);
     cudaMemsetAsync(&B.ctr->n_edges, 0, sizeof(B.ctr->n_edges), s);
     cudaMemsetAsync(&B.ctr->edge_reserved, 0, sizeof(B.ctr->edge_reserved), s);
@@ -332,8 +346,7 @@ void launch_streamed_labels(const Plan &P, const Buffers &B, bool trees, cudaStr
         k_depth<<<grid_for(P.N), kThreads, 0, s>>>(P.N, B.row2uid, B.urow, B.ucore, B.bmin, B.parent,
                                                    B.depth_hist);
     }
-    cudaMemsetAsync(B.rootflag, 0, sizeof(uint32_t) * ((size_t)P.N + 1), s);
-    k_compress<<<grid_wave(k_compress, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ucore, B.parent, B.rootflag);
+    k_compress<<<grid_wave(k_compress, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ucore, B.parent, B.rootflag, P.N, B.stamp(3));
     scan_u32(B.rootflag, B.rootflag, P.N + 1, nullptr, &B.ctr->n_clusters, B.scan_part,
              B.scan_part_cap, s);
     k_labels<<<grid_wave(k_labels, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ucore, B.parent, B.bmin, B.rootflag, B.urep,
@@ -343,7 +356,7 @@ void launch_streamed_labels(const Plan &P, const Buffers &B, bool trees, cudaStr
 void launch_outputs(const Plan &P, const Buffers &B, cudaStream_t s, uint32_t what) {
     const int gu = grid_for(P.N);
     k_rows_out<<<grid_wave(k_rows_out, P.N, kThreads), kThreads, 0, s>>>(P.N, P.min_pts, B.row2uid, B.urow, B.ucopies, B.ucore,
-                                        B.cnt, B.clone_id, B.core, B.copies, B.ctr, what);
+                                        B.cnt, B.clone_id, B.core, B.copies, B.ctr, what, B.stamp(4));
     if (B.uniques && (what & kOutClone)) k_uniques_out<<<gu, kThreads, 0, s>>>(B.ctr, B.urow, B.uniques);
 }
 

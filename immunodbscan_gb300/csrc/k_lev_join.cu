@@ -122,11 +122,12 @@ __device__ __forceinline__ void for_probes(const LevJoinGeom &g, const uint32_t 
 
 __global__ void __launch_bounds__(kThreads)
 k_ljoin_clear(Counters *ctr, uint32_t smax, uint32_t nc, uint64_t cap_mask,
-              unsigned long long *__restrict__ key, uint32_t *__restrict__ cnt) {
+              unsigned long long *__restrict__ key, uint32_t *__restrict__ cnt, unsigned long long *stamp) {
+    stamp_begin(stamp);
     const uint32_t n = join_mask(ctr->n_uniques, smax, cap_mask) + 1u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         ctr->n_jslots = n;
-        ctr->n_groups = 0;
+        ctr->n_binpairs = 0;
         ctr->n_entries = 0;
         ctr->join_pairs = 0;
     }
@@ -255,7 +256,7 @@ k_ljoin_groups(Counters *ctr, uint32_t nc, const uint32_t *__restrict__ tcnt,
                 tb += x.x;
                 te += x.y;
             }
-            if (tb) s_base = make_uint2(atomicAdd(&ctr->n_groups, tb), atomicAdd(&ctr->n_entries, te));
+            if (tb) s_base = make_uint2(atomicAdd(&ctr->n_binpairs, tb), atomicAdd(&ctr->n_entries, te));
         }
         __syncthreads();
         if (bps) {
@@ -346,7 +347,6 @@ k_ljoin_bp_fill(LevJoinGeom g, const Counters *__restrict__ ctr, const unsigned 
             if (at >= cap_bp) { atomicOr(err, kErrBinPairOverflow); ++at; continue; }
             BinPair P;
             P.a_start = first; P.a_n = m; P.b_start = s0; P.b_n = c0;
-            P.unit_base = 0;
             P.ncx = (m + TX - 1) / TX;
             P.la = (uint16_t)(c > 1 ? n - (c - 1) : n); P.lb = (uint16_t)n;
             P.v = (uint16_t)k;                      // segment of the group
@@ -389,7 +389,7 @@ void ljoin_fill(const Plan &P, const Buffers &B, cudaStream_t s) {
 void launch_lev_join(const Plan &P, const Buffers &B, cudaStream_t s) {
     const uint64_t slots = B.jn_mask + 1;
     k_ljoin_clear<<<grid_wave(k_ljoin_clear, slots * P.join_classes / 4, kThreads), kThreads, 0, s>>>(
-        B.ctr, P.join_smax, P.join_classes, B.jn_mask, B.jn_key, B.jn_cnt);
+        B.ctr, P.join_smax, P.join_classes, B.jn_mask, B.jn_key, B.jn_cnt, B.stamp(1));
     switch (P.W) {
         case 1: ljoin_build<1>(P, B, s); break;
         case 2: ljoin_build<2>(P, B, s); break;
