@@ -65,12 +65,12 @@ struct DevBuf {
 };
 
 enum BufId {
-    bSeq, bSeqOff, bV, bVOff, bJ, bJOff, bVGenes, bVGOff, bJGenes, bJGOff, bRepOff, bEps, bCode,
+    bSeq, bSeqOff, bV, bVOff, bJ, bJOff, bTables, bPlanTables,
     bVBits, bJBits, bSlot, bRepRow, bFlag, bUidOfRow, bRow2Uid, bTable, bTCount,
     bURow, bUCopies, bULen, bURep, bBinHist, bBinCursor, bEntUid, bEntRec, bBpCount, bBp,
     bBpSorted, bBpUnits, bClsHist, bPred, bEdges, bCnt, bUCore,
     bParent, bBMin, bRootFlag, bUidFirst, bDepth, bScanPart, bClone, bCore, bCopies, bUniques,
-    bCtr, bVTab, bJTab, bSigAnd, bUClass, bEntMeta, bCallTab, bCallRef, bCallTodo, bBpSmall,
+    bCtr, bSigAnd, bUClass, bEntMeta, bCallTab, bCallRef, bCallTodo, bBpSmall,
     bJnTab, bJnISlot, bJnStart, bJnCur, bJnBpIdx, bJnPos, bEntCopies, bNumBufs
 };
 
@@ -268,15 +268,33 @@ idb_status validate(const idb_input *in, const idb_params *prm, const idb_output
     return IDB_OK;
 }
 
-// Gene name lists -> device (host memory always), plus the hash table of the
-// names used by the gene-bitset kernel.
-idb_status upload_genes(idb_context *c, const char *names, const int64_t *off, uint32_t G,
-                        BufId blob_id, BufId off_id, BufId tab_id, uint32_t *bytes_out,
-                        GeneMatcher *gm) {
-    ++c->stage_epoch;   // the gene tables a captured graph reads are replaced
+// Small host tables of a call (repertoire offsets, gene lists; eps and codes)
+// gathered for one copy to the device.  The copy is from pageable memory: the
+// bytes are staged when the call returns, so no wait is needed.
+struct HostPack {
+    std::vector<char> bytes;
+    size_t add(const void *p, size_t n) {
+        const size_t at = (bytes.size() + 15) & ~(size_t)15;
+        bytes.resize(at + n);
+        if (n) std::memcpy(bytes.data() + at, p, n);
+        return at;
+    }
+    idb_status upload(idb_context *c, BufId id) const {
+        TRY(ensure(c, id, bytes.size()));
+        CU(cudaMemcpyAsync(c->buf[id].p, bytes.data(), bytes.size(), cudaMemcpyHostToDevice, c->stream));
+        return IDB_OK;
+    }
+};
+
+// A gene name list (host memory always) and the hash table of the names used by
+// the gene-bitset kernel, into the pack; places of the names, offsets and table.
+struct GenePlace { size_t names, off, tab; };
+
+GenePlace pack_genes(HostPack &pack, const char *names, const int64_t *off, uint32_t G,
+                     uint32_t *bytes_out, GeneMatcher *gm) {
     std::vector<int32_t> o(G + 1);
     const int64_t base = G ? off[0] : 0;
-    for (uint32_t g = 0; g <= G; ++g) o[g] = (int32_t)(off[g] - base);
+    for (uint32_t g = 0; g <= G; ++g) o[g] = G ? (int32_t)(off[g] - base) : 0;
     const size_t nb = G ? (size_t)(off[G] - base) : 0;
     // table: slots >= 2*G, power of two
     *gm = GeneMatcher();
@@ -298,17 +316,12 @@ idb_status upload_genes(idb_context *c, const char *names, const int64_t *off, u
         gm->maxlen = std::max(gm->maxlen, L);
     }
     gm->ts = ts;
-    TRY(ensure(c, blob_id, nb + 16));
-    TRY(ensure(c, off_id, sizeof(int32_t) * (G + 1)));
-    TRY(ensure(c, tab_id, sizeof(GeneEntry) * ts));
-    if (nb) CU(cudaMemcpyAsync(c->buf[blob_id].p, names + base, nb, cudaMemcpyHostToDevice, c->stream));
-    CU(cudaMemcpyAsync(c->buf[off_id].p, o.data(), sizeof(int32_t) * (G + 1), cudaMemcpyHostToDevice,
-                       c->stream));
-    CU(cudaMemcpyAsync(c->buf[tab_id].p, tab.data(), sizeof(GeneEntry) * ts, cudaMemcpyHostToDevice,
-                       c->stream));
-    CU(cudaStreamSynchronize(c->stream));   // o and tab are locals
     *bytes_out = (uint32_t)nb;
-    return IDB_OK;
+    GenePlace at;
+    at.names = pack.add(G ? names + base : nullptr, nb);
+    at.off = pack.add(o.data(), sizeof(int32_t) * (G + 1));
+    at.tab = pack.add(tab.data(), sizeof(GeneEntry) * ts);
+    return at;
 }
 
 struct Pipeline {
@@ -467,22 +480,24 @@ idb_status stage_inputs_and_survey(Pipeline &pl, const idb_input *in, bool host_
         roff[0] = 0;
         roff[1] = P.N;
     }
-    TRY(ensure(c, bRepOff, sizeof(uint32_t) * (P.R + 1)));
-    CU(cudaMemcpyAsync(c->buf[bRepOff].p, roff.data(), sizeof(uint32_t) * (P.R + 1),
-                       cudaMemcpyHostToDevice, s));
-    B.rep_off = ptr<uint32_t>(c, bRepOff);
+    HostPack pack;
+    const size_t rep_at = pack.add(roff.data(), sizeof(uint32_t) * (P.R + 1));
     // gene lists
     P.Gv = P.no_v ? 1 : in->n_v_genes;
     P.Gj = P.no_j ? 1 : in->n_j_genes;
-    if (!P.no_v)
-        TRY(upload_genes(c, in->v_genes, in->v_gene_offsets, P.Gv, bVGenes, bVGOff, bVTab,
-                         &P.gene_bytes_v, &P.vmatch));
-    if (!P.no_j)
-        TRY(upload_genes(c, in->j_genes, in->j_gene_offsets, P.Gj, bJGenes, bJGOff, bJTab,
-                         &P.gene_bytes_j, &P.jmatch));
-    B.vgenes = ptr<uint8_t>(c, bVGenes); B.vg_off = ptr<int32_t>(c, bVGOff);
-    B.jgenes = ptr<uint8_t>(c, bJGenes); B.jg_off = ptr<int32_t>(c, bJGOff);
-    B.vtab = ptr<GeneEntry>(c, bVTab); B.jtab = ptr<GeneEntry>(c, bJTab);
+    GenePlace gv{}, gj{};
+    if (!P.no_v) gv = pack_genes(pack, in->v_genes, in->v_gene_offsets, P.Gv, &P.gene_bytes_v, &P.vmatch);
+    if (!P.no_j) gj = pack_genes(pack, in->j_genes, in->j_gene_offsets, P.Gj, &P.gene_bytes_j, &P.jmatch);
+    TRY(pack.upload(c, bTables));
+    const uint8_t *tp = ptr<uint8_t>(c, bTables);
+    B.rep_off = reinterpret_cast<const uint32_t *>(tp + rep_at);
+    auto column = [&](const GenePlace &at, const uint8_t **names, const int32_t **off, const GeneEntry **tab) {
+        *names = tp + at.names;
+        *off = reinterpret_cast<const int32_t *>(tp + at.off);
+        *tab = reinterpret_cast<const GeneEntry *>(tp + at.tab);
+    };
+    column(gv, &B.vgenes, &B.vg_off, &B.vtab);
+    column(gj, &B.jgenes, &B.jg_off, &B.jtab);
     P.VW = P.Gv > 64 ? (P.Gv + 63) / 64 : 1;
     P.JW = P.Gj > 64 ? (P.Gj + 63) / 64 : 1;
     if (P.Gv == 0) P.Gv = 1;   // a V column with an empty reference list: all bitsets 0
@@ -649,13 +664,12 @@ idb_status alloc_fixed(Pipeline &pl) {
     Plan &P = pl.P;
     Buffers &B = pl.B;
     const size_t N = P.N, N1 = N + 1;
-    TRY(ensure(c, bEps, sizeof(int16_t) * pl.eps_host.size()));
-    TRY(ensure(c, bCode, 256));
-    CU(cudaMemcpyAsync(c->buf[bEps].p, pl.eps_host.data(), sizeof(int16_t) * pl.eps_host.size(),
-                       cudaMemcpyHostToDevice, c->stream));
-    CU(cudaMemcpyAsync(c->buf[bCode].p, P.codemap, 256, cudaMemcpyHostToDevice, c->stream));
-    B.eps_tab = ptr<int16_t>(c, bEps);
-    B.codemap = ptr<uint8_t>(c, bCode);
+    HostPack pack;
+    const size_t eps_at = pack.add(pl.eps_host.data(), sizeof(int16_t) * pl.eps_host.size());
+    const size_t code_at = pack.add(P.codemap, 256);
+    TRY(pack.upload(c, bPlanTables));
+    B.eps_tab = reinterpret_cast<const int16_t *>(ptr<uint8_t>(c, bPlanTables) + eps_at);
+    B.codemap = ptr<uint8_t>(c, bPlanTables) + code_at;
     TRY(ensure(c, bVBits, sizeof(uint64_t) * N * P.VW));
     TRY(ensure(c, bJBits, sizeof(uint64_t) * N * P.JW));
     TRY(ensure(c, bSlot, 4 * N));
@@ -903,7 +917,7 @@ idb_status run_phases(Pipeline &pl, bool eager, bool stop_after_schedule = false
     launch_binpairs(P, B, s);
     TRY(check_launch());
     if (eager) {
-        TRY(read_counters(pl));
+        if (!P.join) TRY(read_counters(pl));   // a join counted them with its entries
         TRY(alloc_binpairs(pl, c->h_ctr->n_binpairs));
     }
     launch_binpairs_fill(P, B, s);
@@ -1595,11 +1609,14 @@ idb_status idb_diag_gene_bits(idb_context *c, const char *calls, const int64_t *
     if (nbytes) CU(cudaMemcpyAsync(c->buf[bV].p, calls, nbytes, cudaMemcpyHostToDevice, c->stream));
     CU(cudaMemcpyAsync(c->buf[bVOff].p, offsets, sizeof(int64_t) * ((size_t)n_rows + 1),
                        cudaMemcpyHostToDevice, c->stream));
-    TRY(upload_genes(c, genes, gene_offsets, n_genes, bVGenes, bVGOff, bVTab, &P.gene_bytes_v,
-                     &P.vmatch));
+    HostPack pack;
+    ++c->stage_epoch;   // a captured graph's gene tables are replaced
+    const GenePlace at = pack_genes(pack, genes, gene_offsets, n_genes, &P.gene_bytes_v, &P.vmatch);
+    TRY(pack.upload(c, bTables));
     B.vcall = ptr<uint8_t>(c, bV); B.v_off = ptr<int64_t>(c, bVOff);
-    B.vgenes = ptr<uint8_t>(c, bVGenes); B.vg_off = ptr<int32_t>(c, bVGOff);
-    B.vtab = ptr<GeneEntry>(c, bVTab);
+    B.vgenes = ptr<uint8_t>(c, bTables) + at.names;
+    B.vg_off = reinterpret_cast<const int32_t *>(ptr<uint8_t>(c, bTables) + at.off);
+    B.vtab = reinterpret_cast<const GeneEntry *>(ptr<uint8_t>(c, bTables) + at.tab);
     B.vbits = ptr<uint64_t>(c, bVBits);
     TRY(alloc_call_scratch(c, B, n_rows));
     set_row_chunks(P, false, 1);
