@@ -138,7 +138,10 @@ struct EdgeWriter {
         }
     }
 
-    // warp-uniform call; lanes with ok=true append (lo, hi)
+    // warp-uniform call; lanes with ok=true append (lo, hi).  The byte and the
+    // Myers kernels leave the counts of a stored list to k_count: per pair they
+    // cost more here, where a lane waits for both ends' copies.
+    template <bool COUNT>
     __device__ void append(const DistArgs &a, int lane, bool ok, uint32_t lo, uint32_t hi) {
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, ok);
         if (!m) return;
@@ -155,7 +158,8 @@ struct EdgeWriter {
         }
         if (ok) {
             put_edge(a, base + fill + __popc(m & lanemask_lt()), lo, hi);
-            count_pair(a, lo, hi, __ldg(&a.ucopies[lo]), __ldg(&a.ucopies[hi]));
+            if (COUNT || a.sink == kSinkCount)
+                count_pair(a, lo, hi, __ldg(&a.ucopies[lo]), __ldg(&a.ucopies[hi]));
         }
         fill += n;
         written += n;

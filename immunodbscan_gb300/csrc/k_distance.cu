@@ -197,7 +197,7 @@ k_levenshtein(DistArgs a) {
                             bool ok = hit;
                             const uint4 mx = sxm[r * 32 + owner], my = sym[tt];
                             if (ok) ok = canonical_meta(a, U.P, mx, my);
-                            ew.append(a, lane, ok, min(mx.w, my.w), max(mx.w, my.w));
+                            ew.append<false>(a, lane, ok, min(mx.w, my.w), max(mx.w, my.w));
                         }
                     }
                     qn = 0;
@@ -291,7 +291,7 @@ k_generic(DistArgs a) {
                     }
                 }
             }
-            ew.append(a, lane, ok, min(ux, uy), max(ux, uy));
+            ew.append<false>(a, lane, ok, min(ux, uy), max(ux, uy));
         }
         log_unit(a, U, lane);
     }

@@ -57,6 +57,38 @@ __global__ void k_graph_init(Counters *ctr, const uint32_t *__restrict__ ucopies
     }
 }
 
+// Copies-weighted counts (S5) from the edge list, and a smaller neighbour for the
+// larger end, for the kernels that do not sum them as they find the pairs (more
+// than 32 residue values, long sequences, edit distances above 3).  Bound by the
+// count updates; four edges' loads in flight per thread.
+__global__ void __launch_bounds__(kThreads)
+k_count(const Counters *__restrict__ ctr, uint64_t cap, const uint2 *__restrict__ edges,
+        const uint32_t *__restrict__ ucopies, uint32_t *__restrict__ cnt, uint32_t *__restrict__ parent,
+        unsigned long long *stamp) {
+    stamp_begin(stamp);
+    const uint32_t ne = edge_slots(ctr, cap) & ~3u;   // reserved in chunks of 256
+    const uint64_t stride = 4ull * gridDim.x * blockDim.x;
+    for (uint64_t e0 = 4ull * (blockIdx.x * blockDim.x + threadIdx.x); e0 < ne; e0 += stride) {
+        const uint4 v0 = __ldcs(reinterpret_cast<const uint4 *>(edges + e0));
+        const uint4 v1 = __ldcs(reinterpret_cast<const uint4 *>(edges + e0 + 2));
+        const uint2 ed[4] = {{v0.x, v0.y}, {v0.z, v0.w}, {v1.x, v1.y}, {v1.z, v1.w}};
+        uint32_t cx[4], cy[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (ed[k].x != kNone) {
+                cx[k] = __ldg(ucopies + ed[k].x);
+                cy[k] = __ldg(ucopies + ed[k].y);
+            }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (ed[k].x != kNone) {
+                atomicAdd(&cnt[ed[k].x], cy[k]);
+                atomicAdd(&cnt[ed[k].y], cx[k]);
+                parent[ed[k].y] = ed[k].x;   // edges are (smaller, larger)
+            }
+    }
+}
+
 // Core flags (S5) and the forest the unions start from: every core is its own
 // root, or under the smaller neighbour the distance kernel left in its parent
 // when that is core too (such an edge is a union); a non-core unique is marked.
@@ -300,7 +332,11 @@ void launch_graph_init(const Plan &P, const Buffers &B, cudaStream_t s) {
 void launch_graph(const Plan &P, const Buffers &B, bool trees, cudaStream_t s, cudaEvent_t core_out) {
     const uint64_t ecap = P.cap_edges;
     const int gu = grid_for(P.N);
-    k_core<<<grid_wave(k_core, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ctr, B.cnt, P.min_pts, B.ucore, B.parent, B.stamp(3));
+    const bool counted = P.planes();   // by the distance kernel
+    if (!counted)
+        k_count<<<grid_wave(k_count, ecap / 4, kThreads), kThreads, 0, s>>>(B.ctr, ecap, B.edges, B.ucopies, B.cnt,
+                                                                        B.parent, B.stamp(3));
+    k_core<<<grid_wave(k_core, P.N, kThreads), kThreads, 0, s>>>(B.ctr, B.ctr, B.cnt, P.min_pts, B.ucore, B.parent, counted ? B.stamp(3) : nullptr);
     if (core_out) {   // the row core flags now, and an event for their copy
         launch_outputs(P, B, s, kOutCore);
         cudaEventRecordWithFlags(core_out, s, cudaEventRecordExternal);

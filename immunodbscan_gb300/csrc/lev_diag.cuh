@@ -486,7 +486,7 @@ __device__ __forceinline__ void lev_tiny_all(const DistArgs &a, EdgeWriter &ew, 
                 ux = __ldg(&a.meta[P.a_start + p % n].w);
                 uy = __ldg(&a.meta[ystart + p / n].w);
             }
-            ew.append(a, lane, rest != 0, min(ux, uy), max(ux, uy));
+            ew.append<true>(a, lane, rest != 0, min(ux, uy), max(ux, uy));
             rest &= rest - 1;
         }
         if (a.bp_cycles) {   // the batch's cycles, shared out by pairs
