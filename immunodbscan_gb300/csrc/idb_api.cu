@@ -344,7 +344,7 @@ struct Pipeline {
     // that a replay copies them to the host while the rest of the path runs
     bool early_out = false;
     bool copies_issued = false;
-    bool own_shape = true;    // the caller asked for no unit shape
+    int tile_rx = 0, tile_ty = 0;   // the unit shape the caller asked for (0: none)
     bool allow_join = true;   // the segment join finds neighbours, not all admissible pairs
     // every return path (errors included) leaves no copy from the caller's host
     // buffers in flight
@@ -588,24 +588,24 @@ idb_status derive_plan(Pipeline &pl, const idb_params *prm) {
         P.TX = 32 * P.RX;
         P.TY = 256;
     }
-    if (P.fast) apply_shape(P, prm->tile_rx, prm->tile_ty);
-    pl.own_shape = prm->tile_rx <= 0 && prm->tile_ty <= 0;
+    pl.tile_rx = prm->tile_rx;
+    pl.tile_ty = prm->tile_ty;
+    if (P.fast) apply_shape(P, pl.tile_rx, pl.tile_ty);
     P.dLmax = P.hamming ? 0 : dl;
     P.hamming_eps_mode = 0;
     if (P.hamming && emin_same == emax_same && emin_same == 1) P.hamming_eps_mode = 1;
     if (P.hamming && emin_same == emax_same && emin_same == 0) P.hamming_eps_mode = 2;
     P.K = 4;
     P.big_group = 64;
-    P.sig_exact = P.Gv <= 64 && P.Gj <= 32;
+    P.wide = P.Gv > 64 || P.Gj > 30;
     // Hamming with a small eps at every length: candidate pairs by segment join
     // (the side records then carry the V bits and the J bits with the segment;
     // a key holds the repertoire in 24 bits and the table at most 2^31 slots)
     P.join = pl.allow_join && prm->candidates == 0 && P.hamming && P.fast && emax_same <= kJoinMaxEps &&
-             P.Gv <= 64 && P.Gj <= 30 && P.R < (1u << 24) - 1 &&
+             P.R < (1u << 24) - 1 &&
              2ull * (uint64_t)(emax_same + 1) * P.N <= (1ull << 30);
     P.join_smax = P.join ? (uint32_t)std::max(1, emax_same + 1) : 1u;
     P.join_classes = 1;
-    P.vj_meta = P.Gv <= 64 && P.Gj <= 30;
     if (pl.allow_join && prm->candidates == 0 && P.lev_diag && P.R < (1u << 24) - 1) {
         // Levenshtein: the join too (an eager call may still take the buckets,
         // choose_candidates); the table and its class counts stay below 2^31
@@ -880,6 +880,21 @@ idb_status choose_candidates(Pipeline &pl) {
     Buffers &B = pl.B;
     cudaStream_t s = c->stream;
     TRY(read_counters(pl));
+    if (P.wide) {
+        P.compact = c->h_ctr->vj_compact != 0;
+        if (!P.compact && P.join && P.hamming) {
+            // the Hamming join's side records hold the genes: the buckets instead,
+            // in their unit shape
+            P.join = P.front_join = false;
+            P.RX = P.W == 1 ? 8 : 4;
+            P.TX = 32 * P.RX;
+            P.TY = 256;
+            apply_shape(P, pl.tile_rx == 2 ? 4 : pl.tile_rx, pl.tile_ty);
+            launch_buckets(P, B, s);
+            TRY(check_launch());
+            TRY(read_counters(pl));
+        }
+    }
     if (P.join && !P.hamming && c->h_ctr->join_pairs > kJoinSurePairs) {
         const uint32_t join_entries = c->h_ctr->n_entries;
         const unsigned long long join_pairs = c->h_ctr->join_pairs;
@@ -895,7 +910,7 @@ idb_status choose_candidates(Pipeline &pl) {
                                cudaMemcpyHostToDevice, s));
         }
     }
-    if (P.join && !P.hamming && pl.own_shape) set_join_shape(P, c->h_ctr->join_pairs);
+    if (P.join && !P.hamming && pl.tile_rx <= 0 && pl.tile_ty <= 0) set_join_shape(P, c->h_ctr->join_pairs);
     return alloc_entries(pl, c->h_ctr->n_entries);
 }
 

@@ -175,6 +175,10 @@ struct Counters {
     uint32_t n_jslots;           // segment join: table slots in use (the probed prefix)
     uint32_t chunk_uniques[kMaxRowChunks];   // uniques of each row chunk (numbered by chunk)
     uint32_t call_todo[2 * kMaxRowChunks];   // rows that compute their own bitset, per column and chunk
+    // wide gene lists (more than 64 V or 30 J genes): the genes some unique has, and
+    // whether they fit the side records renumbered (64 V, 30 J)
+    unsigned long long used_v[kMaxGeneWords], used_j[kMaxGeneWords];
+    uint32_t used_done, vj_compact;
     unsigned long long join_pairs;    // edit-distance join: candidate pairs of its groups
     unsigned long long bucket_pairs;  // pairs of the buckets (an upper bound), when compared with it
     uint32_t n_tiny;             // tiny bin pairs (one lane each), listed from the small list's end
@@ -219,7 +223,6 @@ struct Plan {
     uint32_t TX = 256, TY = 256, RX = 8;          // unit shape (entries)
     int schedule = 0;
     int hamming_eps_mode = 0;                     // 0 popcount, 1 eps==1, 2 eps==0
-    bool sig_exact = true;                        // V genes <= 64 and J genes <= 32
     bool lev_diag = false;                        // Levenshtein by the diagonal test
     // records are bit planes (else one code byte per residue)
     bool planes() const { return fast && (hamming || lev_diag); }
@@ -227,7 +230,10 @@ struct Plan {
                                                   // kJoinMaxEps; Levenshtein by the diagonal test)
     uint32_t join_classes = 1;                    // counts per table slot (Levenshtein: the indexed
                                                   // uniques, then one per length gap and shift)
-    bool vj_meta = true;                          // side records of the join hold the V and J bits
+    bool wide = false;                            // V genes > 64 or J genes > 30, and then whether the genes
+    bool compact = false;                         // in use fit the side records renumbered (an eager
+                                                  // call reads it, a captured plan expects it)
+    bool side_exact() const { return !wide || compact; }   // side records hold every gene in use
     uint32_t join_smax = 1;                       // most segments of any length
     bool streamed = false;                        // neighbour pairs not stored: the
                                                   // distance work runs twice
@@ -349,6 +355,7 @@ void launch_uniques_rows(const Plan &P, const Buffers &B, uint32_t chunk, cudaSt
 void launch_uniques_finish(const Plan &P, const Buffers &B, cudaStream_t s);
 void launch_uniques(const Plan &P, const Buffers &B, cudaStream_t s);
 void launch_buckets(const Plan &P, const Buffers &B, cudaStream_t s);
+void launch_gene_used(const Plan &P, const Buffers &B, cudaStream_t s);   // wide lists, in launch_buckets
 // segment join: clear the table (sized by the rows when front_join), then the
 // inserts of every unique (chunk < 0) or of one row chunk's uniques
 void launch_join_init(const Plan &P, const Buffers &B, cudaStream_t s);

@@ -364,11 +364,11 @@ static DistArgs make_args(const Plan &P, const Buffers &B) {
     a.bp_cycles = B.bp_cycles;   // set only while profiling
     a.bp_hits = B.bp_hits;
     a.meta = B.ent_meta;
-    a.sig_exact = (P.sig_exact && !P.join) ? 1 : 0;
+    a.sig_exact = (P.side_exact() && !P.join) ? 1 : 0;
     a.small_list = B.bp_small;
     a.small_cap = (uint32_t)P.cap_binpairs + 1u;
     a.join = P.join ? 1 : 0;
-    a.vj_meta = P.vj_meta ? 1 : 0;
+    a.vj_meta = P.side_exact() ? 1 : 0;
     a.sink = kSinkEdges;
     a.cnt = B.cnt;
     a.ucopies = B.ucopies;

@@ -286,8 +286,8 @@ k_ljoin_fill(LevJoinGeom g, const Counters *__restrict__ ctr, const uint32_t *__
              const uint8_t *__restrict__ seq, const int64_t *__restrict__ seq_off,
              const uint8_t *__restrict__ codemap, const unsigned long long *__restrict__ tkey,
              const uint32_t *__restrict__ islot, const uint32_t *__restrict__ irank,
-             const uint32_t *__restrict__ start, uint32_t *cur, const uint64_t *__restrict__ vbits,
-             const uint64_t *__restrict__ jbits, uint32_t VW, uint32_t JW, uint4 *__restrict__ ent_rec,
+             const uint32_t *__restrict__ start, uint32_t *cur, GeneSide gv, GeneSide gj,
+             uint4 *__restrict__ ent_rec,
              uint4 *__restrict__ ent_meta, const uint32_t *__restrict__ ucopies,
              uint32_t *__restrict__ ent_copies, int planes, uint64_t cap_entries, uint32_t *err) {
     __shared__ uint8_t cm[256];
@@ -301,9 +301,9 @@ k_ljoin_fill(LevJoinGeom g, const Counters *__restrict__ ctr, const uint32_t *__
         build_planes(seq + seq_off[row], L, cm, wd);
         uint4 rec[RSC];
         flatten_planes<RSC>(wd, planes, (uint32_t)W, rec);
-        const uint64_t vb = vbits[(size_t)row * VW];
+        const uint64_t vb = gv.row(row);
         const uint32_t copies = ucopies[u];
-        const uint32_t jb = (uint32_t)jbits[(size_t)row * JW] & 0x3FFFFFFFu;
+        const uint32_t jb = (uint32_t)gj.row(row) & 0x3FFFFFFFu;
         auto put = [&](uint64_t pos, uint32_t shift) {
             if (pos >= cap_entries) { atomicOr(err, kErrEntryOverflow); return; }
             ent_meta[pos] = make_uint4((uint32_t)vb, (uint32_t)(vb >> 32), jb | (shift << 30), u);
@@ -380,7 +380,8 @@ void ljoin_fill(const Plan &P, const Buffers &B, cudaStream_t s) {
     auto kern = k_ljoin_fill<RSC, W>;
     kern<<<grid_wave(kern, P.N, kThreads), kThreads, 0, s>>>(
         lev_geom(P, B), B.ctr, B.urow, B.ulen, B.urep, B.seq, B.seq_off, B.codemap, B.jn_key, B.jn_islot,
-        B.jn_cur, B.jn_start, B.jn_pos, B.vbits, B.jbits, P.VW, P.JW, B.ent_rec, B.ent_meta, B.ucopies, B.ent_copies, (int)P.B,
+        B.jn_cur, B.jn_start, B.jn_pos, GeneSide{B.vbits, P.compact ? B.ctr->used_v : nullptr, P.VW},
+        GeneSide{B.jbits, P.compact ? B.ctr->used_j : nullptr, P.JW}, B.ent_rec, B.ent_meta, B.ucopies, B.ent_copies, (int)P.B,
         P.cap_entries, &B.ctr->error);
 }
 

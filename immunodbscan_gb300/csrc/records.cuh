@@ -106,6 +106,35 @@ __device__ __forceinline__ void build_small_record(const uint8_t *s, uint32_t L,
     }
 }
 
+// Gene bitsets as the side records hold them.  Wide lists whose genes in use fit
+// (64 V, 30 J): the genes no unique has are left out, order kept.
+struct GeneSide {
+    const uint64_t *bits;
+    const unsigned long long *used;   // null: the first word as it is
+    uint32_t W;
+    __device__ __forceinline__ uint64_t row(uint32_t r) const {
+        const uint64_t *b = bits + (size_t)r * W;
+        if (!used) return b[0];
+        uint64_t out = 0;
+        uint32_t base = 0;
+        for (uint32_t w = 0; w < W; ++w) {
+            for (uint64_t v = b[w]; v; v &= v - 1) out |= 1ull << (base + rank_in(w, lowest_bit64(v)));
+            base += (uint32_t)popc64(used[w]);
+        }
+        return out;
+    }
+    __device__ __forceinline__ uint32_t rank_in(uint32_t w, int bit) const {
+        return (uint32_t)popc64(used[w] & ((1ull << bit) - 1ull));
+    }
+    // place of gene g in row()
+    __device__ __forceinline__ uint32_t place(uint32_t g) const {
+        if (!used) return g;
+        uint32_t base = 0;
+        for (uint32_t w = 0; w < g / 64; ++w) base += (uint32_t)popc64(used[w]);
+        return base + rank_in(g / 64, (int)(g % 64));
+    }
+};
+
 __device__ __forceinline__ uint32_t seg_count(const int16_t *eps_tab, uint32_t NL, uint32_t li) {
     const int e = eps_tab[(size_t)li * NL + li];
     return e < 0 ? 1u : (uint32_t)e + 1u;
