@@ -465,8 +465,12 @@ def main():
     t_dist = r["ms_dist"] * 1e-3
     if w.use_hamming:
         work_ops = ops_pair * last.pairs_evaluated
-    else:                       # Myers/Hyyro: ops per text column actually consumed
+    elif last.lev_columns:      # Myers/Hyyro: ops per text column actually consumed
         work_ops = ops_pair * last.lev_columns
+    else:                       # diagonal test, eps 2, one word: three masks of 5 planes, 16 for the test
+        ops_pair = 31
+        work_ops = ops_pair * last.pairs_evaluated
+    per_column = not w.use_hamming and last.lev_columns > 0
     achieved = work_ops / t_dist / 1e9 if t_dist > 0 else 0.0
     out["roofline"] = {"bound": "int", "achieved": achieved, "peak": gops.value,
                        "unit": "Gop/s (32-bit integer logic)",
@@ -476,25 +480,25 @@ def main():
                        "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one "
                                          "launch at scale 0.2, scaled by the rows to full size "
                                          "(profiles/k_hamming_workload2_scale0.2.md)",
-                       "kernel": "k_hamming" if w.use_hamming else "k_levenshtein",
+                       "kernel": ("k_hamming" if w.use_hamming else
+                                  "k_levenshtein" if per_column else "k_lev_diag"),
                        "ops_per_unit": ops_pair,
-                       "work_unit": "pair" if w.use_hamming else "pair-column (text residue)",
-                       "work_units": int(last.pairs_evaluated if w.use_hamming else last.lev_columns),
+                       "work_unit": "pair-column (text residue)" if per_column else "pair",
+                       "work_units": int(last.lev_columns if per_column else last.pairs_evaluated),
                        "kernel_ms": t_dist * 1e3,
                        "hit_fraction": (float(last.neighbour_pairs) / float(last.pairs_evaluated)
                                         if w.use_hamming and last.pairs_evaluated else None),
                        "peak_source": "measured: idb_diag_int_peak (lop3/add chains, all SMs)"}
 
     # graph / union-find / border / renumber phases against HBM bandwidth.  The
-    # algorithmic bytes, kernel by kernel: init (copies read, count / parent /
-    # border-minimum written: 16 n_u); count pass (edge 8 B, both ends' copies
-    # 8 B, both ends' count updates 8 B: 24 E); core flags (8 n_u); union pass
-    # (edge 8 B, both ends' core flags 8 B: 16 E, and both ends' parents for a
-    # core-core edge: 8 E_cc); compress (12 n_u); scan of the root flags
-    # (8 n_u); labels (core, parent, border minimum, rank, repertoire, first
-    # unique read, label written: 28 n_u).  Border-minimum updates are left out.
-    n_u, E, E_cc = int(last.n_uniques), int(last.neighbour_pairs), int(last.core_edges)
-    graph_bytes = 40 * E + 8 * E_cc + 72 * n_u
+    # algorithmic bytes, kernel by kernel: core flags (count and parent read, flag
+    # and parent written: 16 n_u); union pass (edge 8 B, both ends' parents 8 B:
+    # 16 E); compress (12 n_u); scan of the root flags (8 n_u); labels (core,
+    # parent, border minimum, rank, repertoire, first unique read, label written:
+    # 28 n_u).  The counts come with the distance kernel; border-minimum updates
+    # and the sampled unions are left out.
+    n_u, E = int(last.n_uniques), int(last.neighbour_pairs)
+    graph_bytes = 16 * E + 64 * n_u
     graph_ms = float(np.mean([p[3] for p in r["phases"]]))
     hbm_peak = measured_hbm_peak()
     out["roofline_graph"] = {"bound": "hbm", "achieved": graph_bytes / (graph_ms * 1e-3) / 1e9,
