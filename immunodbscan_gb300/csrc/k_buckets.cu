@@ -318,7 +318,7 @@ template <bool FILL>
 __device__ __forceinline__ uint32_t visit_pairs(uint32_t sb, const PairGeom &pg,
                                                 const int16_t *eps_tab, const uint32_t *bin_start,
                                                 const unsigned long long *sig, BinPair *out,
-                                                uint32_t k, uint64_t cap_bp, uint32_t *err) {
+                                                uint32_t k, uint64_t cap_bp) {
     const uint32_t a0 = bin_start[sb], nA = bin_start[sb + 1] - a0;
     if (nA == 0) return 0;
     const uint32_t b = sb / pg.K, c = sb % pg.K;
@@ -335,7 +335,7 @@ __device__ __forceinline__ uint32_t visit_pairs(uint32_t sb, const PairGeom &pg,
             if (!sig_disjoint(sig, sb, sb2)) continue;
             if (FILL) {
                 const uint32_t kk = k + n;
-                if (kk >= cap_bp) { atomicOr(err, kErrBinPairOverflow); ++n; continue; }
+                if (kk >= cap_bp) { ++n; continue; }   // flagged by drop_overgrown
                 const uint32_t rest = b / pg.NL;
                 BinPair P;
                 P.a_start = a0; P.a_n = nA; P.b_start = b0; P.b_n = nB;
@@ -361,17 +361,18 @@ __global__ void k_binpairs_count(uint32_t nsub, PairGeom pg, const int16_t *__re
                                  uint32_t *__restrict__ cnt) {
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t sb = blockIdx.x * blockDim.x + threadIdx.x; sb < nsub; sb += stride)
-        cnt[sb] = visit_pairs<false>(sb, pg, eps_tab, bin_start, sig, nullptr, 0, 0, nullptr);
+        cnt[sb] = visit_pairs<false>(sb, pg, eps_tab, bin_start, sig, nullptr, 0, 0);
 }
 
 __global__ void k_binpairs_fill(uint32_t nsub, PairGeom pg, const int16_t *__restrict__ eps_tab,
                                 const uint32_t *__restrict__ bin_start,
                                 const unsigned long long *__restrict__ sig,
-                                const uint32_t *__restrict__ bp_off, uint64_t cap_bp,
-                                BinPair *__restrict__ out, uint32_t *err) {
+                                const uint32_t *__restrict__ bp_off, uint64_t cap_bp, uint64_t cap_entries,
+                                BinPair *__restrict__ out, Counters *ctr) {
+    drop_overgrown(ctr, cap_bp, cap_entries);
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t sb = blockIdx.x * blockDim.x + threadIdx.x; sb < nsub; sb += stride)
-        visit_pairs<true>(sb, pg, eps_tab, bin_start, sig, out, bp_off[sb], cap_bp, err);
+        visit_pairs<true>(sb, pg, eps_tab, bin_start, sig, out, bp_off[sb], cap_bp);
 }
 
 // Pairs of the buckets, before the signatures leave any out.
@@ -707,10 +708,11 @@ k_join_fill(BinGeom g, const Counters *__restrict__ ctr, const uint32_t *__restr
 
 // One bin pair (a group against itself) per key held by two or more uniques:
 // a sequential pass over the probed prefix of the table.
-__global__ void k_join_bp_fill(BinGeom g, const Counters *__restrict__ ctr,
+__global__ void k_join_bp_fill(BinGeom g, Counters *ctr,
                                const unsigned long long *__restrict__ tkey, const uint32_t *__restrict__ tcnt,
                                const uint32_t *__restrict__ start, const uint32_t *__restrict__ bpidx, const int16_t *__restrict__ eps_tab,
-                               uint32_t TX, uint64_t cap_bp, BinPair *__restrict__ out, uint32_t *err) {
+                               uint32_t TX, uint64_t cap_bp, uint64_t cap_entries, BinPair *__restrict__ out) {
+    drop_overgrown(ctr, cap_bp, cap_entries);
     const uint32_t ns = ctr->n_jslots;   // a power of two >= 1024: whole quads of slots
     const uint32_t stride = 4 * gridDim.x * blockDim.x;
     for (uint32_t h0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x); h0 < ns; h0 += stride) {
@@ -723,7 +725,7 @@ __global__ void k_join_bp_fill(BinGeom g, const Counters *__restrict__ ctr,
             if (s0 == kNone) continue;
             const uint32_t c = tcnt[h];
             const uint32_t k = bpidx[h];
-            if (k >= cap_bp) { atomicOr(err, kErrBinPairOverflow); continue; }
+            if (k >= cap_bp) continue;   // flagged above
             const unsigned long long key = tkey[h];
             const uint32_t L = (uint32_t)(key >> 32) & 0xFFu;
             const uint32_t li = L - g.Lmin;
@@ -870,15 +872,15 @@ void launch_binpairs_fill(const Plan &P, const Buffers &B, cudaStream_t s) {
     if (P.join) {
         BinGeom g{P.Gv, P.Gj, P.NL, P.Lmin, P.VW, P.JW, P.K};
         k_join_bp_fill<<<grid_wave(k_join_bp_fill, (B.jn_mask + 1) / 4, kThreads), kThreads, 0, s>>>(
-            g, B.ctr, B.jn_key, B.jn_cnt, B.jn_start, B.jn_bpidx, B.eps_tab, P.TX, P.cap_binpairs, B.bp,
-            &B.ctr->error);
+            g, B.ctr, B.jn_key, B.jn_cnt, B.jn_start, B.jn_bpidx, B.eps_tab, P.TX, P.cap_binpairs,
+            P.cap_entries, B.bp);
         return;
     }
     PairGeom pg{P.NL, P.Lmin, P.Gv, P.Gj, P.K, P.dLmax, P.hamming, P.TX, P.TY, P.TY / P.TX};
     const uint32_t nb = (uint32_t)P.nbins;
     k_binpairs_fill<<<grid_for(nb), kThreads, 0, s>>>(nb, pg, B.eps_tab, B.bin_hist, B.sig_and,
-                                                       B.bp_count, P.cap_binpairs, B.bp,
-                                                       &B.ctr->error);
+                                                       B.bp_count, P.cap_binpairs, P.cap_entries, B.bp,
+                                                       B.ctr);
 }
 
 void launch_bucket_pairs(const Plan &P, const Buffers &B, cudaStream_t s) {

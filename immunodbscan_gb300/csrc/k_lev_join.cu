@@ -327,10 +327,11 @@ k_ljoin_fill(LevJoinGeom g, const Counters *__restrict__ ctr, const uint32_t *__
 
 // Bin pairs of every group: class 0 with itself, every other class with class 0.
 __global__ void __launch_bounds__(kThreads)
-k_ljoin_bp_fill(LevJoinGeom g, const Counters *__restrict__ ctr, const unsigned long long *__restrict__ tkey,
+k_ljoin_bp_fill(LevJoinGeom g, Counters *ctr, const unsigned long long *__restrict__ tkey,
                 const uint32_t *__restrict__ tcnt, const uint32_t *__restrict__ start,
-                const uint32_t *__restrict__ bpidx, uint32_t TX, uint64_t cap_bp,
-                BinPair *__restrict__ out, uint32_t *err) {
+                const uint32_t *__restrict__ bpidx, uint32_t TX, uint64_t cap_bp, uint64_t cap_entries,
+                BinPair *__restrict__ out) {
+    drop_overgrown(ctr, cap_bp, cap_entries);
     const uint32_t ns = ctr->n_jslots;
     for (uint32_t h = blockIdx.x * blockDim.x + threadIdx.x; h < ns; h += gridDim.x * blockDim.x) {
         uint32_t pos = start[h];
@@ -344,7 +345,7 @@ k_ljoin_bp_fill(LevJoinGeom g, const Counters *__restrict__ ctr, const unsigned 
             const uint32_t m = tcnt[(size_t)h * g.nc + c], first = pos;
             pos += m;
             if (c == 0 ? m < 2 : m == 0) continue;
-            if (at >= cap_bp) { atomicOr(err, kErrBinPairOverflow); ++at; continue; }
+            if (at >= cap_bp) { ++at; continue; }   // flagged above
             BinPair P;
             P.a_start = first; P.a_n = m; P.b_start = s0; P.b_n = c0;
             P.ncx = (m + TX - 1) / TX;
@@ -421,8 +422,8 @@ void launch_lev_join_fill(const Plan &P, const Buffers &B, cudaStream_t s) {
 
 void launch_lev_join_binpairs(const Plan &P, const Buffers &B, cudaStream_t s) {
     k_ljoin_bp_fill<<<grid_wave(k_ljoin_bp_fill, B.jn_mask + 1, kThreads), kThreads, 0, s>>>(
-        lev_geom(P, B), B.ctr, B.jn_key, B.jn_cnt, B.jn_start, B.jn_bpidx, P.TX, P.cap_binpairs, B.bp,
-        &B.ctr->error);
+        lev_geom(P, B), B.ctr, B.jn_key, B.jn_cnt, B.jn_start, B.jn_bpidx, P.TX, P.cap_binpairs,
+        P.cap_entries, B.bp);
 }
 
 }  // namespace idb

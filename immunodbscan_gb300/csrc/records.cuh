@@ -140,6 +140,22 @@ __device__ __forceinline__ uint32_t seg_count(const int16_t *eps_tab, uint32_t N
     return e < 0 ? 1u : (uint32_t)e + 1u;
 }
 
+// A replayed plan whose data has more entries or bin pairs than it was captured
+// for: the fill kernels drop what does not fit, but bin pairs may still name
+// entries past the capacity, and the true count runs past the bin pairs.  Called
+// by each kernel that fills the bin pairs (none of them reads their count): no
+// bin pair is left for the predictor, the schedule and the distance kernels, and
+// the host is told.
+__device__ __forceinline__ void drop_overgrown(Counters *ctr, uint64_t cap_bp, uint64_t cap_entries) {
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    const uint32_t over = (ctr->n_binpairs > cap_bp ? kErrBinPairOverflow : 0u) |
+                          (ctr->n_entries > cap_entries ? kErrEntryOverflow : 0u);
+    if (over) {
+        atomicOr(&ctr->error, over);
+        ctr->n_binpairs = 0;
+    }
+}
+
 // Slots of the join table in use: about 1.5 slots per possible key (join_smax
 // per unique), a power of two, at most the allocation.  The allocation is sized
 // for every row being unique; the uniques are counted on the device, so the
