@@ -269,8 +269,9 @@ idb_status validate(const idb_input *in, const idb_params *prm, const idb_output
 }
 
 // Small host tables of a call (repertoire offsets, gene lists; eps and codes)
-// gathered for one copy to the device.  The copy is from pageable memory: the
-// bytes are staged when the call returns, so no wait is needed.
+// gathered for one copy to the device.  The copy is from pageable memory and may
+// read it after the call returned (the runtime stages such memory only where the
+// device cannot read it), so a pack lives in its call's Pipeline.
 struct HostPack {
     std::vector<char> bytes;
     size_t add(const void *p, size_t n) {
@@ -344,14 +345,28 @@ struct Pipeline {
     // that a replay copies them to the host while the rest of the path runs
     bool early_out = false;
     bool copies_issued = false;
+    HostPack tables, plan_tables;   // uploaded from here
+    bool tables_in_flight = false;  // ... and not waited for since
     int tile_rx = 0, tile_ty = 0;   // the unit shape the caller asked for (0: none)
     bool allow_join = true;   // the segment join finds neighbours, not all admissible pairs
+    idb_status upload(HostPack &pack, BufId id) {
+        tables_in_flight = true;
+        return pack.upload(c, id);
+    }
     // every return path (errors included) leaves no copy from the caller's host
-    // buffers in flight
+    // buffers or from the tables in flight
     ~Pipeline() {
         if (copies_issued && c) cudaStreamSynchronize(c->copy_stream);
+        if (tables_in_flight && c) cudaStreamSynchronize(c->stream);
     }
 };
+
+idb_status read_counters(Pipeline &pl) {
+    CU(cudaMemcpyAsync(pl.c->h_ctr, pl.B.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, pl.c->stream));
+    CU(cudaStreamSynchronize(pl.c->stream));
+    pl.tables_in_flight = false;
+    return IDB_OK;
+}
 
 // phase durations from the device time stamps (ms)
 void phase_times(const Counters &h, idb_stats *st) {
@@ -480,7 +495,7 @@ idb_status stage_inputs_and_survey(Pipeline &pl, const idb_input *in, bool host_
         roff[0] = 0;
         roff[1] = P.N;
     }
-    HostPack pack;
+    HostPack &pack = pl.tables;
     const size_t rep_at = pack.add(roff.data(), sizeof(uint32_t) * (P.R + 1));
     // gene lists
     P.Gv = P.no_v ? 1 : in->n_v_genes;
@@ -488,7 +503,7 @@ idb_status stage_inputs_and_survey(Pipeline &pl, const idb_input *in, bool host_
     GenePlace gv{}, gj{};
     if (!P.no_v) gv = pack_genes(pack, in->v_genes, in->v_gene_offsets, P.Gv, &P.gene_bytes_v, &P.vmatch);
     if (!P.no_j) gj = pack_genes(pack, in->j_genes, in->j_gene_offsets, P.Gj, &P.gene_bytes_j, &P.jmatch);
-    TRY(pack.upload(c, bTables));
+    TRY(pl.upload(pack, bTables));
     const uint8_t *tp = ptr<uint8_t>(c, bTables);
     B.rep_off = reinterpret_cast<const uint32_t *>(tp + rep_at);
     auto column = [&](const GenePlace &at, const uint8_t **names, const int32_t **off, const GeneEntry **tab) {
@@ -505,9 +520,7 @@ idb_status stage_inputs_and_survey(Pipeline &pl, const idb_input *in, bool host_
     B.timing = pl.timing;
     launch_survey(P, B, s);
     TRY(check_launch());
-    CU(cudaMemcpyAsync(c->h_ctr, B.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s));
-    CU(cudaStreamSynchronize(s));
-    return IDB_OK;
+    return read_counters(pl);
 }
 
 // Work-unit shape: rx x-entries per lane (the kernels are compiled for
@@ -664,10 +677,10 @@ idb_status alloc_fixed(Pipeline &pl) {
     Plan &P = pl.P;
     Buffers &B = pl.B;
     const size_t N = P.N, N1 = N + 1;
-    HostPack pack;
+    HostPack &pack = pl.plan_tables;
     const size_t eps_at = pack.add(pl.eps_host.data(), sizeof(int16_t) * pl.eps_host.size());
     const size_t code_at = pack.add(P.codemap, 256);
-    TRY(pack.upload(c, bPlanTables));
+    TRY(pl.upload(pack, bPlanTables));
     B.eps_tab = reinterpret_cast<const int16_t *>(ptr<uint8_t>(c, bPlanTables) + eps_at);
     B.codemap = ptr<uint8_t>(c, bPlanTables) + code_at;
     TRY(ensure(c, bVBits, sizeof(uint64_t) * N * P.VW));
@@ -790,12 +803,6 @@ idb_status alloc_edges(Pipeline &pl, uint64_t cap) {
     if (pl.P.edge_budget) held = std::min<uint64_t>(held, pl.P.edge_budget / sizeof(uint2));
     pl.P.cap_edges = std::max(cap, held);
     pl.B.edges = ptr<uint2>(c, bEdges);
-    return IDB_OK;
-}
-
-idb_status read_counters(Pipeline &pl) {
-    CU(cudaMemcpyAsync(pl.c->h_ctr, pl.B.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, pl.c->stream));
-    CU(cudaStreamSynchronize(pl.c->stream));
     return IDB_OK;
 }
 
@@ -1624,10 +1631,10 @@ idb_status idb_diag_gene_bits(idb_context *c, const char *calls, const int64_t *
     if (nbytes) CU(cudaMemcpyAsync(c->buf[bV].p, calls, nbytes, cudaMemcpyHostToDevice, c->stream));
     CU(cudaMemcpyAsync(c->buf[bVOff].p, offsets, sizeof(int64_t) * ((size_t)n_rows + 1),
                        cudaMemcpyHostToDevice, c->stream));
-    HostPack pack;
+    HostPack &pack = pl.tables;
     ++c->stage_epoch;   // a captured graph's gene tables are replaced
     const GenePlace at = pack_genes(pack, genes, gene_offsets, n_genes, &P.gene_bytes_v, &P.vmatch);
-    TRY(pack.upload(c, bTables));
+    TRY(pl.upload(pack, bTables));
     B.vcall = ptr<uint8_t>(c, bV); B.v_off = ptr<int64_t>(c, bVOff);
     B.vgenes = ptr<uint8_t>(c, bTables) + at.names;
     B.vg_off = reinterpret_cast<const int32_t *>(ptr<uint8_t>(c, bTables) + at.off);
@@ -1641,6 +1648,7 @@ idb_status idb_diag_gene_bits(idb_context *c, const char *calls, const int64_t *
     CU(cudaMemcpyAsync(words_out, B.vbits, sizeof(uint64_t) * n_rows * P.VW, cudaMemcpyDeviceToHost,
                        c->stream));
     CU(cudaStreamSynchronize(c->stream));
+    pl.tables_in_flight = false;
     return IDB_OK;
 }
 
@@ -1688,8 +1696,7 @@ idb_status idb_profile_binpairs(idb_context *c, const idb_input *in, const idb_p
         if (st != IDB_OK || !(c->h_ctr->error & kErrEdgeOverflow)) break;
         st = alloc_edges(pl, (uint64_t)c->h_ctr->edge_reserved + 64ull * kEdgeChunk * 1024);
         if (st != IDB_OK) break;
-        uint32_t clear = 0;
-        cudaMemcpyAsync(&B.ctr->error, &clear, 4, cudaMemcpyHostToDevice, s);
+        cudaMemsetAsync(&B.ctr->error, 0, 4, s);
     }
     const uint64_t n = std::min<uint64_t>(nbp, cap);
     if (st == IDB_OK) {
@@ -1910,8 +1917,7 @@ idb_status idb_autotune(idb_context *c, const idb_input *in, const idb_params *p
             TRY(read_counters(pl));
             if (c->h_ctr->error & kErrEdgeOverflow) {   // grow and repeat this shape
                 TRY(alloc_edges(pl, (uint64_t)c->h_ctr->edge_reserved + 64ull * kEdgeChunk * 1024));
-                uint32_t clear = 0;
-                CU(cudaMemcpyAsync(&B.ctr->error, &clear, 4, cudaMemcpyHostToDevice, s));
+                CU(cudaMemsetAsync(&B.ctr->error, 0, 4, s));
                 --rep;
                 ms_best = 1e30f;
             }

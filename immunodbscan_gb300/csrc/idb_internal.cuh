@@ -122,7 +122,6 @@ struct GlobalReader {
         return out;
     }
 };
-#endif
 
 // Bytes [32c, 32c + 32) of a string p[0..L) as 8 little-endian words, bytes
 // past L zero.  The aligned 4-byte words that hold those bytes are read with
@@ -146,7 +145,7 @@ __device__ __forceinline__ void load_chunk32(const uint8_t *p, uint32_t L, uint3
         w[k] = o;
     }
 }
-
+#endif
 
 // Device-resident counters of one clustering call (one struct, zeroed first).
 struct Counters {

@@ -1,0 +1,171 @@
+// test_api_host.cpp -- idb_api.cu on the CPU, with a stand-in for the CUDA runtime and
+// the launchers (fake_cuda.hpp): lifetimes of host tables and what the host does
+// on failed allocations and on the sizes the device reports.
+// usage: test_api_host <test name>
+#include "fake_cuda.hpp"
+
+#include "../../immunodbscan_gb300/csrc/idb_api.cu"
+
+#include <cstdio>
+
+#define CHECK(c)                                                                       \
+    do {                                                                               \
+        if (!(c)) { std::printf("%s:%d: %s (%s)\n", __FILE__, __LINE__, #c, g_err.c_str()); std::exit(1); } \
+    } while (0)
+
+// What the scripted device reports.
+struct Script {
+    uint32_t lmin = 10, lmax = 12;
+    uint32_t join_entries = 100, join_binpairs = 20, bucket_entries = 50, bucket_binpairs = 10;
+    unsigned long long join_pairs = 1000, bucket_pairs = 2000;
+    bool genes_fit = true;
+    std::vector<int16_t> eps_seen;   // the eps table as the device holds it
+} script;
+
+static void note(const char *what, const Plan &P, const Buffers &B) {
+    char b[128];
+    std::snprintf(b, sizeof b, "%s join=%d compact=%d timing=%d", what, (int)P.join, (int)P.compact, (int)B.timing);
+    fake::st().log.push_back(b);
+}
+static int logged(const std::string &s) {
+    int n = 0;
+    for (auto &x : fake::st().log) n += x.find(s) != std::string::npos;
+    return n;
+}
+
+namespace idb {
+void launch_survey(const Plan &P, const Buffers &B, cudaStream_t) {
+    Counters *c = B.ctr;
+    const uint32_t lo = script.lmin, hi = script.lmax;
+    fake::push([=] { c->lmax = hi; c->lmin_inv = ~lo; c->used['A' >> 5] |= 0x1Fu << ('A' & 31); });
+    (void)P;
+}
+void launch_check_plan(const Plan &, const Buffers &, cudaStream_t) {}
+void launch_const_strings(uint8_t *, int64_t *, uint32_t, cudaStream_t) {}
+void launch_call_init(const Plan &, const Buffers &, bool, cudaStream_t) {}
+void launch_gene_bits(const Plan &, const Buffers &, bool, uint32_t, cudaStream_t) {}
+void launch_dedupe_init(const Plan &P, const Buffers &B, cudaStream_t) {
+    const int16_t *e = B.eps_tab;
+    const size_t n = (size_t)P.NL * P.NL;
+    fake::push([=] { script.eps_seen.assign(e, e + n); });
+}
+void launch_dedupe_rows(const Plan &, const Buffers &, uint32_t, cudaStream_t) {}
+void launch_dedupe_final(const Plan &, const Buffers &, cudaStream_t) {}
+void launch_uniques_rows(const Plan &, const Buffers &, uint32_t, cudaStream_t) {}
+void launch_uniques_finish(const Plan &, const Buffers &, cudaStream_t) {}
+void launch_uniques(const Plan &P, const Buffers &B, cudaStream_t) {
+    Counters *c = B.ctr;
+    const uint32_t n = P.N;
+    fake::push([=] { c->n_uniques = n; });
+}
+void launch_join_init(const Plan &, const Buffers &, cudaStream_t) {}
+void launch_join_insert(const Plan &, const Buffers &, int, cudaStream_t) {}
+void launch_buckets(const Plan &P, const Buffers &B, cudaStream_t) {
+    note("buckets", P, B);
+    Counters *c = B.ctr;
+    const bool join = P.join, wide = P.wide, expect = P.compact;
+    fake::push([=] {
+        c->n_entries = join ? script.join_entries : script.bucket_entries;
+        if (join) { c->n_binpairs = script.join_binpairs; c->join_pairs = script.join_pairs; }
+        if (wide) c->vj_compact = script.genes_fit;
+        if (wide && expect && !script.genes_fit) c->error |= kErrAlphabet;
+    });
+}
+void launch_bucket_pairs(const Plan &, const Buffers &B, cudaStream_t) {
+    Counters *c = B.ctr;
+    fake::push([=] { c->bucket_pairs = script.bucket_pairs; });
+}
+void launch_fill(const Plan &P, const Buffers &B, cudaStream_t) { note("fill", P, B); }
+void launch_binpairs(const Plan &P, const Buffers &B, cudaStream_t) {
+    Counters *c = B.ctr;
+    if (!P.join) fake::push([=] { c->n_binpairs = script.bucket_binpairs; });
+}
+void launch_binpairs_fill(const Plan &P, const Buffers &B, cudaStream_t) { note("binpairs", P, B); }
+void launch_schedule(const Plan &, const Buffers &, cudaStream_t) {}
+void launch_distance(const Plan &P, const Buffers &B, int, cudaStream_t, uint32_t) { note("distance", P, B); }
+void launch_count_admissible(const Plan &, const Buffers &, cudaStream_t) {}
+void launch_graph(const Plan &, const Buffers &, bool, cudaStream_t, cudaEvent_t) {}
+void launch_streamed_sweeps(const Plan &, const Buffers &, cudaStream_t) {}
+void launch_streamed_labels(const Plan &, const Buffers &, bool, cudaStream_t) {}
+void launch_outputs(const Plan &, const Buffers &, cudaStream_t, uint32_t) {}
+uint32_t scan_part_needed(uint64_t n) { return (uint32_t)(n / 4096 + 2); }
+void launch_features(const Buffers &, uint32_t, float *, cudaStream_t) {}
+void launch_mlp_predict(const Buffers &, uint32_t, const void *, cudaStream_t) {}
+void launch_mlp_grad(const float *, const float *, uint32_t, const float *, float, float *, float *, cudaStream_t) {}
+void launch_adam(float *, const float *, float *, float *, float, int, cudaStream_t) {}
+void launch_to_bf16(const float *, void *, cudaStream_t) {}
+void launch_mlp_forward_rows(const float *, uint32_t, const void *, float *, cudaStream_t) {}
+}  // namespace idb
+
+// A call of `n` rows; the scripted device reads none of the columns.
+struct Call {
+    std::string seqs, v, j, vg, jg;
+    std::vector<int64_t> so, vo, jo, vgo, jgo;
+    std::vector<uint32_t> clone, copies;
+    std::vector<int32_t> core;
+    idb_input in{};
+    idb_params prm{};
+    idb_output out{};
+    idb_stats stats{};
+    Call(uint32_t n, uint32_t n_vg, uint32_t n_jg, bool hamming, int eps) {
+        so = {0}; vo = {0}; jo = {0}; vgo = {0}; jgo = {0};
+        for (uint32_t i = 0; i < n; ++i) {
+            seqs += "ABCDEABCDE"; so.push_back((int64_t)seqs.size());
+            v += "V1*01"; vo.push_back((int64_t)v.size());
+            j += "J1*01"; jo.push_back((int64_t)j.size());
+        }
+        for (uint32_t g = 0; g < n_vg; ++g) { vg += "V" + std::to_string(g) + "*"; vgo.push_back((int64_t)vg.size()); }
+        for (uint32_t g = 0; g < n_jg; ++g) { jg += "J" + std::to_string(g) + "*"; jgo.push_back((int64_t)jg.size()); }
+        clone.resize(n); copies.resize(n); core.resize(n);
+        in.n_rows = n;
+        in.seqs = seqs.data(); in.seq_offsets = so.data();
+        in.v_calls = v.data(); in.v_offsets = vo.data();
+        in.j_calls = j.data(); in.j_offsets = jo.data();
+        in.v_genes = vg.data(); in.v_gene_offsets = vgo.data(); in.n_v_genes = n_vg;
+        in.j_genes = jg.data(); in.j_gene_offsets = jgo.data(); in.n_j_genes = n_jg;
+        prm.threshold = NAN;
+        prm.abs_eps = eps;
+        prm.min_pts = 2;
+        prm.use_hamming = hamming;
+        out.clone_id = clone.data(); out.core = core.data(); out.copies = copies.data();
+        out.stats = &stats;
+    }
+};
+
+static idb_context *context() {
+    idb_context *c = nullptr;
+    CHECK(idb_context_create(0, &c) == IDB_OK);
+    return c;
+}
+
+// The tables a call uploads are read by copies that may run as late as the next
+// synchronisation: they have to live until then, on error returns too.
+static void test_tables_outlive_their_copies() {
+    idb_context *c = context();
+    Call a(40, 8, 3, false, 2);
+    CHECK(idb_cluster(c, &a.in, &a.prm, &a.out) == IDB_OK);
+    CHECK(script.eps_seen == std::vector<int16_t>(9, 2));
+    // a launch that fails right after the upload of each table
+    fake::st().fail_alloc = [](size_t) { fake::st().last = cudaErrorUnknown; return false; };
+    Call b(5000, 60, 20, false, 3);
+    CHECK(idb_cluster(c, &b.in, &b.prm, &b.out) == IDB_ERR_CUDA);
+    fake::st().fail_alloc = nullptr;
+    fake::st().last = cudaSuccess;
+    CHECK(idb_cluster(c, &b.in, &b.prm, &b.out) == IDB_OK);
+    CHECK(script.eps_seen == std::vector<int16_t>(9, 3));
+    std::vector<uint64_t> words(5000);
+    CHECK(idb_diag_gene_bits(c, b.v.data(), b.vo.data(), 5000, b.vg.data(), b.vgo.data(), 60, words.data()) == IDB_OK);
+    CHECK(idb_context_destroy(c) == IDB_OK);
+    fake::drain();
+}
+
+int main(int argc, char **argv) {
+    const std::map<std::string, void (*)()> tests = {
+        {"tables_outlive_their_copies", test_tables_outlive_their_copies},
+    };
+    const auto it = tests.find(argc > 1 ? argv[1] : "");
+    if (it == tests.end()) { std::printf("unknown test\n"); return 2; }
+    it->second();
+    std::printf("ok\n");
+    return 0;
+}
