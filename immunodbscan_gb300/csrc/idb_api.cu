@@ -95,6 +95,7 @@ struct idb_context {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     idb_output out_dev{};
+    int batch_rx = 0, batch_ty = 0;   // the unit shape the plan's caller asked for
     bool trees = false;
     uint32_t graph_kernels = 0;
     // learned schedule: MLP parameters (BF16 for inference)
@@ -809,7 +810,7 @@ idb_status alloc_edges(Pipeline &pl, uint64_t cap) {
 idb_status device_errors(const Counters &h) {
     if (h.error & kErrHashStall) return fail(IDB_ERR_DEVICE_STALL, "duplicate table probe gave up");
     if (h.error & kErrUnionStall) return fail(IDB_ERR_DEVICE_STALL, "union-find retry bound reached");
-    if (h.error & (kErrAlphabet | kErrLength))
+    if (h.error & (kErrAlphabet | kErrLength | kErrGenesInUse))
         return fail(IDB_ERR_REPLAN, "inputs no longer match the captured plan");
     if (h.error & (kErrEdgeOverflow | kErrUnitOverflow | kErrBinPairOverflow | kErrEntryOverflow))
         return fail(IDB_ERR_CAPACITY, "a plan capacity was exceeded (error bits 0x%x)", h.error);
@@ -1319,6 +1320,88 @@ idb_status cluster_impl(idb_context *c, const idb_input *in, const idb_params *p
     return IDB_OK;
 }
 
+void batch_plan_drop(idb_context *c) {
+    if (c->exec) cudaGraphExecDestroy(c->exec);
+    if (c->graph) cudaGraphDestroy(c->graph);
+    c->exec = nullptr;
+    c->graph = nullptr;
+    c->planned = false;
+}
+
+// After a discovery run: capacities with headroom (the buffers keep their addresses
+// from here on), then the capture of the complete launch sequence.
+idb_status capture_batch_plan(Pipeline &pl, const idb_output &o) {
+    idb_context *c = pl.c;
+    TRY(read_counters(pl));
+    TRY(device_errors(*c->h_ctr));
+    const Counters h = *c->h_ctr;
+    TRY(alloc_entries(pl, (uint64_t)h.n_entries + h.n_entries / 16 + 1024));
+    TRY(alloc_binpairs(pl, (uint64_t)h.n_binpairs + h.n_binpairs / 16 + 1024));
+    if (!pl.P.streamed)
+        TRY(alloc_edges(pl, (uint64_t)h.edge_reserved + h.edge_reserved / 8 + 64ull * kEdgeChunk * 1024));
+    cudaStream_t s = c->stream;
+    CU(cudaStreamSynchronize(s));
+    CU(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    cudaMemsetAsync(pl.B.ctr, 0, sizeof(Counters), s);
+    pl.timing = true;   // time-stamp kernels between the phases
+    pl.B.timing = pl.timing;
+    launch_survey(pl.P, pl.B, s);
+    idb_status st = run_phases(pl, false);
+    cudaGraph_t g = nullptr;
+    cudaError_t ce = cudaStreamEndCapture(s, &g);
+    if (st != IDB_OK) {
+        if (g) cudaGraphDestroy(g);
+        return st;
+    }
+    if (ce != cudaSuccess) return fail(IDB_ERR_CUDA, "graph capture: %s", cudaGetErrorString(ce));
+    c->graph = g;
+    CU(cudaGraphInstantiate(&c->exec, g, 0));
+    CU(cudaGraphUpload(c->exec, s));   // device-side setup now, not in the first replay
+    CU(cudaStreamSynchronize(s));
+    {
+        size_t nn = 0;
+        CU(cudaGraphGetNodes(g, nullptr, &nn));
+        std::vector<cudaGraphNode_t> nodes(nn);
+        CU(cudaGraphGetNodes(g, nodes.data(), &nn));
+        uint32_t k = 0;
+        for (auto nd : nodes) {
+            cudaGraphNodeType t;
+            CU(cudaGraphNodeGetType(nd, &t));
+            k += t == cudaGraphNodeTypeKernel;
+        }
+        c->graph_kernels = k;
+    }
+    c->plan = pl.P;
+    c->bufs = pl.B;
+    c->out_dev = o;
+    c->batch_rx = pl.tile_rx;
+    c->batch_ty = pl.tile_ty;
+    c->planned = true;
+    c->batch_generation = c->generation;
+    c->batch_epoch = c->stage_epoch;
+    return IDB_OK;
+}
+
+// A plan over a wide gene list whose side records held the genes in use, on data
+// that uses more of them: discovery and capture again with the full bitsets, over
+// the staged tables and the same columns and outputs.
+idb_status batch_replan_genes(idb_context *c) {
+    Pipeline pl;
+    pl.c = c;
+    pl.P = c->plan;
+    pl.B = c->bufs;
+    pl.B.timing = false;
+    pl.tile_rx = c->batch_rx;
+    pl.tile_ty = c->batch_ty;
+    pl.P.compact = false;
+    const idb_output o = c->out_dev;
+    batch_plan_drop(c);
+    CU(cudaMemsetAsync(pl.B.ctr, 0, sizeof(Counters), c->stream));
+    launch_survey(pl.P, pl.B, c->stream);
+    TRY(run_phases(pl, true));
+    return capture_batch_plan(pl, o);
+}
+
 thread_local idb_context *t_default_ctx = nullptr;
 
 idb_status get_ctx(idb_context **pc) {
@@ -1485,10 +1568,8 @@ idb_status idb_batch_plan(idb_context *c, const idb_input *in, const idb_params 
     TRY(validate(in, prm, out));
     if (in->n_rows == 0) return fail(IDB_ERR_INVALID_ARG, "empty input");
     CU(cudaSetDevice(c->device));
-    if (c->exec) { cudaGraphExecDestroy(c->exec); c->exec = nullptr; }
-    if (c->graph) { cudaGraphDestroy(c->graph); c->graph = nullptr; }
-    c->planned = false;
-    // 1. discovery run (eager) to learn the sizes
+    batch_plan_drop(c);
+    // a discovery run (eager) learns the sizes
     idb_output o = *out;
     o.stats = nullptr;
     o.tree_depth_hist = nullptr;
@@ -1504,54 +1585,7 @@ idb_status idb_batch_plan(idb_context *c, const idb_input *in, const idb_params 
     pl.B.copies = o.copies;
     pl.B.uniques = o.uniques;
     TRY(run_phases(pl, true));
-    TRY(read_counters(pl));
-    TRY(device_errors(*c->h_ctr));
-    // 2. capacities with headroom; the buffers keep their addresses from here on
-    const Counters h = *c->h_ctr;
-    TRY(alloc_entries(pl, (uint64_t)h.n_entries + h.n_entries / 16 + 1024));
-    TRY(alloc_binpairs(pl, (uint64_t)h.n_binpairs + h.n_binpairs / 16 + 1024));
-    if (!pl.P.streamed)
-        TRY(alloc_edges(pl, (uint64_t)h.edge_reserved + h.edge_reserved / 8 + 64ull * kEdgeChunk * 1024));
-    // 3. capture the complete launch sequence
-    cudaStream_t s = c->stream;
-    CU(cudaStreamSynchronize(s));
-    CU(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    cudaMemsetAsync(pl.B.ctr, 0, sizeof(Counters), s);
-    pl.timing = true;   // time-stamp kernels between the phases
-    pl.B.timing = pl.timing;
-    launch_survey(pl.P, pl.B, s);
-    idb_status st = run_phases(pl, false);
-    cudaGraph_t g = nullptr;
-    cudaError_t ce = cudaStreamEndCapture(s, &g);
-    if (st != IDB_OK) {
-        if (g) cudaGraphDestroy(g);
-        return st;
-    }
-    if (ce != cudaSuccess) return fail(IDB_ERR_CUDA, "graph capture: %s", cudaGetErrorString(ce));
-    c->graph = g;
-    CU(cudaGraphInstantiate(&c->exec, g, 0));
-    CU(cudaGraphUpload(c->exec, s));   // device-side setup now, not in the first replay
-    CU(cudaStreamSynchronize(s));
-    {
-        size_t nn = 0;
-        CU(cudaGraphGetNodes(g, nullptr, &nn));
-        std::vector<cudaGraphNode_t> nodes(nn);
-        CU(cudaGraphGetNodes(g, nodes.data(), &nn));
-        uint32_t k = 0;
-        for (auto nd : nodes) {
-            cudaGraphNodeType t;
-            CU(cudaGraphNodeGetType(nd, &t));
-            k += t == cudaGraphNodeTypeKernel;
-        }
-        c->graph_kernels = k;
-    }
-    c->plan = pl.P;
-    c->bufs = pl.B;
-    c->out_dev = o;
-    c->planned = true;
-    c->batch_generation = c->generation;
-    c->batch_epoch = c->stage_epoch;
-    return IDB_OK;
+    return capture_batch_plan(pl, o);
 }
 
 idb_status idb_batch_run(idb_context *c, idb_stats *stats) {
@@ -1566,6 +1600,11 @@ idb_status idb_batch_run(idb_context *c, idb_stats *stats) {
     CU(cudaEventRecord(c->ev[1], s));
     CU(cudaMemcpyAsync(c->h_ctr, c->bufs.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
+    // (what else the renumbered genes led to in that replay says nothing)
+    if ((c->h_ctr->error & kErrGenesInUse) && !(c->h_ctr->error & (kErrAlphabet | kErrLength))) {
+        TRY(batch_replan_genes(c));
+        return idb_batch_run(c, stats);   // the new plan does not expect them to fit
+    }
     TRY(device_errors(*c->h_ctr));
     if (stats) {
         const Counters &h = *c->h_ctr;

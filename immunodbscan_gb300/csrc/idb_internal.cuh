@@ -65,6 +65,7 @@ enum : uint32_t {
     kErrLength = 32u,         // a length outside the plan's range
     kErrBinPairOverflow = 64u,
     kErrEntryOverflow = 128u,
+    kErrGenesInUse = 256u,    // more genes in use than a captured plan's side records hold
 };
 
 // Gene-name lookup table (built on the host per call): open addressing on the

@@ -79,7 +79,7 @@ __global__ void k_gene_used(Counters *ctr, const uint32_t *__restrict__ urow, co
         nj += popc64(atomicOr(&ctr->used_j[w], 0ull));
     }
     ctr->vj_compact = nv <= 64 && nj <= 30;
-    if (expected && !(nv <= 64 && nj <= 30)) atomicOr(&ctr->error, kErrAlphabet);   // outside the plan
+    if (expected && !(nv <= 64 && nj <= 30)) atomicOr(&ctr->error, kErrGenesInUse);
     ctr->used_done = 0;
 }
 

@@ -68,7 +68,7 @@ void launch_buckets(const Plan &P, const Buffers &B, cudaStream_t) {
         c->n_entries = join ? script.join_entries : script.bucket_entries;
         if (join) { c->n_binpairs = script.join_binpairs; c->join_pairs = script.join_pairs; }
         if (wide) c->vj_compact = script.genes_fit;
-        if (wide && expect && !script.genes_fit) c->error |= kErrAlphabet;
+        if (wide && expect && !script.genes_fit) c->error |= kErrGenesInUse;
     });
 }
 void launch_bucket_pairs(const Plan &, const Buffers &B, cudaStream_t) {
@@ -159,9 +159,37 @@ static void test_tables_outlive_their_copies() {
     fake::drain();
 }
 
+// A batch plan over a wide gene list, made while the genes in use fitted the side
+// records: a run on data that uses more of them plans anew by itself (the
+// join for Hamming needs them to fit) and a later run replays that plan.
+static void test_batch_run_with_more_genes_in_use() {
+    for (const bool hamming : {true, false}) {
+        idb_context *c = context();
+        Call a(200, 100, 3, hamming, 1);
+        a.out.stats = nullptr;
+        script = Script();
+        CHECK(idb_batch_plan(c, &a.in, &a.prm, &a.out) == IDB_OK);
+        fake::st().log.clear();
+        CHECK(idb_batch_run(c, &a.stats) == IDB_OK);
+        CHECK(a.stats.candidates == 1 && c->plan.compact && fake::st().log.empty());
+        script.genes_fit = false;
+        CHECK(idb_batch_run(c, &a.stats) == IDB_OK);
+        CHECK(!c->plan.compact && a.stats.candidates == (hamming ? 0u : 1u));
+        CHECK(a.stats.n_entries == (hamming ? script.bucket_entries : script.join_entries));
+        CHECK(logged(std::string("distance join=") + (hamming ? "0" : "1") + " compact=0") == 2);   // and captured
+        fake::st().log.clear();
+        CHECK(idb_batch_run(c, &a.stats) == IDB_OK);
+        script.genes_fit = true;
+        CHECK(idb_batch_run(c, &a.stats) == IDB_OK);
+        CHECK(fake::st().log.empty());
+        CHECK(idb_context_destroy(c) == IDB_OK);
+    }
+}
+
 int main(int argc, char **argv) {
     const std::map<std::string, void (*)()> tests = {
         {"tables_outlive_their_copies", test_tables_outlive_their_copies},
+        {"batch_run_with_more_genes_in_use", test_batch_run_with_more_genes_in_use},
     };
     const auto it = tests.find(argc > 1 ? argv[1] : "");
     if (it == tests.end()) { std::printf("unknown test\n"); return 2; }
