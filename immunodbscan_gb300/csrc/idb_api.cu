@@ -151,6 +151,15 @@ idb_status ensure(idb_context *c, BufId id, size_t bytes, bool exact = false) {
     return IDB_OK;
 }
 
+idb_status release(idb_context *c, BufId id) {
+    DevBuf &b = c->buf[id];
+    if (!b.p) return IDB_OK;
+    CU(cudaFree(b.p));
+    b = DevBuf();
+    ++c->generation;
+    return IDB_OK;
+}
+
 template <typename T>
 T *ptr(idb_context *c, BufId id) { return reinterpret_cast<T *>(c->buf[id].p); }
 
@@ -669,6 +678,22 @@ idb_status alloc_call_scratch(idb_context *c, Buffers &B, uint64_t N) {
         cs.ntodo = B.ctr->call_todo + k * kMaxRowChunks;
     }
     return IDB_OK;
+}
+
+// Run `call` (its arguments: may it take a join, and did its plan); if memory runs
+// out under a join, once more with the buckets.  A join needs more of it: its
+// table, its group places and up to 26 entries a unique (edit distances up to 3)
+// against one per V and J gene of a unique's calls.
+template <typename F>
+idb_status buckets_if_join_does_not_fit(idb_context *c, F call) {
+    bool joined = false;
+    const idb_status st = call(true, &joined);
+    if (st != IDB_ERR_OUT_OF_MEMORY || !joined) return st;
+    cudaGetLastError();
+    for (const BufId id : {bJnTab, bJnPos, bJnISlot, bJnStart, bJnCur, bJnBpIdx, bEntUid, bEntRec, bEntMeta,
+                           bEntCopies, bBp, bBpSorted, bBpUnits, bBpSmall, bPred})
+        TRY(release(c, id));
+    return call(false, &joined);
 }
 
 // Workspace for everything sized by N and the plan.
@@ -1235,34 +1260,16 @@ idb_status host_plan_run(idb_context *c, const idb_input *in, idb_output *out) {
     return IDB_OK;
 }
 
-idb_status cluster_impl(idb_context *c, const idb_input *in, const idb_params *prm,
-                        idb_output *out, bool host_io) {
-    TRY(validate(in, prm, out));
-    CU(cudaSetDevice(c->device));
-    cudaGetLastError();   // a stale error of an unrelated call must not fail this one
+idb_status cluster_eager(idb_context *c, const idb_input *in, const idb_params *prm, idb_output *out,
+                         bool host_io, bool cacheable, bool seen, bool allow_join, bool *joined) {
     Pipeline pl;
     pl.c = c;
+    pl.allow_join = allow_join;
     pl.trees = prm->eval_trees != 0 && out->tree_depth_hist != nullptr;
     pl.timing = out->stats != nullptr;
-    if (in->n_rows == 0) {
-        if (out->n_uniques) *out->n_uniques = 0;
-        if (out->stats) std::memset(out->stats, 0, sizeof *out->stats);
-        return IDB_OK;
-    }
-    // the plan cache serves host inputs without the tree-depth statistics
-    const bool cacheable = host_io && !pl.trees && (prm->schedule != 1 || c->has_model);
-    bool seen = false;
-    if (cacheable && c->hp.valid && host_plan_key_matches(c, in, prm, out)) {
-        seen = true;
-        if (c->hp.exec && c->hp.generation == c->generation && c->hp.epoch == c->stage_epoch &&
-            c->hp.model == c->has_model) {
-            const idb_status st = host_plan_run(c, in, out);
-            if (st != IDB_ERR_REPLAN && st != IDB_ERR_CAPACITY) return st;
-            host_plan_drop_graph(c);   // the data outgrew the plan: eager, then capture anew
-        }
-    }
     TRY(stage_inputs_and_survey(pl, in, host_io, prm->row_chunks));
     TRY(derive_plan(pl, prm));
+    *joined = pl.P.join;
     TRY(alloc_fixed(pl));
     Buffers &B = pl.B;
     const size_t N = pl.P.N;
@@ -1318,6 +1325,34 @@ idb_status cluster_impl(idb_context *c, const idb_input *in, const idb_params *p
         g_err.clear();
     }
     return IDB_OK;
+}
+
+idb_status cluster_impl(idb_context *c, const idb_input *in, const idb_params *prm,
+                        idb_output *out, bool host_io) {
+    TRY(validate(in, prm, out));
+    CU(cudaSetDevice(c->device));
+    cudaGetLastError();   // a stale error of an unrelated call must not fail this one
+    if (in->n_rows == 0) {
+        if (out->n_uniques) *out->n_uniques = 0;
+        if (out->stats) std::memset(out->stats, 0, sizeof *out->stats);
+        return IDB_OK;
+    }
+    // the plan cache serves host inputs without the tree-depth statistics
+    const bool trees = prm->eval_trees != 0 && out->tree_depth_hist != nullptr;
+    const bool cacheable = host_io && !trees && (prm->schedule != 1 || c->has_model);
+    bool seen = false;
+    if (cacheable && c->hp.valid && host_plan_key_matches(c, in, prm, out)) {
+        seen = true;
+        if (c->hp.exec && c->hp.generation == c->generation && c->hp.epoch == c->stage_epoch &&
+            c->hp.model == c->has_model) {
+            const idb_status st = host_plan_run(c, in, out);
+            if (st != IDB_ERR_REPLAN && st != IDB_ERR_CAPACITY) return st;
+            host_plan_drop_graph(c);   // the data outgrew the plan: eager, then capture anew
+        }
+    }
+    return buckets_if_join_does_not_fit(c, [&](bool allow_join, bool *joined) {
+        return cluster_eager(c, in, prm, out, host_io, cacheable, seen, allow_join, joined);
+    });
 }
 
 void batch_plan_drop(idb_context *c) {
@@ -1400,6 +1435,174 @@ idb_status batch_replan_genes(idb_context *c) {
     launch_survey(pl.P, pl.B, c->stream);
     TRY(run_phases(pl, true));
     return capture_batch_plan(pl, o);
+}
+
+idb_status profile_binpairs(idb_context *c, const idb_input *in, const idb_params &p0, float *features,
+                            float *log2_cycles, uint64_t cap, uint64_t *n_out, bool allow_join, bool *joined) {
+    Pipeline pl;
+    pl.c = c;
+    pl.allow_join = allow_join;
+    TRY(stage_inputs_and_survey(pl, in, true));
+    TRY(derive_plan(pl, &p0));
+    *joined = pl.P.join;
+    TRY(alloc_fixed(pl));
+    Plan &P = pl.P;
+    Buffers &B = pl.B;
+    cudaStream_t s = c->stream;
+    TRY(run_phases(pl, true, true));   // up to the static schedule
+    TRY(read_counters(pl));
+    const uint32_t nbp = c->h_ctr->n_binpairs;
+    if (P.cap_edges == 0) TRY(alloc_edges(pl, std::max<uint64_t>(4ull * P.N, 1ull << 16)));
+    unsigned long long *cyc = nullptr;
+    float *feat = nullptr;
+    CU(cudaMalloc(&cyc, sizeof(unsigned long long) * (nbp + 1)));
+    cudaError_t e = cudaMalloc(&feat, sizeof(float) * kMlpIn * (nbp + 1));
+    if (e != cudaSuccess) { cudaFree(cyc); return fail(IDB_ERR_OUT_OF_MEMORY, "profile buffers"); }
+    idb_status st = IDB_OK;
+    for (int attempt = 0; attempt < 3; ++attempt) {
+        cudaMemsetAsync(cyc, 0, sizeof(unsigned long long) * (nbp + 1), s);
+        cudaMemsetAsync(&B.ctr->unit_cursor, 0, 4, s);
+        cudaMemsetAsync(&B.ctr->edge_reserved, 0, 4, s);
+        B.bp_cycles = cyc;
+        launch_distance(P, B, 0, s);
+        B.bp_cycles = nullptr;
+        st = read_counters(pl);
+        if (st != IDB_OK || !(c->h_ctr->error & kErrEdgeOverflow)) break;
+        st = alloc_edges(pl, (uint64_t)c->h_ctr->edge_reserved + 64ull * kEdgeChunk * 1024);
+        if (st != IDB_OK) break;
+        cudaMemsetAsync(&B.ctr->error, 0, 4, s);
+    }
+    const uint64_t n = std::min<uint64_t>(nbp, cap);
+    if (st == IDB_OK) {
+        launch_features(B, nbp, feat, s);
+        std::vector<unsigned long long> hc(nbp);
+        cudaMemcpyAsync(hc.data(), cyc, sizeof(unsigned long long) * nbp, cudaMemcpyDeviceToHost, s);
+        cudaMemcpyAsync(features, feat, sizeof(float) * kMlpIn * n, cudaMemcpyDeviceToHost, s);
+        if (cudaStreamSynchronize(s) != cudaSuccess) st = fail(IDB_ERR_CUDA, "profile copy failed");
+        for (uint64_t i = 0; i < n; ++i) log2_cycles[i] = std::log2(1.0 + (double)hc[i]);
+        *n_out = n;
+    }
+    cudaFree(cyc);
+    cudaFree(feat);
+    return st;
+}
+
+idb_status autotune(idb_context *c, const idb_input *in, const idb_params *prm, idb_tuning *best,
+                    bool allow_join, bool *joined) {
+    std::memset(best, 0, sizeof *best);
+    Pipeline pl;
+    pl.c = c;
+    pl.allow_join = allow_join;
+    TRY(stage_inputs_and_survey(pl, in, true));
+    TRY(derive_plan(pl, prm));
+    *joined = pl.P.join;
+    TRY(alloc_fixed(pl));
+    Plan &P = pl.P;
+    Buffers &B = pl.B;
+    cudaStream_t s = c->stream;
+    // front and buckets once (independent of the unit shape)
+    TRY(launch_front(pl, s));
+    launch_buckets(P, B, s);
+    TRY(choose_candidates(pl));
+    launch_fill(P, B, s);
+    TRY(check_launch());
+    // candidate shapes
+    std::vector<std::pair<int, int>> cand;
+    if (!P.fast) {
+        cand = {{1, 64}, {1, 256}, {1, 1024}};
+    } else if (P.hamming) {
+        const int rxs[3] = {2, 4, 8};
+        for (int rx : rxs) {
+            if (rx != 4 && P.W != 1) continue;
+            if (rx == 2 && !P.join) continue;
+            for (int ty : {128, 256, 512, 1024})
+                if (ty >= 32 * rx) cand.push_back({rx, ty});
+        }
+    } else {
+        for (int rx : {1, 2}) {
+            if (rx == 2 && P.W != 1) continue;
+            for (int ty : {64, 128, 256, 512, 1024}) cand.push_back({rx, ty});
+        }
+    }
+    if (cand.size() > 16) cand.resize(16);
+    if (P.cap_edges == 0) TRY(alloc_edges(pl, std::max<uint64_t>(4ull * P.N, 1ull << 16)));
+    // one shape and schedule order: bin pairs, the order, then the distance
+    // kernel three times (best of the three)
+    auto time_shape = [&](Plan Q, float *ms_out) -> idb_status {
+        launch_binpairs(Q, B, s);
+        TRY(read_counters(pl));
+        pl.P = Q;
+        TRY(alloc_binpairs(pl, c->h_ctr->n_binpairs));
+        Q.cap_binpairs = pl.P.cap_binpairs;
+        launch_binpairs_fill(Q, B, s);
+        if (Q.schedule == 1) launch_mlp_predict(B, (uint32_t)Q.cap_binpairs, c->mlp_bf16, s);
+        launch_schedule(Q, B, s);
+        float ms_best = 1e30f;
+        for (int rep = 0; rep < 3; ++rep) {
+            CU(cudaMemsetAsync(&B.ctr->unit_cursor, 0, 4, s));
+            CU(cudaMemsetAsync(&B.ctr->edge_reserved, 0, 4, s));
+            CU(cudaMemsetAsync(&B.ctr->n_edges, 0, 4, s));
+            CU(cudaMemsetAsync(&B.ctr->pairs_evaluated, 0, 8, s));
+            CU(cudaEventRecord(c->ev[0], s));
+            Q.cap_edges = pl.P.cap_edges;
+            launch_distance(Q, B, 0, s);
+            CU(cudaEventRecord(c->ev[1], s));
+            TRY(check_launch());
+            CU(cudaEventSynchronize(c->ev[1]));
+            float ms = 0;
+            CU(cudaEventElapsedTime(&ms, c->ev[0], c->ev[1]));
+            ms_best = std::min(ms_best, ms);
+            TRY(read_counters(pl));
+            if (c->h_ctr->error & kErrEdgeOverflow) {   // grow and repeat this shape
+                TRY(alloc_edges(pl, (uint64_t)c->h_ctr->edge_reserved + 64ull * kEdgeChunk * 1024));
+                CU(cudaMemsetAsync(&B.ctr->error, 0, 4, s));
+                --rep;
+                ms_best = 1e30f;
+            }
+        }
+        *ms_out = ms_best;
+        return IDB_OK;
+    };
+    double best_ms = 1e30;
+    Plan best_plan = P;
+    for (auto &cd : cand) {
+        Plan Q = P;
+        Q.schedule = 0;
+        if (P.fast) {
+            Q.RX = cd.first;
+            Q.TX = 32 * Q.RX;
+            Q.TY = cd.second;
+        } else {
+            Q.TY = cd.second;
+        }
+        float ms_best = 0;
+        TRY(time_shape(Q, &ms_best));
+        const int k = best->n_tried++;
+        best->tried_rx[k] = Q.RX;
+        best->tried_ty[k] = (int)Q.TY;
+        best->tried_ms[k] = ms_best;
+        if (ms_best < best_ms) {
+            best_ms = ms_best;
+            best_plan = Q;
+            best->tile_rx = Q.RX;
+            best->tile_ty = (int)Q.TY;
+            best->ms_distance = ms_best;
+        }
+    }
+    // the schedule order for the fastest shape: static heavy-first, or the
+    // learned cost when the context holds a model
+    best->schedule = 0;
+    best->schedule_ms[0] = best_ms;
+    if (c->has_model) {
+        Plan Q = best_plan;
+        Q.schedule = 1;
+        float ms_learned = 0;
+        TRY(time_shape(Q, &ms_learned));
+        best->schedule_ms[1] = ms_learned;
+        if (ms_learned < best_ms) best->schedule = 1;
+    }
+    TRY(device_errors(*c->h_ctr));
+    return IDB_OK;
 }
 
 thread_local idb_context *t_default_ctx = nullptr;
@@ -1574,18 +1777,22 @@ idb_status idb_batch_plan(idb_context *c, const idb_input *in, const idb_params 
     o.stats = nullptr;
     o.tree_depth_hist = nullptr;
     o.n_uniques = nullptr;
-    Pipeline pl;
-    pl.c = c;
-    pl.trees = false;
-    TRY(stage_inputs_and_survey(pl, in, false));
-    TRY(derive_plan(pl, prm));
-    TRY(alloc_fixed(pl));
-    pl.B.clone_id = o.clone_id;
-    pl.B.core = o.core;
-    pl.B.copies = o.copies;
-    pl.B.uniques = o.uniques;
-    TRY(run_phases(pl, true));
-    return capture_batch_plan(pl, o);
+    return buckets_if_join_does_not_fit(c, [&](bool allow_join, bool *joined) -> idb_status {
+        Pipeline pl;
+        pl.c = c;
+        pl.allow_join = allow_join;
+        pl.trees = false;
+        TRY(stage_inputs_and_survey(pl, in, false));
+        TRY(derive_plan(pl, prm));
+        *joined = pl.P.join;
+        TRY(alloc_fixed(pl));
+        pl.B.clone_id = o.clone_id;
+        pl.B.core = o.core;
+        pl.B.copies = o.copies;
+        pl.B.uniques = o.uniques;
+        TRY(run_phases(pl, true));
+        return capture_batch_plan(pl, o);
+    });
 }
 
 idb_status idb_batch_run(idb_context *c, idb_stats *stats) {
@@ -1706,50 +1913,9 @@ idb_status idb_profile_binpairs(idb_context *c, const idb_input *in, const idb_p
     cudaGetLastError();
     idb_params p0 = *prm;
     p0.schedule = 0;
-    Pipeline pl;
-    pl.c = c;
-    TRY(stage_inputs_and_survey(pl, in, true));
-    TRY(derive_plan(pl, &p0));
-    TRY(alloc_fixed(pl));
-    Plan &P = pl.P;
-    Buffers &B = pl.B;
-    cudaStream_t s = c->stream;
-    TRY(run_phases(pl, true, true));   // up to the static schedule
-    TRY(read_counters(pl));
-    const uint32_t nbp = c->h_ctr->n_binpairs;
-    if (P.cap_edges == 0) TRY(alloc_edges(pl, std::max<uint64_t>(4ull * P.N, 1ull << 16)));
-    unsigned long long *cyc = nullptr;
-    float *feat = nullptr;
-    CU(cudaMalloc(&cyc, sizeof(unsigned long long) * (nbp + 1)));
-    cudaError_t e = cudaMalloc(&feat, sizeof(float) * kMlpIn * (nbp + 1));
-    if (e != cudaSuccess) { cudaFree(cyc); return fail(IDB_ERR_OUT_OF_MEMORY, "profile buffers"); }
-    idb_status st = IDB_OK;
-    for (int attempt = 0; attempt < 3; ++attempt) {
-        cudaMemsetAsync(cyc, 0, sizeof(unsigned long long) * (nbp + 1), s);
-        cudaMemsetAsync(&B.ctr->unit_cursor, 0, 4, s);
-        cudaMemsetAsync(&B.ctr->edge_reserved, 0, 4, s);
-        B.bp_cycles = cyc;
-        launch_distance(P, B, 0, s);
-        B.bp_cycles = nullptr;
-        st = read_counters(pl);
-        if (st != IDB_OK || !(c->h_ctr->error & kErrEdgeOverflow)) break;
-        st = alloc_edges(pl, (uint64_t)c->h_ctr->edge_reserved + 64ull * kEdgeChunk * 1024);
-        if (st != IDB_OK) break;
-        cudaMemsetAsync(&B.ctr->error, 0, 4, s);
-    }
-    const uint64_t n = std::min<uint64_t>(nbp, cap);
-    if (st == IDB_OK) {
-        launch_features(B, nbp, feat, s);
-        std::vector<unsigned long long> hc(nbp);
-        cudaMemcpyAsync(hc.data(), cyc, sizeof(unsigned long long) * nbp, cudaMemcpyDeviceToHost, s);
-        cudaMemcpyAsync(features, feat, sizeof(float) * kMlpIn * n, cudaMemcpyDeviceToHost, s);
-        if (cudaStreamSynchronize(s) != cudaSuccess) st = fail(IDB_ERR_CUDA, "profile copy failed");
-        for (uint64_t i = 0; i < n; ++i) log2_cycles[i] = std::log2(1.0 + (double)hc[i]);
-        *n_out = n;
-    }
-    cudaFree(cyc);
-    cudaFree(feat);
-    return st;
+    return buckets_if_join_does_not_fit(c, [&](bool allow_join, bool *joined) {
+        return profile_binpairs(c, in, p0, features, log2_cycles, cap, n_out, allow_join, joined);
+    });
 }
 
 idb_status idb_mlp_train(idb_context *c, const float *features, const float *targets, uint64_t n,
@@ -1893,117 +2059,9 @@ idb_status idb_autotune(idb_context *c, const idb_input *in, const idb_params *p
     if (in->n_rows == 0) return IDB_OK;
     CU(cudaSetDevice(c->device));
     cudaGetLastError();
-    Pipeline pl;
-    pl.c = c;
-    TRY(stage_inputs_and_survey(pl, in, true));
-    TRY(derive_plan(pl, prm));
-    TRY(alloc_fixed(pl));
-    Plan &P = pl.P;
-    Buffers &B = pl.B;
-    cudaStream_t s = c->stream;
-    // front and buckets once (independent of the unit shape)
-    TRY(launch_front(pl, s));
-    launch_buckets(P, B, s);
-    TRY(choose_candidates(pl));
-    launch_fill(P, B, s);
-    TRY(check_launch());
-    // candidate shapes
-    std::vector<std::pair<int, int>> cand;
-    if (!P.fast) {
-        cand = {{1, 64}, {1, 256}, {1, 1024}};
-    } else if (P.hamming) {
-        const int rxs[3] = {2, 4, 8};
-        for (int rx : rxs) {
-            if (rx != 4 && P.W != 1) continue;
-            if (rx == 2 && !P.join) continue;
-            for (int ty : {128, 256, 512, 1024})
-                if (ty >= 32 * rx) cand.push_back({rx, ty});
-        }
-    } else {
-        for (int rx : {1, 2}) {
-            if (rx == 2 && P.W != 1) continue;
-            for (int ty : {64, 128, 256, 512, 1024}) cand.push_back({rx, ty});
-        }
-    }
-    if (cand.size() > 16) cand.resize(16);
-    if (P.cap_edges == 0) TRY(alloc_edges(pl, std::max<uint64_t>(4ull * P.N, 1ull << 16)));
-    // one shape and schedule order: bin pairs, the order, then the distance
-    // kernel three times (best of the three)
-    auto time_shape = [&](Plan Q, float *ms_out) -> idb_status {
-        launch_binpairs(Q, B, s);
-        TRY(read_counters(pl));
-        pl.P = Q;
-        TRY(alloc_binpairs(pl, c->h_ctr->n_binpairs));
-        Q.cap_binpairs = pl.P.cap_binpairs;
-        launch_binpairs_fill(Q, B, s);
-        if (Q.schedule == 1) launch_mlp_predict(B, (uint32_t)Q.cap_binpairs, c->mlp_bf16, s);
-        launch_schedule(Q, B, s);
-        float ms_best = 1e30f;
-        for (int rep = 0; rep < 3; ++rep) {
-            CU(cudaMemsetAsync(&B.ctr->unit_cursor, 0, 4, s));
-            CU(cudaMemsetAsync(&B.ctr->edge_reserved, 0, 4, s));
-            CU(cudaMemsetAsync(&B.ctr->n_edges, 0, 4, s));
-            CU(cudaMemsetAsync(&B.ctr->pairs_evaluated, 0, 8, s));
-            CU(cudaEventRecord(c->ev[0], s));
-            Q.cap_edges = pl.P.cap_edges;
-            launch_distance(Q, B, 0, s);
-            CU(cudaEventRecord(c->ev[1], s));
-            TRY(check_launch());
-            CU(cudaEventSynchronize(c->ev[1]));
-            float ms = 0;
-            CU(cudaEventElapsedTime(&ms, c->ev[0], c->ev[1]));
-            ms_best = std::min(ms_best, ms);
-            TRY(read_counters(pl));
-            if (c->h_ctr->error & kErrEdgeOverflow) {   // grow and repeat this shape
-                TRY(alloc_edges(pl, (uint64_t)c->h_ctr->edge_reserved + 64ull * kEdgeChunk * 1024));
-                CU(cudaMemsetAsync(&B.ctr->error, 0, 4, s));
-                --rep;
-                ms_best = 1e30f;
-            }
-        }
-        *ms_out = ms_best;
-        return IDB_OK;
-    };
-    double best_ms = 1e30;
-    Plan best_plan = P;
-    for (auto &cd : cand) {
-        Plan Q = P;
-        Q.schedule = 0;
-        if (P.fast) {
-            Q.RX = cd.first;
-            Q.TX = 32 * Q.RX;
-            Q.TY = cd.second;
-        } else {
-            Q.TY = cd.second;
-        }
-        float ms_best = 0;
-        TRY(time_shape(Q, &ms_best));
-        const int k = best->n_tried++;
-        best->tried_rx[k] = Q.RX;
-        best->tried_ty[k] = (int)Q.TY;
-        best->tried_ms[k] = ms_best;
-        if (ms_best < best_ms) {
-            best_ms = ms_best;
-            best_plan = Q;
-            best->tile_rx = Q.RX;
-            best->tile_ty = (int)Q.TY;
-            best->ms_distance = ms_best;
-        }
-    }
-    // the schedule order for the fastest shape: static heavy-first, or the
-    // learned cost when the context holds a model
-    best->schedule = 0;
-    best->schedule_ms[0] = best_ms;
-    if (c->has_model) {
-        Plan Q = best_plan;
-        Q.schedule = 1;
-        float ms_learned = 0;
-        TRY(time_shape(Q, &ms_learned));
-        best->schedule_ms[1] = ms_learned;
-        if (ms_learned < best_ms) best->schedule = 1;
-    }
-    TRY(device_errors(*c->h_ctr));
-    return IDB_OK;
+    return buckets_if_join_does_not_fit(c, [&](bool allow_join, bool *joined) {
+        return autotune(c, in, prm, best, allow_join, joined);
+    });
 }
 
 idb_status idb_count_admissible(idb_context *c, const idb_input *in, const idb_params *prm,

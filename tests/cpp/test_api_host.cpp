@@ -186,10 +186,58 @@ static void test_batch_run_with_more_genes_in_use() {
     }
 }
 
+// A join whose table, entries or bin pairs the device has no room for: every entry
+// point takes the buckets instead, as it would without a join, and gives the join's
+// memory back first; without room for the buckets either, out of memory.
+static void test_buckets_when_the_join_does_not_fit() {
+    struct Short { const char *what; uint32_t entries, binpairs; size_t lo, hi; };
+    const Short shorts[] = {{"table", 100, 20, 1000000, 100000000},
+                            {"entries", 1000000, 20, 15000000, 100000000},
+                            {"bin pairs", 100, 1000000, 15000000, 100000000}};
+    for (const bool hamming : {false, true})
+        for (const Short &sh : shorts) {
+            if (hamming && sh.hi == 100000000 && sh.lo == 1000000) continue;   // its table is smaller
+            idb_context *c = context();
+            Call a(5000, 60, 20, hamming, hamming ? 2 : 3);
+            script = Script();
+            CHECK(idb_cluster(c, &a.in, &a.prm, &a.out) == IDB_OK && a.stats.candidates == 1);
+            CHECK(idb_context_destroy(c) == IDB_OK);
+            c = context();
+            script.join_entries = sh.entries;
+            script.join_binpairs = sh.binpairs;
+            fake::st().fail_alloc = [&](size_t n) { return n >= sh.lo && n < sh.hi; };
+            for (int k = 0; k < 3; ++k) {   // eager, eager and captured, replayed
+                CHECK(idb_cluster(c, &a.in, &a.prm, &a.out) == IDB_OK);
+                CHECK(a.stats.candidates == 0 && a.stats.n_entries == script.bucket_entries);
+            }
+            CHECK(!c->buf[bJnTab].p && !c->buf[bJnPos].p);
+            CHECK(idb_cluster_device(c, &a.in, &a.prm, &a.out) == IDB_OK && a.stats.candidates == 0);
+            idb_stats st{};
+            idb_output o = a.out;
+            o.stats = nullptr;
+            CHECK(idb_batch_plan(c, &a.in, &a.prm, &o) == IDB_OK && idb_batch_run(c, &st) == IDB_OK);
+            CHECK(st.candidates == 0);
+            idb_tuning t{};
+            CHECK(idb_autotune(c, &a.in, &a.prm, &t) == IDB_OK && t.n_tried > 0);
+            std::vector<float> f(16 * script.bucket_binpairs), y(script.bucket_binpairs);
+            uint64_t n = 0;
+            CHECK(idb_profile_binpairs(c, &a.in, &a.prm, f.data(), y.data(), y.size(), &n) == IDB_OK);
+            CHECK(n == script.bucket_binpairs);
+            fake::st().fail_alloc = [](size_t b) { return b >= 20000; };
+            CHECK(idb_context_destroy(c) == IDB_OK);
+            c = context();
+            CHECK(idb_cluster(c, &a.in, &a.prm, &a.out) == IDB_ERR_OUT_OF_MEMORY);
+            fake::st().fail_alloc = nullptr;
+            CHECK(idb_cluster(c, &a.in, &a.prm, &a.out) == IDB_OK && a.stats.candidates == 1);
+            CHECK(idb_context_destroy(c) == IDB_OK);
+        }
+}
+
 int main(int argc, char **argv) {
     const std::map<std::string, void (*)()> tests = {
         {"tables_outlive_their_copies", test_tables_outlive_their_copies},
         {"batch_run_with_more_genes_in_use", test_batch_run_with_more_genes_in_use},
+        {"buckets_when_the_join_does_not_fit", test_buckets_when_the_join_does_not_fit},
     };
     const auto it = tests.find(argc > 1 ? argv[1] : "");
     if (it == tests.end()) { std::printf("unknown test\n"); return 2; }
