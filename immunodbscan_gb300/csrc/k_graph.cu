@@ -166,9 +166,7 @@ __global__ void k_flatten(const Counters *__restrict__ ctr, uint32_t *parent) {
     for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < nu; u += stride) {
         uint32_t r = vp[u];
         if (r & kNonCore) continue;
-        uint32_t pr = vp[r];
-        while (pr < r) { r = pr; pr = vp[r]; }   // strictly decreasing, terminates
-        vp[u] = r;
+        while (climb(vp, u, r)) {}   // strictly decreasing, terminates
     }
 }
 
@@ -239,11 +237,11 @@ __global__ void k_depth(uint32_t N, const uint32_t *__restrict__ row2uid, const 
         if (h[k]) atomicAdd(&hist[k], h[k]);
 }
 
-// Full compression: parent[u] = root of u for every core u.  The walk to the
-// root only reads: with path halving here, a halving step computed from a stale
-// parent could land after another thread's final root write and leave that
-// node pointing at an inner ancestor.  Each thread writes only its own node,
-// and the roots no longer change, so every write is final.
+// Full compression: parent[u] = root of u for every core u.  No path halving: a
+// halving step computed from a stale parent could land after another thread's
+// final root write and leave that node pointing at an inner ancestor.  Each
+// thread writes only its own node (climb, bitops.cuh), and the roots no longer
+// change, so its last write is final.
 __global__ void k_compress(const Counters *__restrict__ ctr, const uint32_t *__restrict__ ucore,
                            uint32_t *parent, uint32_t *__restrict__ rootflag, uint32_t N,
                            unsigned long long *stamp) {
@@ -252,16 +250,12 @@ __global__ void k_compress(const Counters *__restrict__ ctr, const uint32_t *__r
     const uint32_t stride = gridDim.x * blockDim.x;
     volatile uint32_t *vp = parent;
     for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < nu; u += stride) {
-        uint32_t r = u;
+        uint32_t r = kNone;
         if (ucore[u]) {
-            uint32_t pr = vp[r];
-            while (pr < r) {   // parent[y] <= y: strictly decreasing, terminates
-                r = pr;
-                pr = vp[r];
-            }
-            parent[u] = r;
+            r = vp[u];
+            while (climb(vp, u, r)) {}   // parent[y] <= y: strictly decreasing, terminates
         }
-        rootflag[u] = ucore[u] && r == u;
+        rootflag[u] = r == u;
     }
     // the scan runs over [0, N]: nothing past the uniques
     for (uint64_t u = (uint64_t)nu + blockIdx.x * blockDim.x + threadIdx.x; u <= N; u += stride) rootflag[u] = 0u;
