@@ -19,6 +19,7 @@ struct DistArgs {
     uint32_t A;                      // number of codes (Levenshtein)
     uint2 *edges;
     uint64_t cap_edges;
+    uint32_t chunk_log;              // edge slots a warp reserves at a time: 1 << chunk_log
     Counters *ctr;
     unsigned long long *bp_cycles;   // optional per bin-pair cycle log
     uint32_t *bp_hits;
@@ -120,10 +121,10 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
     return m;
 }
 
-// Edge writer: each warp reserves kEdgeChunk slots at a time; slots a warp
-// does not fill are set to the sentinel (x = kNone) before it moves on.
+// Edge writer: each warp reserves a chunk of 1 << chunk_log slots at a time; slots
+// a warp does not fill are set to the sentinel (x = kNone) at the end.
 struct EdgeWriter {
-    uint64_t base;     // kNone64 = no chunk held
+    uint64_t base;     // kNoChunk = no chunk held
     uint32_t fill;
     uint32_t written;
     static constexpr uint64_t kNoChunk = ~0ull;
@@ -132,7 +133,7 @@ struct EdgeWriter {
 
     __device__ void pad(const DistArgs &a, int lane) {
         if (base == kNoChunk || a.sink != kSinkEdges) return;
-        for (uint32_t t = fill + lane; t < kEdgeChunk; t += 32) {
+        for (uint32_t t = fill + lane; t < 1u << a.chunk_log; t += 32) {
             const uint64_t slot = base + t;
             if (slot < a.cap_edges) a.edges[slot] = make_uint2(kNone, kNone);
         }
@@ -145,55 +146,42 @@ struct EdgeWriter {
     __device__ void append(const DistArgs &a, int lane, bool ok, uint32_t lo, uint32_t hi) {
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, ok);
         if (!m) return;
-        const uint32_t n = __popc(m);
-        if (base == kNoChunk || fill + n > kEdgeChunk) {
-            pad(a, lane);
-            uint32_t b = 0;
-            if (lane == 0) b = atomicAdd(&a.ctr->edge_reserved, kEdgeChunk);
-            b = __shfl_sync(0xFFFFFFFFu, b, 0);
-            base = b;
-            fill = 0;
-            if ((uint64_t)b + kEdgeChunk > a.cap_edges && lane == 0)
-                atomicOr(&a.ctr->error, kErrEdgeOverflow);
-        }
+        const Bulk bk = reserve(a, lane, (uint32_t)__popc(m));
         if (ok) {
-            put_edge(a, base + fill + __popc(m & lanemask_lt()), lo, hi);
+            put_edge(a, slot_of(bk, (uint32_t)__popc(m & lanemask_lt())), lo, hi);
             if (COUNT || a.sink == kSinkCount)
                 count_pair(a, lo, hi, __ldg(&a.ucopies[lo]), __ldg(&a.ucopies[hi]));
         }
-        fill += n;
-        written += n;
     }
 
     // Bulk append, warp-uniform: the warp appends T edges at logical positions
     // 0..T-1 (each lane knows its own); the room left in the held chunk is
     // used first, then as many new chunks as needed, reserved with one atomic.
-    struct Bulk { uint64_t b0; uint32_t f0; uint64_t nb; };
+    struct Bulk { uint64_t b0, nb; uint32_t room; };
     __device__ Bulk reserve(const DistArgs &a, int lane, uint32_t T) {
+        const uint32_t chunk = 1u << a.chunk_log;
         Bulk k;
-        k.f0 = base == kNoChunk ? kEdgeChunk : fill;
-        k.b0 = base;
+        k.room = base == kNoChunk ? 0u : chunk - fill;
+        k.b0 = base + fill;
         k.nb = kNoChunk;
-        const uint32_t room = kEdgeChunk - k.f0;
-        if (T > room) {
-            const uint32_t nch = (T - room + kEdgeChunk - 1) / kEdgeChunk;
+        if (T > k.room) {
+            const uint32_t nch = (T - k.room + chunk - 1) >> a.chunk_log;
             uint32_t nb = 0;
-            if (lane == 0) nb = atomicAdd(&a.ctr->edge_reserved, nch * kEdgeChunk);
+            if (lane == 0) nb = atomicAdd(&a.ctr->edge_reserved, nch << a.chunk_log);
             nb = __shfl_sync(0xFFFFFFFFu, nb, 0);
-            if ((uint64_t)nb + (uint64_t)nch * kEdgeChunk > a.cap_edges && lane == 0)
+            if ((uint64_t)nb + ((uint64_t)nch << a.chunk_log) > a.cap_edges && lane == 0)
                 atomicOr(&a.ctr->error, kErrEdgeOverflow);
             k.nb = nb;
-            base = (uint64_t)nb + (uint64_t)(nch - 1) * kEdgeChunk;
-            fill = (T - room) - (nch - 1) * kEdgeChunk;
+            base = (uint64_t)nb + ((uint64_t)(nch - 1) << a.chunk_log);
+            fill = (T - k.room) - ((nch - 1) << a.chunk_log);
         } else {
-            fill = k.f0 + T;
+            fill += T;
         }
         written += T;
         return k;
     }
     __device__ __forceinline__ uint64_t slot_of(const Bulk &k, uint32_t i) const {
-        const uint32_t room = kEdgeChunk - k.f0;
-        return i < room ? k.b0 + k.f0 + i : k.nb + (i - room);
+        return i < k.room ? k.b0 + i : k.nb + (i - k.room);
     }
 };
 

@@ -16,7 +16,8 @@ constexpr int kFastMaxCodes = 32;       // alphabet of the fast (bit-plane) path
 constexpr int kFastMaxWords = 4;        // 128 residues on the fast path
 constexpr int kGenericMaxLen = 1024;    // Levenshtein on the generic path
 constexpr int kDepthMax = 50;           // tree-depth histogram cap (cuda/PSDBSCAN.hcu:1029)
-constexpr uint32_t kEdgeChunk = 256;    // edge slots reserved per warp at a time
+constexpr uint32_t kEdgeChunk = 256;    // edge slots reserved per warp at a time, in a long list
+constexpr uint32_t kEdgeChunkMin = 8;   // ... in the shortest (edge_chunk_log)
 constexpr uint32_t kUnionSample = 32;   // long edge lists: this fraction of them is merged first
 constexpr uint32_t kUnionSampleMin = 1u << 20;   // edge slots from which they are
 constexpr uint32_t kSpinCap = 1u << 22; // bound of every device-side retry loop

@@ -391,6 +391,19 @@ const char *distance_variant_name(const Plan &P) {
     return P.hamming ? "k_hamming" : (P.lev_diag ? "k_lev_diag" : "k_levenshtein");
 }
 
+// Slots a warp reserves at a time.  Every warp may leave most of a chunk unused, and
+// when there are few bin pairs nearly every resident warp finds an edge: with 256
+// slots each, 20k rows with 15k neighbour pairs reserved 0.6M slots, ran over
+// their first list (so the sweep ran twice and the list grew by 134 MB) and were
+// streamed under any edge-memory limit below that.  So at most a 64th of an SM's
+// share of the list; 256 from 2.5M slots on, where the counter's atomics count.
+static uint32_t edge_chunk_log(uint64_t cap_edges) {
+    const uint64_t share = cap_edges / (64ull * (uint64_t)sm_count());
+    uint32_t lg = 0;
+    while ((2u << lg) <= kEdgeChunk && ((2u << lg) <= share || (2u << lg) <= kEdgeChunkMin)) ++lg;
+    return lg;
+}
+
 void launch_distance(const Plan &P, const Buffers &B, int grid, cudaStream_t s, uint32_t sink) {
     DistArgs a = make_args(P, B);
     a.sink = sink;
@@ -398,6 +411,7 @@ void launch_distance(const Plan &P, const Buffers &B, int grid, cudaStream_t s, 
         a.edges = nullptr;
         a.cap_edges = ~0ull;
     }
+    a.chunk_log = edge_chunk_log(a.cap_edges);
     if (sink != kSinkGrow) {   // the work queues too; a repeated sweep counts anew
         launch_graph_init(P, B, s);
     } else {

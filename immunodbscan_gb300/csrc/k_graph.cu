@@ -66,7 +66,7 @@ k_count(const Counters *__restrict__ ctr, uint64_t cap, const uint2 *__restrict_
         const uint32_t *__restrict__ ucopies, uint32_t *__restrict__ cnt, uint32_t *__restrict__ parent,
         unsigned long long *stamp) {
     stamp_begin(stamp);
-    const uint32_t ne = edge_slots(ctr, cap) & ~3u;   // reserved in chunks of 256
+    const uint32_t ne = edge_slots(ctr, cap) & ~3u;   // reserved in chunks of 8 to 256
     const uint64_t stride = 4ull * gridDim.x * blockDim.x;
     for (uint64_t e0 = 4ull * (blockIdx.x * blockDim.x + threadIdx.x); e0 < ne; e0 += stride) {
         const uint4 v0 = __ldcs(reinterpret_cast<const uint4 *>(edges + e0));
@@ -179,7 +179,7 @@ __global__ void k_flatten(const Counters *__restrict__ ctr, uint32_t *parent) {
 __global__ void __launch_bounds__(kThreads)
 k_union(Counters *ctr, uint64_t cap, const uint2 *__restrict__ edges, uint32_t *parent,
         uint32_t *__restrict__ bmin) {
-    const uint32_t ne = edge_slots(ctr, cap) & ~3u;   // reserved in chunks of 256
+    const uint32_t ne = edge_slots(ctr, cap) & ~3u;   // reserved in chunks of 8 to 256
     const uint64_t stride = 4ull * gridDim.x * blockDim.x;
     uint32_t n_cc = 0;
     for (uint64_t e0 = 4ull * (blockIdx.x * blockDim.x + threadIdx.x); e0 < ne; e0 += stride) {
