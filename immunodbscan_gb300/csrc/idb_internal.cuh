@@ -234,7 +234,9 @@ struct Plan {
     bool wide = false;                            // V genes > 64 or J genes > 30, and then whether the genes
     bool compact = false;                         // in use fit the side records renumbered (an eager
                                                   // call reads it, a captured plan expects it)
-    bool side_exact() const { return !wide || compact; }   // side records hold every gene in use
+    // side records hold every gene in use: a join's next to 2 bits of the segment,
+    // the buckets' in whole words, renumbered or as they are
+    bool side_exact() const { return join ? !wide || compact : compact || (Gv <= 64 && Gj <= 32); }
     uint32_t join_smax = 1;                       // most segments of any length
     bool streamed = false;                        // neighbour pairs not stored: the
                                                   // distance work runs twice

@@ -233,11 +233,30 @@ static void test_buckets_when_the_join_does_not_fit() {
         }
 }
 
+// Which side records hold every gene in use and so decide a hit by themselves.
+static void test_side_records_decide() {
+    struct { uint32_t gv, gj; bool join, fits, exact; } cases[] = {
+        {64, 30, true, true, true},  {64, 30, false, true, true},  {64, 31, true, true, true},
+        {64, 31, true, false, false}, {64, 31, false, false, true}, {64, 32, false, false, true},
+        {64, 33, false, false, false}, {65, 32, false, false, false}, {65, 32, false, true, true},
+        {300, 200, true, true, true}};
+    for (const auto &t : cases) {
+        Plan P;
+        P.Gv = t.gv;
+        P.Gj = t.gj;
+        P.join = t.join;
+        P.wide = t.gv > 64 || t.gj > 30;
+        P.compact = P.wide && t.fits;
+        CHECK(P.side_exact() == t.exact);
+    }
+}
+
 int main(int argc, char **argv) {
     const std::map<std::string, void (*)()> tests = {
         {"tables_outlive_their_copies", test_tables_outlive_their_copies},
         {"batch_run_with_more_genes_in_use", test_batch_run_with_more_genes_in_use},
         {"buckets_when_the_join_does_not_fit", test_buckets_when_the_join_does_not_fit},
+        {"side_records_decide", test_side_records_decide},
     };
     const auto it = tests.find(argc > 1 ? argv[1] : "");
     if (it == tests.end()) { std::printf("unknown test\n"); return 2; }
