@@ -901,6 +901,13 @@ void set_join_shape(Plan &P, uint64_t pairs) {
     while (P.TY < 256 && (uint64_t)P.TX * P.TY * 2 <= want) P.TY *= 2;
 }
 
+// For a second run of a phase's first kernel, which would move the phase's start.
+Buffers without_stamps(const Buffers &B) {
+    Buffers q = B;
+    q.timing = false;
+    return q;
+}
+
 // After launch_buckets of an eager call with the edit-distance join: entries are
 // allocated for the join, or for the buckets where those score fewer pairs.  A
 // join pair costs about what a bucket pair does (the same test; its hits a few
@@ -912,6 +919,8 @@ idb_status choose_candidates(Pipeline &pl) {
     Plan &P = pl.P;
     Buffers &B = pl.B;
     cudaStream_t s = c->stream;
+    // the bucket phase began with the join that was built first
+    const Buffers again = without_stamps(B);
     TRY(read_counters(pl));
     if (P.wide) {
         P.compact = c->h_ctr->vj_compact != 0;
@@ -923,7 +932,7 @@ idb_status choose_candidates(Pipeline &pl) {
             P.TX = 32 * P.RX;
             P.TY = 256;
             apply_shape(P, pl.tile_rx == 2 ? 4 : pl.tile_rx, pl.tile_ty);
-            launch_buckets(P, B, s);
+            launch_buckets(P, again, s);
             TRY(check_launch());
             TRY(read_counters(pl));
         }
@@ -932,7 +941,7 @@ idb_status choose_candidates(Pipeline &pl) {
         const uint32_t join_entries = c->h_ctr->n_entries;
         const unsigned long long join_pairs = c->h_ctr->join_pairs;
         P.join = false;
-        launch_buckets(P, B, s);
+        launch_buckets(P, again, s);
         launch_bucket_pairs(P, B, s);
         TRY(check_launch());
         TRY(read_counters(pl));
@@ -985,8 +994,9 @@ idb_status run_phases(Pipeline &pl, bool eager, bool stop_after_schedule = false
         if (P.edge_budget) first = std::max<uint64_t>(std::min(first, P.edge_budget / kEdgeBytes), 4096);
         TRY(alloc_edges(pl, first));
     }
-    for (int attempt = 0; !P.streamed && attempt < 3; ++attempt) {
-        launch_distance(P, B, 0, s);
+    int attempt = 0;
+    for (; !P.streamed && attempt < 3; ++attempt) {
+        launch_distance(P, attempt ? without_stamps(B) : B, 0, s);
         TRY(check_launch());
         if (!eager) break;
         TRY(read_counters(pl));
@@ -1012,7 +1022,7 @@ idb_status run_phases(Pipeline &pl, bool eager, bool stop_after_schedule = false
         CU(cudaStreamSynchronize(s));
     }
     if (P.streamed) {
-        launch_streamed_sweeps(P, B, s);
+        launch_streamed_sweeps(P, attempt ? without_stamps(B) : B, s);
         TRY(check_launch());
         launch_streamed_labels(P, B, pl.trees, s);
     } else {

@@ -19,6 +19,7 @@ struct Script {
     uint32_t join_entries = 100, join_binpairs = 20, bucket_entries = 50, bucket_binpairs = 10;
     unsigned long long join_pairs = 1000, bucket_pairs = 2000;
     bool genes_fit = true;
+    uint32_t edge_overflows = 0;     // sweeps that run over their list
     std::vector<int16_t> eps_seen;   // the eps table as the device holds it
 } script;
 
@@ -82,10 +83,17 @@ void launch_binpairs(const Plan &P, const Buffers &B, cudaStream_t) {
 }
 void launch_binpairs_fill(const Plan &P, const Buffers &B, cudaStream_t) { note("binpairs", P, B); }
 void launch_schedule(const Plan &, const Buffers &, cudaStream_t) {}
-void launch_distance(const Plan &P, const Buffers &B, int, cudaStream_t, uint32_t) { note("distance", P, B); }
+void launch_distance(const Plan &P, const Buffers &B, int, cudaStream_t, uint32_t) {
+    note("distance", P, B);
+    Counters *c = B.ctr;
+    fake::push([=] {
+        c->edge_reserved = 100000;
+        if (script.edge_overflows) { --script.edge_overflows; c->error |= kErrEdgeOverflow; }
+    });
+}
 void launch_count_admissible(const Plan &, const Buffers &, cudaStream_t) {}
 void launch_graph(const Plan &, const Buffers &, bool, cudaStream_t, cudaEvent_t) {}
-void launch_streamed_sweeps(const Plan &, const Buffers &, cudaStream_t) {}
+void launch_streamed_sweeps(const Plan &P, const Buffers &B, cudaStream_t) { note("streamed", P, B); }
 void launch_streamed_labels(const Plan &, const Buffers &, bool, cudaStream_t) {}
 void launch_outputs(const Plan &, const Buffers &, cudaStream_t, uint32_t) {}
 uint32_t scan_part_needed(uint64_t n) { return (uint32_t)(n / 4096 + 2); }
@@ -251,12 +259,60 @@ static void test_side_records_decide() {
     }
 }
 
+// Candidates of a call whose join has many pairs: the buckets are counted and the
+// smaller side taken, eagerly and in the plan captured after; the join's time
+// stays in the bucket phase (one kernel writes its time stamp).
+static void test_candidates_by_pairs() {
+    for (const bool buckets_win : {false, true}) {
+        idb_context *c = context();
+        Call a(500, 8, 3, false, 2);
+        script = Script();
+        script.join_pairs = kJoinSurePairs + 1;
+        script.bucket_pairs = buckets_win ? kJoinSurePairs : kJoinSurePairs + 1;
+        fake::st().log.clear();
+        CHECK(idb_cluster_device(c, &a.in, &a.prm, &a.out) == IDB_OK);
+        CHECK(a.stats.candidates == (buckets_win ? 0u : 1u));
+        CHECK(a.stats.n_entries == (buckets_win ? script.bucket_entries : script.join_entries));
+        CHECK(c->h_ctr->n_binpairs == (buckets_win ? script.bucket_binpairs : script.join_binpairs));
+        CHECK(logged("buckets join=1") == 1 && logged("buckets join=0") == 1);
+        CHECK(logged("buckets join=1 compact=0 timing=1") == 1 && logged("buckets join=0 compact=0 timing=0") == 1);
+        CHECK(logged(std::string("distance join=") + (buckets_win ? "0" : "1") + " compact=0 timing=1") == 1);
+        idb_output o = a.out;
+        o.stats = nullptr;
+        CHECK(idb_batch_plan(c, &a.in, &a.prm, &o) == IDB_OK);
+        CHECK(idb_batch_run(c, &a.stats) == IDB_OK && a.stats.candidates == (buckets_win ? 0u : 1u));
+        CHECK(a.stats.n_entries == (buckets_win ? script.bucket_entries : script.join_entries));
+        CHECK(idb_context_destroy(c) == IDB_OK);
+    }
+}
+
+// A sweep that runs over its list is repeated with a longer one, or streamed under
+// an edge-memory limit: the distance phase begins with the first sweep.
+static void test_repeated_sweeps_keep_the_stamp() {
+    for (const int mb : {0, 1, -1}) {
+        idb_context *c = context();
+        Call a(500, 8, 3, false, 2);
+        script = Script();
+        script.edge_overflows = mb < 0 ? 0 : 1;
+        a.prm.edge_memory_mb = mb;
+        fake::st().log.clear();
+        CHECK(idb_cluster_device(c, &a.in, &a.prm, &a.out) == IDB_OK);
+        CHECK(a.stats.streamed == (mb != 0));
+        const std::string at = " join=1 compact=0 timing=";
+        CHECK(logged("distance" + at + "1") == (mb >= 0) && logged("distance" + at + "0") == (mb == 0));
+        CHECK(logged("streamed" + at + "0") == (mb > 0) && logged("streamed" + at + "1") == (mb < 0));
+        CHECK(idb_context_destroy(c) == IDB_OK);
+    }
+}
+
 int main(int argc, char **argv) {
     const std::map<std::string, void (*)()> tests = {
         {"tables_outlive_their_copies", test_tables_outlive_their_copies},
         {"batch_run_with_more_genes_in_use", test_batch_run_with_more_genes_in_use},
         {"buckets_when_the_join_does_not_fit", test_buckets_when_the_join_does_not_fit},
         {"side_records_decide", test_side_records_decide},
+        {"candidates_by_pairs", test_candidates_by_pairs},
+        {"repeated_sweeps_keep_the_stamp", test_repeated_sweeps_keep_the_stamp},
     };
     const auto it = tests.find(argc > 1 ? argv[1] : "");
     if (it == tests.end()) { std::printf("unknown test\n"); return 2; }
