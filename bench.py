@@ -461,30 +461,19 @@ def main():
     gops = C.c_double()
     pms = C.c_double()
     L.idb_diag_int_peak(local, C.byref(gops), C.byref(pms))
-    ops_pair = ops_per_pair(w, None)
+    kernel, unit, units, ops_unit = distance_work(w, last)
     t_dist = r["ms_dist"] * 1e-3
-    if w.use_hamming:
-        work_ops = ops_pair * last.pairs_evaluated
-    elif last.lev_columns:      # Myers/Hyyro: ops per text column actually consumed
-        work_ops = ops_pair * last.lev_columns
-    else:                       # diagonal test, eps 2, one word: three masks of 5 planes, 16 for the test
-        ops_pair = 31
-        work_ops = ops_pair * last.pairs_evaluated
-    per_column = not w.use_hamming and last.lev_columns > 0
-    achieved = work_ops / t_dist / 1e9 if t_dist > 0 else 0.0
+    achieved = ops_unit * units / t_dist / 1e9 if ops_unit and t_dist > 0 else None
     out["roofline"] = {"bound": "int", "achieved": achieved, "peak": gops.value,
                        "unit": "Gop/s (32-bit integer logic)",
-                       "frac": achieved / gops.value if gops.value else None,
+                       "frac": achieved / gops.value if achieved is not None and gops.value else None,
                        "traffic": (profiled_traffic("k_hamming", w.name)
                                    if w.use_hamming and args.scale == 1.0 else None),
                        "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one "
                                          "launch at scale 0.2, scaled by the rows to full size "
                                          "(profiles/k_hamming_workload2_scale0.2.md)",
-                       "kernel": ("k_hamming" if w.use_hamming else
-                                  "k_levenshtein" if per_column else "k_lev_diag"),
-                       "ops_per_unit": ops_pair,
-                       "work_unit": "pair-column (text residue)" if per_column else "pair",
-                       "work_units": int(last.lev_columns if per_column else last.pairs_evaluated),
+                       "kernel": kernel, "ops_per_unit": ops_unit, "work_unit": unit,
+                       "work_units": units,
                        "kernel_ms": t_dist * 1e3,
                        "hit_fraction": (float(last.neighbour_pairs) / float(last.pairs_evaluated)
                                         if w.use_hamming and last.pairs_evaluated else None),
@@ -898,8 +887,20 @@ def copy_times(host_inputs, host_outputs, reps: int = 5):
     return up, down
 
 
-def ops_per_pair(w, batch) -> int:
-    """Algorithmic 32-bit integer ops per evaluated pair of the distance kernel.
+def distance_work(w, last):
+    """(kernel, unit of its work, units done, integer operations a unit) of a run with
+    statistics ``last``.  The diagonal test has no one count: its operations follow
+    the eps and the length gap of each pair, which the statistics do not hold."""
+    pairs, columns = int(last.pairs_evaluated), int(last.lev_columns)
+    if w.use_hamming:
+        return "k_hamming", "pair", pairs, ops_per_pair(w)
+    if columns:
+        return "k_levenshtein", "pair-column (text residue)", columns, ops_per_pair(w)
+    return "k_lev_diag", "pair", pairs, None
+
+
+def ops_per_pair(w) -> int:
+    """Algorithmic 32-bit integer ops per unit of the distance kernel's work.
 
     Hamming (bit planes): one LOP3 per plane word folds XOR and OR, then the
     population test (eps==1: x & (x-1) == 0 -> 2 ops + 1 compare; otherwise
