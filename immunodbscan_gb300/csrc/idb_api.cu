@@ -703,12 +703,19 @@ idb_status alloc_fixed(Pipeline &pl) {
     Plan &P = pl.P;
     Buffers &B = pl.B;
     const size_t N = P.N, N1 = N + 1;
+    // the code map and the eps table in one copy; a long table (a wide length range)
+    // from where it is
     HostPack &pack = pl.plan_tables;
-    const size_t eps_at = pack.add(pl.eps_host.data(), sizeof(int16_t) * pl.eps_host.size());
-    const size_t code_at = pack.add(P.codemap, 256);
+    const size_t code_at = pack.add(P.codemap, 256), eps_bytes = sizeof(int16_t) * pl.eps_host.size();
+    const bool packed = eps_bytes <= 65536;
+    const size_t eps_at = packed ? pack.add(pl.eps_host.data(), eps_bytes) : 256;
+    TRY(ensure(c, bPlanTables, eps_at + eps_bytes));
     TRY(pl.upload(pack, bPlanTables));
-    B.eps_tab = reinterpret_cast<const int16_t *>(ptr<uint8_t>(c, bPlanTables) + eps_at);
-    B.codemap = ptr<uint8_t>(c, bPlanTables) + code_at;
+    uint8_t *const tables = ptr<uint8_t>(c, bPlanTables);
+    if (!packed)
+        CU(cudaMemcpyAsync(tables + eps_at, pl.eps_host.data(), eps_bytes, cudaMemcpyHostToDevice, c->stream));
+    B.eps_tab = reinterpret_cast<const int16_t *>(tables + eps_at);
+    B.codemap = tables + code_at;
     TRY(ensure(c, bVBits, sizeof(uint64_t) * N * P.VW));
     TRY(ensure(c, bJBits, sizeof(uint64_t) * N * P.JW));
     TRY(ensure(c, bSlot, 4 * N));

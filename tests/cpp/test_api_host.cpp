@@ -305,6 +305,30 @@ static void test_repeated_sweeps_keep_the_stamp() {
     }
 }
 
+// The eps table of a wide length range (2 bytes a pair of lengths) goes to the device
+// from where it was made, without a second copy of it on the host.
+static void test_long_eps_table() {
+    for (const uint32_t lmax : {40u, 3000u}) {
+        idb_context *c = context();
+        Call a(100, 8, 3, true, 2);
+        script = Script();
+        script.lmin = 1;
+        script.lmax = lmax;
+        CHECK(idb_cluster(c, &a.in, &a.prm, &a.out) == IDB_OK);
+        CHECK(script.eps_seen == std::vector<int16_t>((size_t)lmax * lmax, 2));
+        {
+            Pipeline pl;
+            pl.c = c;
+            CHECK(stage_inputs_and_survey(pl, &a.in, true) == IDB_OK);
+            CHECK(derive_plan(pl, &a.prm) == IDB_OK && alloc_fixed(pl) == IDB_OK);
+            CHECK(pl.plan_tables.bytes.size() <= 70000);
+            CHECK(read_counters(pl) == IDB_OK);
+            CHECK(std::memcmp(pl.B.codemap, pl.P.codemap, 256) == 0);
+        }
+        CHECK(idb_context_destroy(c) == IDB_OK);
+    }
+}
+
 int main(int argc, char **argv) {
     const std::map<std::string, void (*)()> tests = {
         {"tables_outlive_their_copies", test_tables_outlive_their_copies},
@@ -313,6 +337,7 @@ int main(int argc, char **argv) {
         {"side_records_decide", test_side_records_decide},
         {"candidates_by_pairs", test_candidates_by_pairs},
         {"repeated_sweeps_keep_the_stamp", test_repeated_sweeps_keep_the_stamp},
+        {"long_eps_table", test_long_eps_table},
     };
     const auto it = tests.find(argc > 1 ? argv[1] : "");
     if (it == tests.end()) { std::printf("unknown test\n"); return 2; }

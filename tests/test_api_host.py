@@ -28,7 +28,7 @@ def exe(tmp_path_factory):
 
 @pytest.mark.parametrize("name", ["tables_outlive_their_copies", "batch_run_with_more_genes_in_use",
                                   "buckets_when_the_join_does_not_fit", "side_records_decide",
-                                  "candidates_by_pairs", "repeated_sweeps_keep_the_stamp"])
+                                  "candidates_by_pairs", "repeated_sweeps_keep_the_stamp", "long_eps_table"])
 def test_api_host(exe, name):
     r = subprocess.run([exe, name], capture_output=True, text=True, timeout=120,
                        env=dict(os.environ, ASAN_OPTIONS="detect_leaks=0"))
