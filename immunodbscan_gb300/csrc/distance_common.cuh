@@ -1,6 +1,6 @@
 // distance_common.cuh -- what the distance kernels share: their arguments, where
 // neighbour pairs go (the edge list, or the two sweeps of the streamed mode), the
-// work queue of tiled units, deferred hits and the small bin pairs' helpers.
+// work queue of tiled units, batches of hits and the small bin pairs' helpers.
 #pragma once
 #include "idb_internal.cuh"
 
@@ -22,14 +22,13 @@ struct DistArgs {
     uint32_t chunk_log;              // edge slots a warp reserves at a time: 1 << chunk_log
     Counters *ctr;
     unsigned long long *bp_cycles;   // optional per bin-pair cycle log
-    uint32_t *bp_hits;
     const uint4 *meta;               // per entry {sigV lo, sigV hi, sigJ, uid}
     int sig_exact;                   // signatures decide canonicity exactly
     const uint32_t *small_list;      // schedule positions of the small bin pairs (from the
                                      // front) and of the tiny ones (from small_cap - 1 down)
     uint32_t small_cap;
-    // segment join: a hit is a neighbour pair if the V and J sets intersect and
-    // no lower segment is identical (that segment's group emits it)
+    // segment join: a hit is a neighbour pair if the V and J sets intersect and no
+    // lower segment (edit distance: no earlier look-up) holds, whose group emits it
     int join;
     int vj_meta;                     // the join's side records hold the V and J bits
     // where neighbour pairs go: kSinkEdges = the edge list; kSinkCount /

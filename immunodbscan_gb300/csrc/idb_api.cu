@@ -1395,7 +1395,7 @@ idb_status capture_batch_plan(Pipeline &pl, const idb_output &o) {
     CU(cudaStreamSynchronize(s));
     CU(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(pl.B.ctr, 0, sizeof(Counters), s);
-    pl.timing = true;   // time-stamp kernels between the phases
+    pl.timing = true;   // the phases' first kernels write their time stamps
     pl.B.timing = pl.timing;
     launch_survey(pl.P, pl.B, s);
     idb_status st = run_phases(pl, false);

@@ -164,7 +164,6 @@ struct Counters {
     uint32_t n_clusters;
     uint32_t n_noise_rows;
     uint32_t error;
-    uint32_t heavy_count;
     unsigned long long pairs_evaluated;
     unsigned long long admissible_pairs;
     unsigned long long stamp[8];  // %globaltimer at the phase boundaries (ns)
@@ -250,7 +249,7 @@ struct Plan {
     uint8_t codemap[256];
     int first_byte = -1;                          // byte value with code 0
     // capacities
-    uint64_t cap_entries = 0, cap_binpairs = 0, cap_units = 0, cap_edges = 0;
+    uint64_t cap_entries = 0, cap_binpairs = 0, cap_edges = 0;
 };
 
 // Scratch of the call-string collapse of one gene column.
@@ -277,7 +276,6 @@ struct Buffers {
     const uint8_t *codemap = nullptr;               // [256]
     // row level [N]
     uint64_t *vbits = nullptr, *jbits = nullptr;    // [N*VW], [N*JW]
-    uint64_t *rhash = nullptr;
     uint32_t *slot = nullptr, *rep_row = nullptr, *flag = nullptr, *uid_of_row = nullptr;
     uint32_t *row2uid = nullptr;
     // duplicate table
@@ -336,7 +334,6 @@ struct Buffers {
     unsigned long long *stamp(int k) const { return timing ? &ctr->stamp[k] : nullptr; }
     // per bin-pair timing log (optional)
     unsigned long long *bp_cycles = nullptr;
-    uint32_t *bp_hits = nullptr;
 };
 
 // ---- launchers (each enqueues on `s`, never synchronises) ----

@@ -678,7 +678,6 @@ k_join_fill(BinGeom g, const Counters *__restrict__ ctr, const uint32_t *__restr
     __syncthreads();
     const uint32_t nu = ctr->n_uniques;
     const uint32_t stride = gridDim.x * blockDim.x;
-    const uint32_t lane = threadIdx.x & 31;
     for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < nu; u += stride) {
         const uint32_t row = urow[u], L = ulen[u];
         if (!g.in_range(L)) continue;
@@ -702,7 +701,6 @@ k_join_fill(BinGeom g, const Counters *__restrict__ ctr, const uint32_t *__restr
 #pragma unroll
             for (int q = 0; q < RSC; ++q) dst[q] = rec[q];
         }
-        (void)lane;
     }
 }
 

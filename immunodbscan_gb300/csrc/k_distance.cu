@@ -27,12 +27,17 @@
 //    diagonal value never decreases, so the early exit is exact).
 //  * A neighbour pair is kept only in the bin of its lowest common V gene and
 //    lowest common J gene, so a pair that shares several bins counts once.
-//  * Segment join (Hamming, eps <= 2): the "bins" are groups of uniques that
-//    share one whole segment; a pair is kept only in the group of its lowest
-//    identical segment, and only if its V and J sets intersect.
-//  * Bin pairs of at most 32 entries a side are scored pair-parallel (records
-//    by shuffles), and a bin with itself of at most 8 entries by one lane.
-//  * Hits are queued per lane and written as one warp-compacted bulk append.
+//  * Segment joins: the "bins" are groups of uniques that share a whole segment
+//    (Hamming, eps <= 2) or in which one holds a segment of the other at a small
+//    shift (edit distance, eps <= 3); a pair is kept only in the group of its
+//    lowest identical segment, or of its first look-up that holds, and only if
+//    its V and J sets intersect.
+//  * Bin pairs of at most 32 entries a side are scored pair-parallel (Hamming:
+//    records by shuffles; edit distance: from L1), and those of at most 28 pairs
+//    by one lane (Hamming: a bin with itself).
+//  * With bit planes a lane's hits are bits of a batch of 32 y-entries, written as
+//    one bulk append with both sides' counts; the byte and the Myers kernels
+//    append each round's hits, and k_count sums their counts from the list.
 #include "distance_common.cuh"
 
 namespace idb {
@@ -362,7 +367,6 @@ static DistArgs make_args(const Plan &P, const Buffers &B) {
     a.cap_edges = P.cap_edges;
     a.ctr = B.ctr;
     a.bp_cycles = B.bp_cycles;   // set only while profiling
-    a.bp_hits = B.bp_hits;
     a.meta = B.ent_meta;
     a.sig_exact = (P.side_exact() && !P.join) ? 1 : 0;
     a.small_list = B.bp_small;

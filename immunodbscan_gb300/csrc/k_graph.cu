@@ -13,9 +13,9 @@
 //  tree depths       cuda/PSDBSCAN.hcu:154-177, 1020-1040
 //
 // Here the neighbour pairs found by the distance kernel form an edge list.
-// Counts come with it (PairSums, count_pair); core-core edges are merged by unions that
-// hook the larger root under the smaller one with atomicCAS while find()
-// halves paths, so every component's root is its minimum core index, as in the
+// Counts come with it (the emit functions and count_pair of distance_common.cuh, or
+// k_count); core-core edges are merged by unions that hook the larger root under
+// the smaller one with atomicCAS while find() halves paths, so every component's root is its minimum core index, as in the
 // reference.  In the same pass every core-to-non-core edge offers its core end
 // to the non-core end with atomicMin, so a non-core unique joins the cluster
 // of its minimum-index core neighbour (deterministic; one of the outcomes the

@@ -1,4 +1,4 @@
-// k_ham_aa.cu -- Hamming distances on 5-plane records (up to 32 residues).
+// k_ham_aa.cu -- Hamming distances on 5-plane records (up to 32 residue values).
 #include "hamming.cuh"
 
 namespace idb {

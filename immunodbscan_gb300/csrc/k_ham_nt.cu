@@ -1,4 +1,4 @@
-// k_ham_nt.cu -- Hamming distances on 2-plane records (up to 4 residues).
+// k_ham_nt.cu -- Hamming distances on 2-plane records (up to 4 residue values).
 #include "hamming.cuh"
 
 namespace idb {

@@ -1,4 +1,4 @@
-// k_lev_aa.cu -- edit distances up to 3 on 5-plane records (up to 32 residues).
+// k_lev_aa.cu -- edit distances up to 3 on 5-plane records (up to 32 residue values).
 #include "lev_diag.cuh"
 
 namespace idb {

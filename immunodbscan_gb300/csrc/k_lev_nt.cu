@@ -1,4 +1,4 @@
-// k_lev_nt.cu -- edit distances up to 3 on 2-plane records (up to 4 residues).
+// k_lev_nt.cu -- edit distances up to 3 on 2-plane records (up to 4 residue values).
 #include "lev_diag.cuh"
 
 namespace idb {

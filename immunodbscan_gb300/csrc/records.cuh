@@ -24,8 +24,7 @@ struct BinGeom {
 //  codes (other Levenshtein and the generic path): one code byte per residue.
 // Codes are a bijection of the byte values present, so equality of codes is
 // equality of bytes.
-// The record of one unique (fast paths: at most NR 16-byte words): bit planes
-// or code bytes, residues read 4 at a time.
+
 // Bit planes of one sequence (L <= 128): bit i of wd[p][w] is bit p of the
 // code of residue 32w + i; positions past L keep code 0.  Residues are read 4
 // at a time.
@@ -76,6 +75,8 @@ __device__ __forceinline__ void flatten_planes(const uint32_t (&wd)[5][4], int p
         rec[q] = make_uint4(flat[4 * q], flat[4 * q + 1], flat[4 * q + 2], flat[4 * q + 3]);
 }
 
+// The record of one unique (fast paths: at most NR 16-byte words): bit planes, or
+// code bytes (planes == 0).
 template <int NR>
 __device__ __forceinline__ void build_small_record(const uint8_t *s, uint32_t L,
                                                    const uint8_t *cm, int planes, uint32_t W,

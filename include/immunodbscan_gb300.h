@@ -62,7 +62,8 @@ typedef struct idb_params {
     int32_t  tile_ty;          /* y-entries of a work unit (0 = default)           */
     int32_t  candidates;       /* 0 = automatic (Hamming eps <= 2 and edit distance
                                   eps <= 3: segment join, unless the buckets
-                                  hold fewer pairs than an edit-distance join),
+                                  hold fewer pairs than an edit-distance join
+                                  or the device has no room for the join),
                                   1 = every admissible pair of the buckets        */
     int32_t  edge_memory_mb;   /* device memory for the neighbour-pair list:
                                   0 = as much as the pairs need; > 0 = at most this
@@ -174,7 +175,9 @@ idb_status idb_cluster_device(idb_context *ctx, const idb_input *in, const idb_p
    repertoires, graph, labels) into a CUDA graph; idb_batch_run replays it and
    recomputes everything from the inputs.  If new data at the same addresses
    exceeds the plan, idb_batch_run returns IDB_ERR_CAPACITY or IDB_ERR_REPLAN
-   and the caller plans again. */
+   and the caller plans again.  (A plan over a list of more than 64 V or 30 J
+   genes whose data come to use more of them than when it was made is planned
+   again inside idb_batch_run: that run takes as long as a plan.) */
 idb_status idb_batch_plan(idb_context *ctx, const idb_input *in, const idb_params *prm,
                           const idb_output *out);
 idb_status idb_batch_run(idb_context *ctx, idb_stats *stats);
