@@ -202,7 +202,7 @@ __device__ __forceinline__ void hamming_tiny_all(const DistArgs &a, EdgeWriter &
                 dw[w] = d;
                 dist += __popc(d);
             }
-            const uint32_t sc = EM == 2 ? dw[0] : (EM == 1 ? (dw[0] & (dw[0] - 1u)) : dist);
+            const uint32_t sc = W == 1 && EM == 2 ? dw[0] : (W == 1 && EM == 1 ? (dw[0] & (dw[0] - 1u)) : dist);
             if (sc > thr) continue;
             const uint4 mx = __ldg(a.meta + P.a_start + i), my = __ldg(a.meta + P.a_start + j);
             bool ok;
