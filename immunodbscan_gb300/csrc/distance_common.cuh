@@ -532,8 +532,7 @@ int occupancy_grid(K kernel, size_t smem) {
 
 template <typename K>
 void run(K kernel, const DistArgs &a, size_t smem, int grid, cudaStream_t s) {
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_dynamic_smem(reinterpret_cast<const void *>(kernel));
     if (grid <= 0) grid = occupancy_grid(kernel, smem);
     kernel<<<grid, kWarps * 32, smem, s>>>(a);
 }

@@ -1653,6 +1653,24 @@ int resident_blocks(const void *kern, int threads, size_t smem) {
     return per_sm;
 }
 
+void allow_dynamic_smem(const void *kern) {
+    struct Entry { const void *k; int dev; };
+    static std::mutex mu;
+    static std::vector<Entry> done;
+    int d = 0, most = 0;
+    cudaGetDevice(&d);
+    std::lock_guard<std::mutex> lock(mu);
+    for (const Entry &e : done)
+        if (e.k == kern && e.dev == d) return;
+    cudaFuncAttributes fa{};
+    if (cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, d) != cudaSuccess ||
+        cudaFuncGetAttributes(&fa, kern) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             most - (int)fa.sharedSizeBytes) != cudaSuccess)
+        return;   // the launch reports it
+    done.push_back(Entry{kern, d});
+}
+
 int sm_count() {
     static thread_local int dev = -1, n = 0;
     int d = 0;

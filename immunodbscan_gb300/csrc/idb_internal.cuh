@@ -407,6 +407,11 @@ const char *distance_variant_name(const Plan &P);
 // shared memory), from the occupancy calculator; cached per kernel and device.
 int resident_blocks(const void *kern, int threads, size_t smem);
 
+// Lets a kernel launch with any dynamic shared memory the device has.  The limit
+// belongs to the kernel, not to the caller: raised to one caller's size, another
+// thread with a smaller size would lower it under the first one's next launch.
+void allow_dynamic_smem(const void *kern);
+
 // Grid of a grid-stride kernel over n items: one block per `threads` items, at
 // most one full wave of resident blocks, so that no block starts in a second
 // wave after the first has drained.

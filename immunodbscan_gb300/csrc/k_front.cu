@@ -1115,11 +1115,7 @@ void launch_gene_bits(const Plan &P, const Buffers &B, bool v_column, uint32_t c
         calls, off, r0, r1, cs.tab, cs.mask, cs.ref, todo, ntodo);
     // 2. bitsets of the representatives
     const size_t smem = gene_bits_smem(G, GW, gm.ts, name_bytes);
-    static thread_local size_t attr_set = 0;
-    if (smem > 48 * 1024 && smem > attr_set) {
-        cudaFuncSetAttribute(k_gene_bits, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr_set = smem;
-    }
+    if (smem > 48 * 1024) allow_dynamic_smem(reinterpret_cast<const void *>(k_gene_bits));
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gene_bits, kGbWarps * 32, smem);
     const uint64_t want = ((uint64_t)nrows + kGbRows * kGbWarps - 1) / (kGbRows * kGbWarps);

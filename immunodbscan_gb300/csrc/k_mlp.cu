@@ -326,11 +326,7 @@ void launch_mlp_predict(const Buffers &B, uint32_t cap, const void *wq_bf16, cud
 
 void launch_mlp_grad(const float *X, const float *T, uint32_t n, const float *p, float scale,
                      float *grad, float *loss, cudaStream_t s) {
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGradSmem);
-        attr = true;
-    }
+    allow_dynamic_smem(reinterpret_cast<const void *>(k_mlp_grad));
     const int grid = (int)std::min<uint64_t>((n + kTile - 1) / kTile, (uint64_t)sm_count() * 2);
     k_mlp_grad<<<grid > 0 ? grid : 1, kGradThreads, kGradSmem, s>>>(X, T, n, p, scale, grad, loss);
 }
